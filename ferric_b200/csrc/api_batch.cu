@@ -22,7 +22,7 @@ fc_status batch_alloc(fc_rimp2_batch* b, size_t bytes, void** out) {
     if (bytes == 0) bytes = 256;
     FC_TRY(pool_reserve(bytes));
     void* p = nullptr;
-    FC_CUDA(cudaMalloc(&p, bytes));
+    FC_CUDA(spare_malloc(&p, bytes));
     b->allocs.push_back(p);
     b->bytes += bytes;
     ctx().handle_bytes += bytes;

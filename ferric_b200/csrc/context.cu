@@ -52,14 +52,65 @@ uint64_t ws_bytes() {
     return t;
 }
 
+// Give back the residue slots (false if they held nothing).
+static bool drop_mg() {
+    Context& c = ctx();
+    bool any = false;
+    for (int s = WS_MG_A; s <= WS_MG_MISC; ++s) any |= c.ws[s].ptr != nullptr;
+    if (!any || cudaDeviceSynchronize() != cudaSuccess) return false;
+    for (int s = WS_MG_A; s <= WS_MG_MISC; ++s) {
+        if (c.ws[s].ptr) cudaFree(c.ws[s].ptr);
+        c.ws[s] = Workspace{};
+    }
+    return true;
+}
+
 fc_status pool_reserve(uint64_t bytes) {
     Context& c = ctx();
+    if (c.pool_cap && ws_bytes() + c.handle_bytes + bytes > c.pool_cap) drop_mg();
     if (c.pool_cap && ws_bytes() + c.handle_bytes + bytes > c.pool_cap)
         return fail(FC_ERR_POOL_FULL,
                     "device pool full: need " + std::to_string(bytes) + " B, held " +
                         std::to_string(ws_bytes() + c.handle_bytes) + " B of cap " +
                         std::to_string(c.pool_cap) + " B");
     return FC_OK;
+}
+
+cudaError_t spare_malloc(void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && drop_mg()) {
+        cudaGetLastError();
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
+}
+
+bool ws_get_mg(const size_t (&need)[WS_MG_SLOTS], void* (&out)[WS_MG_SLOTS]) {
+    Context& c = ctx();
+    uint64_t extra = 0;
+    for (int k = 0; k < WS_MG_SLOTS; ++k) {
+        const Workspace& w = c.ws[WS_MG_A + k];
+        if (need[k] > w.bytes) extra += need[k] + 256 - w.bytes;
+    }
+    if (extra) {
+        if (c.pool_cap) {
+            const uint64_t held = ws_bytes() + c.handle_bytes;
+            if (held >= c.pool_cap || extra > (c.pool_cap - held) / 2) return false;
+        }
+        size_t avail = 0, total = 0;
+        if (cudaMemGetInfo(&avail, &total) != cudaSuccess || extra > avail / 2) {
+            cudaGetLastError();
+            return false;
+        }
+    }
+    for (int k = 0; k < WS_MG_SLOTS; ++k) {
+        out[k] = nullptr;
+        if (need[k] && ws_get(WS_MG_A + k, need[k], &out[k]) != FC_OK) {
+            cudaGetLastError();
+            return false;
+        }
+    }
+    return true;
 }
 
 fc_status ws_get(int slot, size_t bytes, void** out) {
@@ -69,6 +120,8 @@ fc_status ws_get(int slot, size_t bytes, void** out) {
     Workspace& w = c.ws[slot];
     if (w.bytes < bytes) {
         uint64_t others = ws_bytes() - w.bytes + c.handle_bytes;
+        if (c.pool_cap && others + bytes > c.pool_cap && slot < WS_MG_A && drop_mg())
+            others = ws_bytes() - w.bytes + c.handle_bytes;
         if (c.pool_cap && others + bytes > c.pool_cap)
             return fail(FC_ERR_POOL_FULL, "device pool full: workspace of " +
                                               std::to_string(bytes) + " B over cap " +
@@ -80,7 +133,11 @@ fc_status ws_get(int slot, size_t bytes, void** out) {
             w.ptr = nullptr;
             w.bytes = 0;
         }
-        FC_CUDA(cudaMalloc(&w.ptr, bytes));
+        const cudaError_t e = slot < WS_MG_A ? spare_malloc(&w.ptr, bytes) : cudaMalloc(&w.ptr, bytes);
+        if (e != cudaSuccess) {
+            w.ptr = nullptr;
+            return cuda_fail(e, "cudaMalloc(workspace)");
+        }
         w.bytes = bytes;
     }
     *out = w.ptr;

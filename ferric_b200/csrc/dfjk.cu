@@ -429,7 +429,7 @@ fc_status dfjk_prepare_mixed(fc_dfjk* h, cudaStream_t st) {
     h->ld32 = (h->pair + 3) / 4 * 4;
     const int64_t npk = h->naux * h->ld32;
     FC_TRY(pool_reserve((uint64_t)npk * 4));
-    FC_CUDA(cudaMalloc(&h->pk32, (size_t)npk * 4));
+    FC_CUDA(spare_malloc((void**)&h->pk32, (size_t)npk * 4));
     h->bytes += (uint64_t)npk * 4;
     if (h->ld32 != h->pair) FC_CUDA(cudaMemsetAsync(h->pk32, 0, (size_t)npk * 4, st));
     void* vf;
@@ -629,10 +629,10 @@ fc_status create_common(const double* b, int64_t naux, int64_t n, int32_t layout
     };
     cudaError_t e;
     if (bytes_sq) {
-        e = cudaMalloc(&h->b_sq, bytes_sq);
+        e = spare_malloc((void**)&h->b_sq, bytes_sq);
         if (e != cudaSuccess) return bail(cuda_fail(e, "cudaMalloc(B square)"));
     }
-    e = cudaMalloc(&h->b_pk, bytes_pk);
+    e = spare_malloc((void**)&h->b_pk, bytes_pk);
     if (e != cudaSuccess) return bail(cuda_fail(e, "cudaMalloc(B packed)"));
     const cudaMemcpyKind kind = host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
     if (layout == FC_LAYOUT_SQUARE) {
@@ -678,7 +678,7 @@ fc_status fc_dfj_set_metric_chol(fc_dfjk* h, const double* l) {
     const uint64_t bytes = (uint64_t)h->naux * h->naux * 8;
     if (!h->l_chol) {
         FC_TRY(pool_reserve(bytes));
-        FC_CUDA(cudaMalloc(&h->l_chol, bytes));
+        FC_CUDA(spare_malloc((void**)&h->l_chol, bytes));
         h->bytes += bytes;
         ctx().handle_bytes += bytes;
     }

@@ -228,7 +228,7 @@ fc_status dfk_prepare_split(fc_dfjk* h, cudaStream_t st) {
     const size_t bytes = rup((int64_t)sbytes, 256) + scl;
     if (rows > INT32_MAX || 3 * nkb * rows > INT32_MAX) return fail(FC_ERR_LAYOUT, "DF-K: naux*n too large");
     FC_TRY(pool_reserve(bytes));
-    FC_CUDA(cudaMalloc(&h->sq_split, bytes));
+    FC_CUDA(spare_malloc(&h->sq_split, bytes));
     h->bytes += bytes;
     h->sq_scale = (double*)((char*)h->sq_split + rup((int64_t)sbytes, 256));
     dfk_split_b_kblk_kernel<<<(unsigned)rows, 256, 0, st>>>(h->b_sq, h->n, nkb, rows, h->sq_scale,

@@ -78,6 +78,14 @@ enum WsSlot {
     WS_DSLAB,      // MP2 densities: amplitude slabs (t and Tt)
     WS_DPART,      // MP2 densities: row scales, partial tiles, work items
     WS_DSTORE,     // MP2 densities: FP32 amplitude blocks kept for a later column chunk
+    // FP64 products through residues (mgemm.cuh).  Spare memory: a later
+    // ws_get that would not fit otherwise gives these back, so a call takes
+    // them after every other slot it uses.
+    WS_MG_A,       // residues of one operand
+    WS_MG_B,       // residues of the other operand
+    WS_MG_T,       // residues of an intermediate (amplitudes)
+    WS_MG_SCR,     // residues of the GEMM's tiles in flight
+    WS_MG_MISC,    // scales, partial norms, tile lists
     WS_COUNT
 };
 
@@ -103,6 +111,14 @@ uint64_t ws_bytes();
 // FC_ERR_POOL_FULL before allocating when the cap would be exceeded.
 fc_status ws_get(int slot, size_t bytes, void** out);
 fc_status pool_reserve(uint64_t bytes);  // handle allocation check
+// cudaMalloc for memory outside the slots (handles): gives the residue slots
+// back and tries again where the device is full.
+cudaError_t spare_malloc(void** p, size_t bytes);
+// Slots of at least need[k] bytes for WS_MG_A + k (0: not used), or false,
+// with nothing allocated, where they would take more than half of what the
+// pool cap or the device has left: the caller then takes its other path.
+constexpr int WS_MG_SLOTS = WS_MG_MISC - WS_MG_A + 1;
+bool ws_get_mg(const size_t (&need)[WS_MG_SLOTS], void* (&out)[WS_MG_SLOTS]);
 cudaStream_t pick_stream(void* s);
 // At least 2*n timing events (created on first use, kept by the context).
 fc_status timing_events(int n, cudaEvent_t** out);

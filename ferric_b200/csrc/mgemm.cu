@@ -1,0 +1,547 @@
+// Residue conversion kernels and the tcgen05 GEMM of mgemm.cuh.
+#include <algorithm>
+#include <cmath>
+
+#include "mgemm.cuh"
+#include "tc.cuh"
+#include "tmap.cuh"
+
+namespace fc {
+
+namespace {
+
+// The largest 15 pairwise coprime integers up to 256 (greedily).
+constexpr int MOD[MG_N] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 197};
+
+constexpr int symmod(int64_t x, int p) {
+    int64_t r = x % p;
+    if (r < 0) r += p;
+    return (int)(2 * r > p ? r - p : r);
+}
+// 256^b mod p for b = 0..7, symmetric (a signed byte: 256^0 mod 256 = 1, the
+// others 0), four to a word
+constexpr uint32_t coef(int p, int word) {
+    uint32_t w = 0;
+    int64_t v = 1;
+    for (int b = 0; b < 8; ++b) {
+        const int c = symmod(v, p);
+        if (b / 4 == word) w |= (uint32_t)(c & 255) << (8 * (b % 4));
+        v = (v * 256) % p;
+    }
+    return w;
+}
+constexpr int64_t powmod2(int e, int p) {
+    int64_t v = 1 % p;
+    for (int k = 0; k < e; ++k) v = v * 2 % p;
+    return v;
+}
+constexpr int MAGIC = 0x4B400000;  // bits of 1.5 2^23: MAGIC + v are those of 1.5 2^23 + v, |v| < 2^22
+constexpr int OFF_EXP = 60;        // integers are shifted by 2^60 to be positive
+
+// (P / MOD[l])^-1 mod MOD[l]
+constexpr int crt_inv(int l) {
+    int64_t q = 1;
+    for (int m = 0; m < MG_N; ++m)
+        if (m != l) q = q * MOD[m] % MOD[l];
+    for (int i = 1; i < MOD[l]; ++i)
+        if (q * i % MOD[l] == 1) return i;
+    return 0;
+}
+
+// The remainder theorem in fractions: x / P = sum_l s_l / p_l (mod 1), s_l =
+// r_l inv_l.  Two moduli a, b at a time: (s_a p_b + s_b p_a) / (p_a p_b) with
+// an integer numerator below 2^25; 1 / (p_a p_b) = fh + fl, fh a multiple of
+// 2^-40, so the sum of the numerators times fh is exact in FP64 and loses its
+// integer part exactly.  MG_N is odd: the last one stands alone.
+constexpr int NPAIR = (MG_N + 1) / 2;
+struct Crt {
+    uint32_t wa[NPAIR], wb[NPAIR];
+    double fh[NPAIR], fl[NPAIR];
+    double ph, pl;  // P = ph + pl
+};
+constexpr Crt make_crt() {
+    Crt c{};
+    for (int k = 0; k < NPAIR; ++k) {
+        const int a = 2 * k, b = 2 * k + 1;
+        const int64_t pa = MOD[a], pb = b < MG_N ? MOD[b] : 1;
+        c.wa[k] = (uint32_t)(crt_inv(a) * pb);
+        c.wb[k] = b < MG_N ? (uint32_t)(crt_inv(b) * pa) : 0u;
+        const int64_t q = (int64_t(1) << 40) / (pa * pb), r = (int64_t(1) << 40) % (pa * pb);
+        c.fh[k] = (double)q / 1099511627776.0;
+        c.fl[k] = (double)r / (double)(pa * pb) / 1099511627776.0;
+    }
+    unsigned __int128 P = 1;
+    for (int l = 0; l < MG_N; ++l) P *= (unsigned)MOD[l];
+    // top 53 bits and the rest
+    const unsigned __int128 top = (P >> 65) << 65;
+    c.ph = (double)(uint64_t)(P >> 65) * 36893488147419103232.0;  // 2^65; P < 2^118: 53 bits
+    const unsigned __int128 rest = P - top;
+    c.pl = (double)(uint64_t)(rest >> 33) * 8589934592.0;  // 2^33 (what is left is below 2^-85 P)
+    return c;
+}
+static_assert(make_crt().ph > 1.6615e35 && make_crt().ph < 3.3231e35, "P lies in [2^117, 2^118)");
+__constant__ Crt c_crt = make_crt();
+
+// floor(c / p) = (c * m) >> 38 with m = floor(2^38 / p) + 1 for 0 <= c < 2^30;
+// for -2^30 < c < 0 it is one less where p divides c, which leaves the residue
+// p instead of 0.
+struct ModTab {
+    int m[MG_N], p[MG_N];
+};
+constexpr ModTab make_modtab() {
+    ModTab t{};
+    for (int l = 0; l < MG_N; ++l) {
+        t.m[l] = (int)((int64_t(1) << 38) / MOD[l] + (MOD[l] == 256 ? 0 : 1));
+        t.p[l] = MOD[l];
+    }
+    return t;
+}
+__constant__ ModTab c_mod = make_modtab();
+
+__device__ __forceinline__ int dp4a_us(uint32_t a, uint32_t b, int c) {
+    int d;
+    asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
+
+// The residue (low byte, two's complement, |r| <= p / 2) of the integer whose
+// shifted form is hi:lo: the bytes' weighted sum v (|v| < 2^18.1) in two
+// dp4a, then v - p rint(v / p); v / p is at least 1 / (2 p) away from a tie,
+// the FP32 quotient within 2^-13.
+template <int L>
+__device__ __forceinline__ uint32_t residue(uint32_t lo, uint32_t hi) {
+    constexpr int p = MOD[L];
+    constexpr uint32_t cl = coef(p, 0), ch = coef(p, 1);
+    constexpr int init = MAGIC + symmod(-powmod2(OFF_EXP, p), p);
+    constexpr float inv = 1.0f / (float)p;
+    const int b = dp4a_us(hi, ch, dp4a_us(lo, cl, init));
+    const float t = __fmaf_rn(__int_as_float(b) - 12582912.0f, inv, 12582912.0f);
+    return (uint32_t)(b - __float_as_int(t) * p);
+}
+
+template <int L>
+__device__ __forceinline__ void store_residues(const uint32_t (&lo)[16], const uint32_t (&hi)[16], int8_t* dst,
+                                               int64_t plane) {
+    if constexpr (L < MG_N) {
+        uint32_t w[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint32_t a = __byte_perm(residue<L>(lo[4 * q], hi[4 * q]), residue<L>(lo[4 * q + 1], hi[4 * q + 1]),
+                                           0x0040);
+            const uint32_t b = __byte_perm(residue<L>(lo[4 * q + 2], hi[4 * q + 2]),
+                                           residue<L>(lo[4 * q + 3], hi[4 * q + 3]), 0x0040);
+            w[q] = __byte_perm(a, b, 0x5410);
+        }
+        *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+        store_residues<L + 1>(lo, hi, dst + plane, plane);
+    }
+}
+
+// 16 consecutive k of one operand row: x(i) -> residues at dst (16-byte
+// aligned), planes `plane` bytes apart.
+template <class F>
+__device__ __forceinline__ void convert16(const F& x, double inv_scale, int8_t* dst, int64_t plane) {
+    uint32_t lo[16], hi[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        const long long v = __double2ll_rn(x(i) * inv_scale) + (1ll << OFF_EXP);
+        lo[i] = (uint32_t)v;
+        hi[i] = (uint32_t)((unsigned long long)v >> 32);
+    }
+    store_residues<0>(lo, hi, dst, plane);
+}
+
+// Scale of a row with squared norm n2: the power of two s with
+// n2 / s^2 in (2^114.7, 2^116.7].
+__device__ __forceinline__ double mg_scale(double n2, int* bad) {
+    if (n2 == 0.0) return 1.0;
+    if (!(n2 >= 1e-200 && n2 <= 1e200)) {  // also NaN
+        *bad = 1;
+        return 1.0;
+    }
+    int k;
+    const double f = frexp(n2, &k);  // n2 = f 2^k, f in [0.5, 1)
+    int e = (116 - k) >> 1;          // n2 4^e < 2^116
+    const int up = k + 2 * (e + 1);  // n2 4^(e+1) = f 2^up, up = 117 or 118
+    if (up == 117 && f <= 0.8122) ++e;  // 0.8122 2^117 < 2^116.7
+    return ldexp(1.0, -e);
+}
+
+constexpr int ROWS_PER_CTA = 8;
+
+// One warp per row: its 2-norm, in a fixed order, and its scale.
+__global__ void __launch_bounds__(256) mg_row_scale_kernel(const double* __restrict__ x, int64_t ld, int64_t R,
+                                                           int64_t K, double* __restrict__ scale, int* bad) {
+    const int64_t r = (int64_t)blockIdx.x * ROWS_PER_CTA + (threadIdx.x >> 5);
+    if (r >= R) return;
+    const int lane = threadIdx.x & 31;
+    const double* row = x + r * ld;
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    int64_t k = lane;
+    for (; k + 96 < K; k += 128) {
+        double v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = row[k + 32 * u];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) s[u] += v[u] * v[u];
+    }
+    for (; k < K; k += 32) s[0] += row[k] * row[k];
+    const double n2 = warp_sum((s[0] + s[1]) + (s[2] + s[3]));
+    if (lane == 0) scale[r] = mg_scale(n2, bad);
+}
+
+// Partial squared norms of the columns over 256 rows each.
+__global__ void __launch_bounds__(256) mg_col_part_kernel(const double* __restrict__ x, int64_t ld, int64_t R,
+                                                          int64_t K, double* __restrict__ part) {
+    const int64_t c = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    if (c >= R) return;
+    const int64_t k0 = (int64_t)blockIdx.y * 256, k1 = k0 + 256 < K ? k0 + 256 : K;
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    int64_t k = k0;
+    for (; k + 3 < k1; k += 4) {
+        double v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = x[(k + u) * ld + c];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) s[u] += v[u] * v[u];
+    }
+    for (; k < k1; ++k) s[0] += x[k * ld + c] * x[k * ld + c];
+    part[(int64_t)blockIdx.y * R + c] = (s[0] + s[1]) + (s[2] + s[3]);
+}
+
+__global__ void __launch_bounds__(256) mg_col_scale_kernel(const double* __restrict__ part, int64_t R, int64_t nch,
+                                                           double* __restrict__ scale, int* bad) {
+    const int64_t c = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    if (c >= R) return;
+    double s = 0.0;
+    for (int64_t y = 0; y < nch; ++y) s += part[y * R + c];
+    scale[c] = mg_scale(s, bad);
+}
+
+// Rows of x -> residues.  A warp takes 512 k of one row: coalesced loads into
+// its shared-memory strip (one double of padding per 16, so the 16 k a lane
+// then reads lie in other banks than its neighbours'), 16 bytes of each plane
+// per lane.  Bound by the integer pipes: about 100 instructions per element.
+__global__ void __launch_bounds__(256) mg_rows_kernel(const double* __restrict__ x, int64_t ld, int64_t R, int64_t K,
+                                                      int64_t kp, const double* __restrict__ scale,
+                                                      int8_t* __restrict__ out) {
+    __shared__ double sm[8][512 + 32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t segs = (kp + 511) / 512;
+    const int64_t id = (int64_t)blockIdx.x * 8 + warp;
+    if (id >= R * segs) return;
+    const int64_t r = id / segs, k0 = (id % segs) * 512;
+    const double* row = x + r * ld;
+    double* s = sm[warp];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        const int k = i * 32 + lane;
+        s[k + (k >> 4)] = k0 + k < K ? row[k0 + k] : 0.0;
+    }
+    __syncwarp();
+    const int64_t kk = k0 + lane * 16;
+    if (kk >= kp) return;
+    const double* mine = s + lane * 17;
+    convert16([&](int i) { return mine[i]; }, 1.0 / scale[r], out + r * kp + kk, R * kp);
+}
+
+// Columns of x (K x R) -> residues: a CTA takes 32 columns by 128 k through
+// shared memory (columns rotated by 4 per 16 k against bank conflicts).
+__global__ void __launch_bounds__(256) mg_cols_kernel(const double* __restrict__ x, int64_t ld, int64_t R, int64_t K,
+                                                      int64_t kp, const double* __restrict__ scale,
+                                                      int8_t* __restrict__ out) {
+    __shared__ double sm[128 * 32];
+    const int64_t c0 = (int64_t)blockIdx.x * 32, k0 = (int64_t)blockIdx.y * 128;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        const int idx = i * 256 + threadIdx.x, k = idx >> 5, c = idx & 31;
+        sm[k * 32 + ((c + 4 * (k >> 4)) & 31)] = k0 + k < K && c0 + c < R ? x[(k0 + k) * ld + c0 + c] : 0.0;
+    }
+    __syncthreads();
+    const int c = threadIdx.x >> 3, kg = threadIdx.x & 7;
+    if (c0 + c >= R) return;
+    const double* mine = sm + kg * 16 * 32 + ((c + 4 * kg) & 31);
+    convert16([&](int i) { return mine[i * 32]; }, 1.0 / scale[c0 + c], out + (c0 + c) * kp + k0 + kg * 16, R * kp);
+}
+
+// ------------------------------------------------------------------ GEMM --
+
+constexpr int S = 4;
+constexpr int A_BYTES = MG_BM * MG_KT, B_BYTES = MG_BN * MG_KT;  // 16 + 32 KiB
+constexpr int STAGE = A_BYTES + B_BYTES;
+constexpr int SMEM = S * STAGE + 1024 + 256;
+constexpr int EPI_WARPS = 8;
+constexpr int EPI_THREADS = 32 * EPI_WARPS;
+constexpr int THREADS = 64 + EPI_THREADS;
+constexpr uint32_t IDESC = tc::idesc_i8_s32(MG_BM, MG_BN);
+constexpr size_t CTA_SCRATCH = (size_t)MG_N * MG_BM * MG_BN;
+
+struct MgArgs {
+    const int4* items;  // (tm, tn, first k-step, k-steps | split << 20)
+    int64_t nitems;
+    int M, N, planeM, planeN;
+    const double* sm;  // scales of the rows of A, B
+    const double* sn;
+    MgOut o;
+    uint4* scratch;
+    int* err;
+};
+
+// Persistent: a CTA takes tiles of 128 x 256; per tile it runs the 15 moduli
+// one after another, each over all of K, into one of two 256-column TMEM
+// accumulators, so the epilogue of one modulus overlaps the products of the
+// next.  The epilogue reduces the int32 sums modulo p and parks the residue
+// bytes of the tile (480 KiB per CTA, in L2) until the last modulus is done;
+// then each thread reads its own bytes back and forms the FP64 results.
+// Lanes are consecutive m, so stores to out[n * ld + m] are coalesced.
+__global__ void __launch_bounds__(THREADS, 1)
+    mg_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const MgArgs p) {
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t raw_u32 = smem_u32(smem_raw);
+    const uint32_t base_u32 = (raw_u32 + 1023u) & ~1023u;
+    uint8_t* base = smem_raw + (base_u32 - raw_u32);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(base + S * STAGE);
+    uint64_t* full = bars;
+    uint64_t* empty = bars + S;
+    uint64_t* tfull = bars + 2 * S;       // [2]
+    uint64_t* tempty = bars + 2 * S + 2;  // [2]
+    uint64_t* drain = bars + 2 * S + 4;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * S + 5);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {
+        for (int s = 0; s < S; ++s) {
+            tc::mbar_init(&full[s], 1);
+            tc::mbar_init(&empty[s], 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            tc::mbar_init(&tfull[b], 1);
+            tc::mbar_init(&tempty[b], EPI_THREADS);
+        }
+        tc::mbar_init(drain, 1);
+        *abort_flag = 0;
+        tc::fence_barrier_init();
+    }
+    if (warp == 0 && lane == 0) {
+        tc::prefetch_tmap(&tmA);
+        tc::prefetch_tmap(&tmB);
+    }
+    if (warp == 1) {
+        tc::tmem_alloc(tmem_slot, 512);
+        tc::tmem_relinquish();
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
+    const uint32_t tmem_base = *tmem_slot;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            uint32_t g = 0;
+            for (int64_t t = blockIdx.x; t < p.nitems && !*abort_flag; t += gridDim.x) {
+                const int4 it = p.items[t];
+                const int nk = it.w & 0xfffff;
+                for (int l = 0; l < MG_N; ++l)
+                    for (int kt = 0; kt < nk; ++kt, ++g) {
+                        const int s = g % S;
+                        if (!tc::mbar_wait(&empty[s], ((g / S) & 1) ^ 1, abort_flag, p.err)) goto prod_done;
+                        tc::mbar_arrive_expect_tx(&full[s], STAGE);
+                        uint8_t* st = base + s * STAGE;
+                        tc::tma_load_2d(st, &tmA, &full[s], (it.z + kt) * MG_KT, l * p.planeM + it.x * MG_BM);
+                        tc::tma_load_2d(st + A_BYTES, &tmB, &full[s], (it.z + kt) * MG_KT, l * p.planeN + it.y * MG_BN);
+                    }
+            }
+        prod_done:
+            // the loads in flight land before the CTA leaves
+            for (uint32_t q = 0; q < (uint32_t)S && q < g; ++q) {
+                const uint32_t gg = g - 1 - q;
+                int no_abort = 0;
+                tc::mbar_wait(&full[gg % S], (gg / S) & 1, &no_abort, p.err);
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            uint32_t g = 0, c = 0;
+            for (int64_t t = blockIdx.x; t < p.nitems && !*abort_flag; t += gridDim.x) {
+                const int nk = p.items[t].w & 0xfffff;
+                for (int l = 0; l < MG_N; ++l, ++c) {
+                    const uint32_t b = c & 1;
+                    if (!tc::mbar_wait(&tempty[b], ((c >> 1) & 1) ^ 1, abort_flag, p.err)) goto mma_done;
+                    tc::fence_after_sync();
+                    for (int kt = 0; kt < nk; ++kt, ++g) {
+                        const int s = g % S;
+                        if (!tc::mbar_wait(&full[s], (g / S) & 1, abort_flag, p.err)) goto mma_done;
+                        tc::fence_after_sync();
+                        const uint64_t da = tc::sdesc_k128(base_u32 + s * STAGE);
+                        const uint64_t db = tc::sdesc_k128(base_u32 + s * STAGE + A_BYTES);
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            tc::umma_i8(tmem_base + b * 256, da + 2 * k, db + 2 * k, IDESC, (kt | k) != 0);
+                        tc::umma_commit(&empty[s]);
+                    }
+                    tc::umma_commit(&tfull[b]);
+                }
+            }
+        mma_done:
+            tc::umma_commit(drain);
+            int no_abort = 0;
+            tc::mbar_wait(drain, 0, &no_abort, p.err);
+        }
+        __syncwarp();
+    } else {
+        const int q = warp & 3, h = (warp - 2) >> 2;
+        const int row = q * 32 + lane;
+        const int et = tid - 64;
+        uint4* scr = p.scratch + (int64_t)blockIdx.x * (CTA_SCRATCH / 16) + et;
+        const uint32_t tl0 = tmem_base + ((uint32_t)(q * 32) << 16) + h * 128;
+        uint32_t c = 0;
+        bool ok = true;
+        for (int64_t t = blockIdx.x; t < p.nitems && ok; t += gridDim.x) {
+            const int4 it = p.items[t];
+            for (int l = 0; l < MG_N; ++l, ++c) {
+                const uint32_t b = c & 1;
+                if (!tc::mbar_wait(&tfull[b], (c >> 1) & 1, abort_flag, p.err)) {
+                    ok = false;
+                    break;
+                }
+                tc::fence_after_sync();
+                const int m = c_mod.m[l], pp = c_mod.p[l];
+#pragma unroll
+                for (int cg = 0; cg < 4; ++cg) {
+                    float v[32];
+                    tc::tmem_ld32(tl0 + b * 256 + cg * 32, v);
+                    tc::tmem_wait_ld();
+                    uint32_t w[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        uint32_t r[4];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const int x = __float_as_int(v[4 * j + u]);
+                            r[u] = (uint32_t)(x - (__mulhi(x, m) >> 6) * pp);
+                        }
+                        w[j] = __byte_perm(__byte_perm(r[0], r[1], 0x0040), __byte_perm(r[2], r[3], 0x0040), 0x5410);
+                    }
+                    __stcg(scr + (l * 8 + 2 * cg) * EPI_THREADS, make_uint4(w[0], w[1], w[2], w[3]));
+                    __stcg(scr + (l * 8 + 2 * cg + 1) * EPI_THREADS, make_uint4(w[4], w[5], w[6], w[7]));
+                }
+                tc::fence_before_sync();
+                tc::mbar_arrive(&tempty[b]);
+            }
+            if (!ok) break;
+            const int m = it.x * MG_BM + row;
+            const bool vm = m < p.M;
+            const double sr = vm ? p.o.alpha * p.sm[m] : 0.0;
+            double* o = p.o.out + (int64_t)(it.w >> 20) * p.o.split_stride + m;
+#pragma unroll 1
+            for (int cg = 0; cg < 8; ++cg) {
+                const int n0 = it.y * MG_BN + h * 128 + cg * 16;
+                if (n0 >= p.N) break;
+                uint32_t w[MG_N][4];
+#pragma unroll
+                for (int l = 0; l < MG_N; ++l) {
+                    const uint4 x = __ldcg(scr + (l * 8 + cg) * EPI_THREADS);
+                    w[l][0] = x.x;
+                    w[l][1] = x.y;
+                    w[l][2] = x.z;
+                    w[l][3] = x.w;
+                }
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    double hi = 0.0, lo = 0.0;
+#pragma unroll
+                    for (int k = 0; k < NPAIR; ++k) {
+                        const uint32_t ra = __byte_perm(w[2 * k][j / 4], 0, 0x4440 + j % 4);
+                        uint32_t v = ra * c_crt.wa[k];
+                        if (2 * k + 1 < MG_N) v += __byte_perm(w[2 * k + 1][j / 4], 0, 0x4440 + j % 4) * c_crt.wb[k];
+                        const double d = __hiloint2double(0x43300000, (int)v) - 4503599627370496.0;
+                        hi = __fma_rn(d, c_crt.fh[k], hi);
+                        lo = __fma_rn(d, c_crt.fl[k], lo);
+                    }
+                    const double t0 = (hi - ((hi + 6755399441055744.0) - 6755399441055744.0)) + lo;
+                    const double x = __fma_rn(t0, c_crt.pl, t0 * c_crt.ph);
+                    const int n = n0 + j;
+                    if (vm && n < p.N) {
+                        const double y = x * sr * p.sn[n];
+                        double* d = o + (int64_t)n * p.o.ld;
+                        *d = p.o.accumulate ? *d + y : y;
+                    }
+                }
+            }
+        }
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
+    if (warp == 1) {
+        __syncwarp();
+        tc::tmem_dealloc(tmem_base, 512);
+    }
+}
+
+}  // namespace
+
+fc_status mg_convert_rows(const double* src, int64_t ld, int64_t R, int64_t K, MgOperand* o, int* bad,
+                          cudaStream_t st) {
+    o->rows = o->plane = R;
+    o->K = K;
+    o->kp = mg_kp(K);
+    mg_row_scale_kernel<<<(unsigned)((R + ROWS_PER_CTA - 1) / ROWS_PER_CTA), 256, 0, st>>>(src, ld, R, K, o->scale,
+                                                                                           bad);
+    const int64_t work = R * ((o->kp + 511) / 512);
+    mg_rows_kernel<<<(unsigned)((work + 7) / 8), 256, 0, st>>>(src, ld, R, K, o->kp, o->scale, o->r);
+    return check_launch("residue conversion (rows)");
+}
+
+fc_status mg_convert_cols(const double* src, int64_t ld, int64_t R, int64_t K, MgOperand* o, double* part, int* bad,
+                          cudaStream_t st) {
+    o->rows = o->plane = R;
+    o->K = K;
+    o->kp = mg_kp(K);
+    const int64_t nch = mg_colchunks(K);
+    mg_col_part_kernel<<<dim3((unsigned)((R + 255) / 256), (unsigned)nch), 256, 0, st>>>(src, ld, R, K, part);
+    mg_col_scale_kernel<<<(unsigned)((R + 255) / 256), 256, 0, st>>>(part, R, nch, o->scale, bad);
+    mg_cols_kernel<<<dim3((unsigned)((R + 31) / 32), (unsigned)(o->kp / 128)), 256, 0, st>>>(src, ld, R, K, o->kp,
+                                                                                            o->scale, o->r);
+    return check_launch("residue conversion (columns)");
+}
+
+int64_t mg_tiles(int64_t M, int64_t N, int64_t K, bool upper, int splits, std::vector<int4>* items) {
+    const int ntm = (int)((M + MG_BM - 1) / MG_BM), ntn = (int)((N + MG_BN - 1) / MG_BN);
+    const int nks = (int)(mg_kp(K) / MG_KT), kps = (nks + splits - 1) / splits;
+    constexpr int GM = 16;  // 16 x 9 tiles in flight: 2048 x 2304 of the product
+    const size_t n0 = items->size();
+    for (int s = 0; s * kps < nks; ++s)
+        for (int g = 0; g < ntm; g += GM)
+            for (int tn = 0; tn < ntn; ++tn)
+                for (int tm = g; tm < std::min(ntm, g + GM); ++tm) {
+                    if (upper && (int64_t)tm * MG_BM + MG_BM - 1 < (int64_t)tn * MG_BN) continue;
+                    items->push_back(make_int4(tm, tn, s * kps, std::min(kps, nks - s * kps) | (s << 20)));
+                }
+    return (int64_t)(items->size() - n0);
+}
+
+size_t mg_scratch_bytes() { return CTA_SCRATCH * (size_t)ctx().sm_count; }
+
+fc_status mg_gemm(const MgOperand& A, const MgOperand& B, const MgOut& out, const int4* items, int64_t nitems,
+                  void* scratch, int* err, cudaStream_t st) {
+    static std::atomic<uint64_t> done{0};
+    uint64_t bit = 0;
+    if (attrs_needed(done, &bit)) {
+        FC_CUDA(cudaFuncSetAttribute(mg_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
+        done.fetch_or(bit);
+    }
+    if (A.kp != B.kp || A.K > MG_KMAX || MG_N * std::max(A.plane, B.plane) + MG_BN > INT32_MAX) return fail(FC_ERR_LAYOUT, "residue GEMM: K differs or is too large");
+    CUtensorMap ta, tb;
+    FC_TRY(make_tmap_i8_2d(&ta, A.r, A.kp, (uint64_t)(MG_N - 1) * A.plane + A.rows, A.kp, MG_KT, MG_BM));
+    FC_TRY(make_tmap_i8_2d(&tb, B.r, B.kp, (uint64_t)(MG_N - 1) * B.plane + B.rows, B.kp, MG_KT, MG_BN));
+    const MgArgs a{items,   nitems,  (int)A.rows, (int)B.rows, (int)A.plane, (int)B.plane,
+                   A.scale, B.scale, out, (uint4*)scratch, err};
+    const int grid = (int)std::min<int64_t>(nitems, ctx().sm_count);
+    if (grid > 0)
+        mg_gemm_kernel<<<grid, THREADS, SMEM, st>>>(ta, tb, a);
+    return check_launch("mg_gemm_kernel");
+}
+
+}  // namespace fc

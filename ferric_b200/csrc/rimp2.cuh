@@ -59,6 +59,12 @@ fc_status rimp2_grad_f64(const Rimp2Dev& d, cudaStream_t st, double* e_os, doubl
                          double* gamma, double* de_docc, double* de_dvir, fc_stats* stats,
                          const GammaSink* sink = nullptr, const DensOut* dens = nullptr);
 
+// FP64 through residues on the int8 tensor cores (rimp2_mod.cu): where it
+// pays, and the calls; *ran = false asks for the DMMA form.
+bool mod_grad_pays(int64_t naux, int64_t nocc, int64_t nvir);
+fc_status rimp2_grad_mod(const Rimp2Dev& d, cudaStream_t st, double* e_os, double* e_ss, double* gamma,
+                         double* de_docc, double* de_dvir, fc_stats* stats, const GammaSink* sink, bool* ran);
+
 // Tensor-core (tcgen05) kernel sets.  _fx: int8 integer slices with exact
 // int32 accumulation (FC_PREC_MIXED).  _mixed: floating bf16 hi+lo split, 3
 // products, FP32 accumulation (FC_PREC_MIXED_FAST; energy only).

@@ -399,6 +399,12 @@ fc_status rimp2_grad_f64(const Rimp2Dev& d, cudaStream_t st, double* e_os, doubl
                          const GammaSink* sink, const DensOut* dens) {
     FC_TRY(set_smem_once());
     if (dens && d.nshards != 1) return fail(FC_ERR_INVALID, "RI-MP2 densities: no sharded form");
+    // shards keep the DMMA form's partition of the chunk pairs (fc_rimp2_shard_pairs)
+    if (!dens && d.nshards == 1 && mod_grad_pays(d.naux, d.nocc, d.nvir)) {
+        bool ran = false;
+        FC_TRY(rimp2_grad_mod(d, st, e_os, e_ss, gamma, de_docc, de_dvir, stats, sink, &ran));
+        if (ran) return FC_OK;
+    }
     const int64_t nocc = d.nocc, nvir = d.nvir, naux = d.naux, nov = nocc * nvir;
     const int ntile = (int)((nvir + PR_T - 1) / PR_T);
     const int ntile2 = ntile * ntile;  // every tile (ta, tb) of a pair, ta-major
