@@ -173,4 +173,35 @@ __device__ __forceinline__ double block_sum(double v, double* sh /* >= 32 */) {
     return t;
 }
 
+// Deterministic compensated block sum (blockDim.x a multiple of 32, <= 1024):
+// the threads' sums and corrections merge in a fixed tree, five shuffles and
+// one pass over the warps, so a CTA's sum costs about 2 us; one thread adding
+// 1024 partials in turn took 38.  Thread 0 gets the result.
+__device__ __forceinline__ KSum ksum_warp(KSum a) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const double s = __shfl_down_sync(0xffffffffu, a.s, o), c = __shfl_down_sync(0xffffffffu, a.c, o);
+        a.add(s);
+        a.c += c;
+    }
+    return a;
+}
+
+__device__ __forceinline__ double block_ksum(KSum a, double2* sh /* >= 32 */) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    a = ksum_warp(a);
+    __syncthreads();
+    if (lane == 0) sh[warp] = make_double2(a.s, a.c);
+    __syncthreads();
+    if (warp == 0) {
+        a = KSum{};
+        if (lane < (int)(blockDim.x >> 5)) {
+            a.s = sh[lane].x;
+            a.c = sh[lane].y;
+        }
+        a = ksum_warp(a);
+    }
+    return a.value();
+}
+
 }  // namespace fc

@@ -237,23 +237,16 @@ __global__ void __launch_bounds__(256, 2) pair_f64_kernel(PairArgs p) {
 // Fixed-order compensated sum of n (os, ss) partials -> out[0..1].
 __global__ void __launch_bounds__(1024) reduce_pairs_kernel(const double* __restrict__ part,
                                                             int64_t n, double* out) {
-    __shared__ double so[1024], sss[1024];
+    __shared__ double2 sh[32];
     KSum a, b;
     for (int64_t k = threadIdx.x; k < n; k += 1024) {
         a.add(part[2 * k]);
         b.add(part[2 * k + 1]);
     }
-    so[threadIdx.x] = a.value();
-    sss[threadIdx.x] = b.value();
-    __syncthreads();
+    const double va = block_ksum(a, sh), vb = block_ksum(b, sh);
     if (threadIdx.x == 0) {
-        KSum x, y;
-        for (int k = 0; k < 1024; ++k) {
-            x.add(so[k]);
-            y.add(sss[k]);
-        }
-        out[0] = x.value();
-        out[1] = y.value();
+        out[0] = va;
+        out[1] = vb;
     }
 }
 
@@ -264,7 +257,7 @@ __global__ void __launch_bounds__(256) reduce_occ_kernel(const double* __restric
                                                          const int2* __restrict__ pairs, int64_t npairs,
                                                          int ntile2, int i0, int ni, int j0,
                                                          double* acc_occ) {
-    __shared__ double sh[256];
+    __shared__ double2 sh[32];
     const int o = (int)blockIdx.x < ni ? i0 + (int)blockIdx.x : j0 + ((int)blockIdx.x - ni);
     KSum a;
     const int64_t n = npairs * ntile2;
@@ -273,13 +266,8 @@ __global__ void __launch_bounds__(256) reduce_occ_kernel(const double* __restric
         if (pr.x == o) a.add(occ_part[2 * k]);
         else if (pr.y == o) a.add(occ_part[2 * k + 1]);
     }
-    sh[threadIdx.x] = a.value();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        KSum x;
-        for (int k = 0; k < 256; ++k) x.add(sh[k]);
-        acc_occ[o] += x.value();
-    }
+    const double v = block_ksum(a, sh);
+    if (threadIdx.x == 0) acc_occ[o] += v;
 }
 
 __global__ void scale_copy_f64_kernel(const double* __restrict__ x, int64_t n, double s, double* __restrict__ y) {

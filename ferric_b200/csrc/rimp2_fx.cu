@@ -267,28 +267,43 @@ __global__ void __launch_bounds__(256) split_pair4_kernel(const double* __restri
 }
 
 // gd[i*a_pad + a] = sum_q B[q, ia]^2 in FP64 (fixed order), the exact
-// (ia|ia) of the pair kernel's i == j blocks, for the columns ia in [c0, c0+cols)
-// of B (row pitch ld).  One thread per column; rows in one pass.
+// (ia|ia) of the pair kernel's i == j blocks, for the columns ia of B (row
+// pitch ld).  A CTA takes 32 columns, eight warps the rows r = warp (mod 8), so
+// a few thousand columns fill the chip (with a thread per column over all rows
+// 12201 columns x 1036 rows took 147 us, 48 CTAs in a chain of loads).
+// Threads without a column pass B = nullptr.
 __device__ __forceinline__ void colsq_body(const double* __restrict__ B, int64_t rows, int64_t nvir, int64_t ld,
                                            int64_t a_pad, int64_t c, double* __restrict__ gd) {
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-    int64_t r = 0;
-    for (; r + 4 <= rows; r += 4) {
-        const double v0 = B[r * ld + c], v1 = B[(r + 1) * ld + c], v2 = B[(r + 2) * ld + c], v3 = B[(r + 3) * ld + c];
-        s0 = fma(v0, v0, s0);
-        s1 = fma(v1, v1, s1);
-        s2 = fma(v2, v2, s2);
-        s3 = fma(v3, v3, s3);
+    __shared__ double sh[8][32];
+    const int g = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    if (B) {
+        const double* x = B + c;
+        int64_t r = g;
+        for (; r + 24 < rows; r += 32) {
+            double v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) v[u] = x[(r + 8 * u) * ld];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) s[u] = fma(v[u], v[u], s[u]);
+        }
+        for (; r < rows; r += 8) s[0] = fma(x[r * ld], x[r * ld], s[0]);
     }
-    for (; r < rows; ++r) s0 = fma(B[r * ld + c], B[r * ld + c], s0);
-    gd[(c / nvir) * a_pad + c % nvir] = (s0 + s1) + (s2 + s3);
+    sh[g][lane] = (s[0] + s[1]) + (s[2] + s[3]);
+    __syncthreads();
+    if (g == 0 && B) {
+        double t = 0.0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) t += sh[k][lane];
+        gd[(c / nvir) * a_pad + c % nvir] = t;
+    }
 }
 
 __global__ void __launch_bounds__(256) colsq_kernel(const double* __restrict__ B, int64_t rows, int64_t nvir,
                                                     int64_t ld, int64_t a_pad, int64_t c0, int64_t c1,
                                                     double* __restrict__ gd) {
-    const int64_t c = c0 + (int64_t)blockIdx.x * 256 + threadIdx.x;
-    if (c < c1) colsq_body(B, rows, nvir, ld, a_pad, c, gd);
+    const int64_t c = c0 + (int64_t)blockIdx.x * 32 + (threadIdx.x & 31);
+    colsq_body(c < c1 ? B : nullptr, rows, nvir, ld, a_pad, c, gd);
 }
 
 __global__ void fill_kernel(double* __restrict__ x, int64_t n, double v) {
@@ -1384,23 +1399,16 @@ __global__ void __launch_bounds__(GF_THREADS, 1)
 
 __global__ void __launch_bounds__(1024) fx_reduce_pairs_kernel(const double* __restrict__ part, int64_t n,
                                                                double* out) {
-    __shared__ double so[1024], sss[1024];
+    __shared__ double2 sh[32];
     KSum a, b;
     for (int64_t k = threadIdx.x; k < n; k += 1024) {
         a.add(part[2 * k]);
         b.add(part[2 * k + 1]);
     }
-    so[threadIdx.x] = a.value();
-    sss[threadIdx.x] = b.value();
-    __syncthreads();
+    const double va = block_ksum(a, sh), vb = block_ksum(b, sh);
     if (threadIdx.x == 0) {
-        KSum x, y;
-        for (int k = 0; k < 1024; ++k) {
-            x.add(so[k]);
-            y.add(sss[k]);
-        }
-        out[0] = x.value();
-        out[1] = y.value();
+        out[0] = va;
+        out[1] = vb;
     }
 }
 
@@ -1410,7 +1418,7 @@ __global__ void __launch_bounds__(256) fx_reduce_occ_kernel(const double* __rest
                                                             const int2* __restrict__ pairs, int64_t npairs,
                                                             int ntiles, int i0, int ni, int j0,
                                                             double* acc_occ) {
-    __shared__ double sh[256];
+    __shared__ double2 sh[32];
     const int o = (int)blockIdx.x < ni ? i0 + (int)blockIdx.x : j0 + ((int)blockIdx.x - ni);
     KSum a;
     const int64_t n = npairs * ntiles;
@@ -1418,13 +1426,8 @@ __global__ void __launch_bounds__(256) fx_reduce_occ_kernel(const double* __rest
         const int2 pr = pairs[k / ntiles];
         if (pr.x == o || pr.y == o) a.add(occ_part[k]);
     }
-    sh[threadIdx.x] = a.value();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        KSum x;
-        for (int k = 0; k < 256; ++k) x.add(sh[k]);
-        acc_occ[o] += x.value();
-    }
+    const double v = block_ksum(a, sh);
+    if (threadIdx.x == 0) acc_occ[o] += v;
 }
 
 __global__ void scale_copy_kernel(const double* __restrict__ x, int64_t n, double s, double* __restrict__ y) {
@@ -1536,11 +1539,11 @@ __global__ void __launch_bounds__(256) batch_transpose_kernel(const BatchPrep* _
 
 __global__ void __launch_bounds__(256) batch_colsq_kernel(const BatchPrep* __restrict__ mp,
                                                           const int64_t* __restrict__ pre, int nmol) {
-    const int64_t x = (int64_t)blockIdx.x * 256 + threadIdx.x;
-    if (x >= pre[nmol]) return;
-    const int m = seg_find(pre, 0, nmol, x);
+    const int64_t n = pre[nmol];
+    const int64_t x = (int64_t)blockIdx.x * 32 + (threadIdx.x & 31);
+    const int m = seg_find(pre, 0, nmol, x < n ? x : n - 1);
     const BatchPrep& d = mp[m];
-    colsq_body(d.b, d.naux, d.nvir, d.nocc * d.nvir, d.a_pad, x - pre[m], d.gd);
+    colsq_body(x < n ? d.b : nullptr, d.naux, d.nvir, d.nocc * d.nvir, d.a_pad, x - pre[m], d.gd);
 }
 
 __global__ void __launch_bounds__(256) batch_qrows_kernel(const BatchPrep* __restrict__ mp,
@@ -1566,7 +1569,7 @@ __global__ void __launch_bounds__(256) batch_trows_kernel(const BatchPrep* __res
 __global__ void __launch_bounds__(256) batch_occ_kernel(const BatchPrep* __restrict__ mp,
                                                         const int64_t* __restrict__ pre, int m0, int m1,
                                                         const double* __restrict__ occ_part) {
-    __shared__ double sh[256];
+    __shared__ double2 sh[32];
     const int64_t x = pre[m0] + blockIdx.x;
     const int m = seg_find(pre, m0, m1, x);
     const BatchPrep& d = mp[m];
@@ -1578,13 +1581,8 @@ __global__ void __launch_bounds__(256) batch_occ_kernel(const BatchPrep* __restr
         const int64_t pidx = i * n - i * (i - 1) / 2 + (j - i);
         a.add(occ_part[d.seg0 + pidx * d.ntp + t]);
     }
-    sh[threadIdx.x] = a.value();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        KSum t;
-        for (int k = 0; k < 256; ++k) t.add(sh[k]);
-        d.de_docc[o] = -2.0 * t.value();
-    }
+    const double v = block_ksum(a, sh);
+    if (threadIdx.x == 0) d.de_docc[o] = -2.0 * v;
 }
 
 // dE/deps_v = 2 sum of the row-virtual partials of v (v in the a-tile) and
@@ -1618,24 +1616,17 @@ __global__ void __launch_bounds__(256) batch_vir_kernel(const BatchPrep* __restr
 __global__ void __launch_bounds__(256) batch_energy_kernel(const double* __restrict__ part,
                                                            const int64_t* __restrict__ seg, int m0,
                                                            double* out) {
-    __shared__ double so[256], sn[256];
+    __shared__ double2 sh[32];
     const int m = m0 + blockIdx.x;
     KSum a, b;
     for (int64_t k = seg[m] + threadIdx.x; k < seg[m + 1]; k += 256) {
         a.add(part[2 * k]);
         b.add(part[2 * k + 1]);
     }
-    so[threadIdx.x] = a.value();
-    sn[threadIdx.x] = b.value();
-    __syncthreads();
+    const double va = block_ksum(a, sh), vb = block_ksum(b, sh);
     if (threadIdx.x == 0) {
-        KSum x, y;
-        for (int t = 0; t < 256; ++t) {
-            x.add(so[t]);
-            y.add(sn[t]);
-        }
-        out[2 * m] = x.value();
-        out[2 * m + 1] = y.value();
+        out[2 * m] = va;
+        out[2 * m + 1] = vb;
     }
 }
 
@@ -1692,7 +1683,7 @@ fc_status fx_split_range(const Rimp2Dev& d, cudaStream_t st, int* bad, const FxS
         dim3 g((unsigned)((nc + 255) / 256), (unsigned)((d.naux + rps - 1) / rps));
         colmax_kernel<<<g, 256, 0, st>>>(d.b_ov, d.naux, nc, rps, o.cmax, bad, nov, c0);
     }
-    colsq_kernel<<<(unsigned)((nc + 255) / 256), 256, 0, st>>>(d.b_ov, d.naux, d.nvir, nov, o.a_pad, c0, c0 + nc,
+    colsq_kernel<<<(unsigned)((nc + 31) / 32), 256, 0, st>>>(d.b_ov, d.naux, d.nvir, nov, o.a_pad, c0, c0 + nc,
                                                                o.gd);
     const int64_t r0 = o0 * o.a_pad, r1 = o1 * o.a_pad;
     row_scale_kernel<SliceI8><<<(unsigned)((r1 - r0 + 255) / 256), 256, 0, st>>>(o.cmax, d.nocc, d.nvir, o.a_pad,
@@ -2676,7 +2667,7 @@ fc_status rimp2_batch_build_fx(fc_rimp2_batch* b, const std::vector<BatchMolIn>&
         batch_row_scale_kernel<<<(unsigned)((P(PRE_ROWSCALE, nmol) + 255) / 256), 256, 0, st>>>(
             dp, PD(PRE_ROWSCALE), nmol);
         batch_transpose_kernel<<<(unsigned)P(PRE_TRANSPOSE, nmol), 256, 0, st>>>(dp, PD(PRE_TRANSPOSE), nmol);
-        batch_colsq_kernel<<<(unsigned)((P(PRE_COLSQ, nmol) + 255) / 256), 256, 0, st>>>(dp, PD(PRE_COLSQ), nmol);
+        batch_colsq_kernel<<<(unsigned)((P(PRE_COLSQ, nmol) + 31) / 32), 256, 0, st>>>(dp, PD(PRE_COLSQ), nmol);
         launches += 4;
         if (grad) {
             batch_qrows_kernel<<<(unsigned)P(PRE_QROWS, nmol), 256, 0, st>>>(dp, PD(PRE_QROWS), nmol);

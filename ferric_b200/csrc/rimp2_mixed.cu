@@ -337,23 +337,16 @@ __global__ void __launch_bounds__(192, 1)
 
 __global__ void __launch_bounds__(1024) reduce_parts_kernel(const double* __restrict__ part, int64_t n,
                                                             double* out) {
-    __shared__ double so[1024], sss[1024];
+    __shared__ double2 sh[32];
     KSum a, b;
     for (int64_t k = threadIdx.x; k < n; k += 1024) {
         a.add(part[2 * k]);
         b.add(part[2 * k + 1]);
     }
-    so[threadIdx.x] = a.value();
-    sss[threadIdx.x] = b.value();
-    __syncthreads();
+    const double va = block_ksum(a, sh), vb = block_ksum(b, sh);
     if (threadIdx.x == 0) {
-        KSum x, y;
-        for (int k = 0; k < 1024; ++k) {
-            x.add(so[k]);
-            y.add(sss[k]);
-        }
-        out[0] = x.value();
-        out[1] = y.value();
+        out[0] = va;
+        out[1] = vb;
     }
 }
 
