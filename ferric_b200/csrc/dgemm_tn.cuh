@@ -6,66 +6,89 @@
 // (Gamma = 4 B_ov Tt^T), the DF-K half-transform and rank update, the MP2
 // densities and the RI response products.
 //
-// Tile 128 x 64 x 16, 8 warps (4 x 2), each warp 32 x 32 = 4 x 4 DMMA tiles;
+// Tile BM x BN x 16 (128 x 64 where nothing else is said; narrower ones for
+// products whose M or N would leave most of that empty), 8 warps (4 x 2);
 // 3-stage cp.async pipeline; split-K over blockIdx.z.  Shared-memory rows are
 // padded to 20 doubles so the fragment reads (g*20 + t) hit distinct banks.
+// A K-major operand whose rows start on 16 bytes is copied 16 bytes at a time
+// (half the copy instructions), any other 8.
 #pragma once
+#include <type_traits>
+
 #include "dmma.cuh"
 
 namespace fc {
 
 constexpr int DG_BM = 128, DG_BN = 64, DG_BK = 16, DG_LDK = 20, DG_STAGES = 3;
-constexpr int DG_SMEM = DG_STAGES * (DG_BM + DG_BN) * DG_LDK * 8;
+constexpr int dg_smem(int bm, int bn) { return DG_STAGES * (bm + bn) * DG_LDK * 8; }
+constexpr int DG_SMEM = dg_smem(DG_BM, DG_BN);
 
 // The tile body.  A(m, k) = TA ? A[k*lda + m] : A[m*lda + k], and B(n, k) the
 // same with TB: a transposed (MN-major) operand is read with consecutive
 // threads on consecutive m (n), so its global loads stay coalesced.  The
 // epilogue gets `z` (the split or the batch index).
-template <class Epi, bool TA, bool TB>
+template <class Epi, bool TA, bool TB, int BM = DG_BM, int BN = DG_BN>
 __device__ __forceinline__ void dgemm_tile(const double* __restrict__ A, int64_t lda, const double* __restrict__ B,
                                            int64_t ldb, int M, int N, int64_t kbeg, int64_t kend, int upper_only,
                                            const Epi& epi, int z) {
-    extern __shared__ __align__(16) double dg_smem[];
-    double* sA = dg_smem;                                   // [STAGES][BM][LDK]
-    double* sB = dg_smem + DG_STAGES * DG_BM * DG_LDK;      // [STAGES][BN][LDK]
+    static_assert(BM % 32 == 0 && BN % 16 == 0, "4 x 2 warps of 8 x 8 DMMA tiles");
+    constexpr int MT = BM / 32, NT = BN / 16;  // DMMA tiles per warp
+    extern __shared__ __align__(16) double dg_smem_buf[];
+    double* sA = dg_smem_buf;                               // [STAGES][BM][LDK]
+    double* sB = dg_smem_buf + DG_STAGES * BM * DG_LDK;     // [STAGES][BN][LDK]
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
     const int wm = warp & 3, wn = warp >> 2;
-    const int m0 = blockIdx.y * DG_BM, n0 = blockIdx.x * DG_BN;
-    if (upper_only && m0 > n0 + DG_BN - 1) return;  // tile strictly below the diagonal
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    if (upper_only && m0 > n0 + BN - 1) return;  // tile strictly below the diagonal
     if (kbeg >= kend) return;
     const int nk = (int)((kend - kbeg + DG_BK - 1) / DG_BK);
+    const bool va = !TA && !(((uintptr_t)A & 15) | (uintptr_t)(lda & 1) | (uintptr_t)(kbeg & 1));
+    const bool vb = !TB && !(((uintptr_t)B & 15) | (uintptr_t)(ldb & 1) | (uintptr_t)(kbeg & 1));
 
-    auto load = [&](int stage, int kt) {
-        const int64_t kb = kbeg + (int64_t)kt * DG_BK;
-        double* a = sA + stage * DG_BM * DG_LDK;
-        double* b = sB + stage * DG_BN * DG_LDK;
+    // rows [r0, r0 + ROWS) of a K-major operand (R rows), 16 bytes a copy
+    auto load16 = [&](double* s, const double* X, int64_t ld, int r0, int R, int64_t kb, auto rows) {
+        constexpr int ROWS = decltype(rows)::value;
 #pragma unroll
-        for (int e = 0; e < (DG_BM * DG_BK) / 256; ++e) {
-            const int idx = tid + 256 * e;
-            const int row = TA ? idx % DG_BM : idx >> 4, kk = TA ? idx / DG_BM : idx & 15;
-            const int gm = m0 + row;
-            const int64_t gk = kb + kk;
-            const bool ok = gm < M && gk < kend;
-            cp_async8(a + row * DG_LDK + kk, ok ? (TA ? A + gk * lda + gm : A + (int64_t)gm * lda + gk) : A, ok);
-        }
-#pragma unroll
-        for (int e = 0; e < (DG_BN * DG_BK) / 256; ++e) {
-            const int idx = tid + 256 * e;
-            const int row = TB ? idx % DG_BN : idx >> 4, kk = TB ? idx / DG_BN : idx & 15;
-            const int gn = n0 + row;
-            const int64_t gk = kb + kk;
-            const bool ok = gn < N && gk < kend;
-            cp_async8(b + row * DG_LDK + kk, ok ? (TB ? B + gk * ldb + gn : B + (int64_t)gn * ldb + gk) : B, ok);
+        for (int e = 0; e < (ROWS * DG_BK / 2 + 255) / 256; ++e) {
+            const int idx = tid + 256 * e, row = idx >> 3, kk = (idx & 7) * 2, gr = r0 + row;
+            if (row >= ROWS) break;
+            const int64_t left = kend - (kb + kk);
+            const int bytes = gr < R && left > 0 ? (left > 1 ? 16 : 8) : 0;
+            cp_async16n(s + row * DG_LDK + kk, bytes ? X + (int64_t)gr * ld + kb + kk : X, bytes);
         }
     };
+    auto load8 = [&](double* s, const double* X, int64_t ld, int r0, int R, int64_t kb, auto rows, auto trans) {
+        constexpr int ROWS = decltype(rows)::value;
+        constexpr bool T = decltype(trans)::value;
+#pragma unroll
+        for (int e = 0; e < ROWS * DG_BK / 256; ++e) {
+            const int idx = tid + 256 * e;
+            const int row = T ? idx % ROWS : idx >> 4, kk = T ? idx / ROWS : idx & 15;
+            const int gr = r0 + row;
+            const int64_t gk = kb + kk;
+            const bool ok = gr < R && gk < kend;
+            cp_async8(s + row * DG_LDK + kk, ok ? (T ? X + gk * ld + gr : X + (int64_t)gr * ld + gk) : X, ok);
+        }
+    };
+    auto load = [&](int stage, int kt) {
+        const int64_t kb = kbeg + (int64_t)kt * DG_BK;
+        using RA = std::integral_constant<int, BM>;
+        using RB = std::integral_constant<int, BN>;
+        double* a = sA + stage * BM * DG_LDK;
+        double* b = sB + stage * BN * DG_LDK;
+        if (va) load16(a, A, lda, m0, M, kb, RA{});
+        else load8(a, A, lda, m0, M, kb, RA{}, std::integral_constant<bool, TA>{});
+        if (vb) load16(b, B, ldb, n0, N, kb, RB{});
+        else load8(b, B, ldb, n0, N, kb, RB{}, std::integral_constant<bool, TB>{});
+    };
 
-    double acc[4][4][2];
+    double acc[MT][NT][2];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < MT; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+        for (int j = 0; j < NT; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
 
 #pragma unroll
     for (int s = 0; s < DG_STAGES - 1; ++s) {
@@ -78,52 +101,53 @@ __device__ __forceinline__ void dgemm_tile(const double* __restrict__ A, int64_t
         const int pf = kt + DG_STAGES - 1;
         if (pf < nk) load(pf % DG_STAGES, pf);
         cp_async_commit();
-        const double* a = sA + (kt % DG_STAGES) * DG_BM * DG_LDK;
-        const double* b = sB + (kt % DG_STAGES) * DG_BN * DG_LDK;
+        const double* a = sA + (kt % DG_STAGES) * BM * DG_LDK;
+        const double* b = sB + (kt % DG_STAGES) * BN * DG_LDK;
 #pragma unroll
         for (int ks = 0; ks < DG_BK / 4; ++ks) {
-            double af[4], bf[4];
+            double af[MT], bf[NT];
 #pragma unroll
-            for (int mt = 0; mt < 4; ++mt) af[mt] = a[(wm * 32 + mt * 8 + g) * DG_LDK + ks * 4 + t];
+            for (int mt = 0; mt < MT; ++mt) af[mt] = a[(wm * (BM / 4) + mt * 8 + g) * DG_LDK + ks * 4 + t];
 #pragma unroll
-            for (int nt = 0; nt < 4; ++nt) bf[nt] = b[(wn * 32 + nt * 8 + g) * DG_LDK + ks * 4 + t];
+            for (int nt = 0; nt < NT; ++nt) bf[nt] = b[(wn * (BN / 2) + nt * 8 + g) * DG_LDK + ks * 4 + t];
 #pragma unroll
-            for (int mt = 0; mt < 4; ++mt)
+            for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-                for (int nt = 0; nt < 4; ++nt) dmma_8x8x4(acc[mt][nt], af[mt], bf[nt]);
+                for (int nt = 0; nt < NT; ++nt) dmma_8x8x4(acc[mt][nt], af[mt], bf[nt]);
         }
     }
     cp_async_wait<0>();
 
 #pragma unroll
-    for (int mt = 0; mt < 4; ++mt)
+    for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt)
+        for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const int m = m0 + wm * 32 + mt * 8 + g;
-                const int n = n0 + wn * 32 + nt * 8 + 2 * t + h;
+                const int m = m0 + wm * (BM / 4) + mt * 8 + g;
+                const int n = n0 + wn * (BN / 2) + nt * 8 + 2 * t + h;
                 if (m < M && n < N) epi(m, n, acc[mt][nt][h], z);
             }
 }
 
-template <class Epi, bool TA = false, bool TB = false>
+template <class Epi, bool TA = false, bool TB = false, int BM = DG_BM, int BN = DG_BN>
 __global__ void __launch_bounds__(256) dgemm_tn_kernel(const double* __restrict__ A, int64_t lda,
                                                        const double* __restrict__ B, int64_t ldb,
                                                        int M, int N, int64_t K, int64_t k_per_split,
-                                                       int upper_only, Epi epi) {
+                                                       int upper_only, Epi epi, const int* run_if = nullptr) {
+    if (run_if && !(run_if[0] | run_if[1])) return;  // the residue form's result stands (mgemm.cuh)
     const int64_t kbeg = (int64_t)blockIdx.z * k_per_split;
     const int64_t kend = kbeg + k_per_split < K ? kbeg + k_per_split : K;
-    dgemm_tile<Epi, TA, TB>(A, lda, B, ldb, M, N, kbeg, kend, upper_only, epi, (int)blockIdx.z);
+    dgemm_tile<Epi, TA, TB, BM, BN>(A, lda, B, ldb, M, N, kbeg, kend, upper_only, epi, (int)blockIdx.z);
 }
 
 // Batched over blockIdx.z: operands z * sa and z * sb elements on, all of K.
 template <class Epi, bool TA = false, bool TB = false>
 __global__ void __launch_bounds__(256) dgemm_batched_kernel(const double* __restrict__ A, int64_t lda, int64_t sa,
                                                             const double* __restrict__ B, int64_t ldb, int64_t sb,
-                                                            int M, int N, int64_t K, Epi epi) {
+                                                            int M, int N, int64_t K, Epi epi, int upper_only = 0) {
     const int z = (int)blockIdx.z;
-    dgemm_tile<Epi, TA, TB>(A + z * sa, lda, B + z * sb, ldb, M, N, 0, K, 0, epi, z);
+    dgemm_tile<Epi, TA, TB>(A + z * sa, lda, B + z * sb, ldb, M, N, 0, K, upper_only, epi, z);
 }
 
 // value * alpha -> C[m*ldc + n]
@@ -135,6 +159,15 @@ struct EpiStore {
     __device__ __forceinline__ void operator()(int m, int n, double v, int) const {
         double* c = C + (int64_t)m * ldc + n;
         *c = accumulate ? *c + alpha * v : alpha * v;
+    }
+};
+
+// v -> C[z stride + m ldc + n]
+struct EpiBatchStore {
+    double* C;
+    int64_t ldc, stride;
+    __device__ __forceinline__ void operator()(int m, int n, double v, int z) const {
+        C[(int64_t)z * stride + (int64_t)m * ldc + n] = v;
     }
 };
 

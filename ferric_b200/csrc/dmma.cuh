@@ -35,6 +35,12 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src, bool vali
                  "r"(n));
 }
 
+// 16 bytes of which the first n (0, 8 or 16) are read and the rest are zero.
+__device__ __forceinline__ void cp_async16n(void* dst, const void* src, int n) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_u32(dst)), "l"(src),
+                 "r"(n));
+}
+
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 
 template <int N>

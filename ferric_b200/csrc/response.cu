@@ -25,15 +25,6 @@ namespace fc {
 
 namespace {
 
-// v -> C[z stride + m ldc + n]
-struct EpiBatchStore {
-    double* C;
-    int64_t ldc, stride;
-    __device__ __forceinline__ void operator()(int m, int n, double v, int z) const {
-        C[(int64_t)z * stride + (int64_t)m * ldc + n] = v;
-    }
-};
-
 // out[P][mu][nu] = w (G[P][mu][nu] + G[P][nu][mu])
 __global__ void __launch_bounds__(256) sym_slab_kernel(const double* __restrict__ g, int64_t np, int64_t n, double w,
                                                        double* __restrict__ out) {

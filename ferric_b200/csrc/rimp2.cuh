@@ -63,7 +63,12 @@ fc_status rimp2_grad_f64(const Rimp2Dev& d, cudaStream_t st, double* e_os, doubl
 // pays, and the calls; *ran = false asks for the DMMA form.
 bool mod_grad_pays(int64_t naux, int64_t nocc, int64_t nvir);
 fc_status rimp2_grad_mod(const Rimp2Dev& d, cudaStream_t st, double* e_os, double* e_ss, double* gamma,
-                         double* de_docc, double* de_dvir, fc_stats* stats, const GammaSink* sink, bool* ran);
+                         double* de_docc, double* de_dvir, fc_stats* stats, const GammaSink* sink,
+                         const DensOut* dens, bool* ran);
+// Energies: rows x cols products over naux (one spin: nov x nov / 2).
+bool mod_energy_pays(int64_t naux, int64_t rows, int64_t cols);
+fc_status rimp2_energy_mod(const Rimp2Dev& d, cudaStream_t st, double* e_os, double* e_ss, fc_stats* stats,
+                           bool* ran);
 
 // Tensor-core (tcgen05) kernel sets.  _fx: int8 integer slices with exact
 // int32 accumulation (FC_PREC_MIXED).  _mixed: floating bf16 hi+lo split, 3
@@ -116,9 +121,10 @@ struct DensF64 {
     double* ts;       // [nocc nvir][ld]
     double* as;       // [nocc nvir][ld]
     double* part_oo;  // [splits][nocc x nocc]
+    double* part_vv;  // [gvv][nvir x nvir]
     double* acc_vv;   // [nvir x nvir] running P_vv (upper tiles)
     double* acc_oo;   // [nocc x nocc] running P_oo
-    int splits;
+    int splits, gvv;
 };
 int64_t dens_chunk_f64(int64_t nocc, int64_t nvir, int64_t cc, int64_t budget);
 fc_status dens_f64_alloc(int64_t nocc, int64_t nvir, int64_t cc, cudaStream_t st, DensF64* o);
@@ -138,6 +144,9 @@ struct UmpSpin {
     const double* eps_vir;  // [nvir]
     int64_t nocc, nvir;
 };
+// Every component of an unrestricted energy through residues (rimp2_mod.cu).
+fc_status ump2_energy_mod(const UmpSpin& a, const UmpSpin& b, int64_t naux, int64_t budget, cudaStream_t st,
+                          double* e_aa, double* e_bb, double* e_ab, fc_stats* stats, bool* ran);
 // Opposite-spin energy sum_{i a J B} (ia|JB)^2 / D: FP64 DMMA, or exact
 // slices on tcgen05.
 fc_status ump2_cross_f64(const UmpSpin& a, const UmpSpin& b, int64_t naux, cudaStream_t st, double* e_ab,

@@ -310,6 +310,11 @@ fc_status rimp2_energy_f64(const Rimp2Dev& d, cudaStream_t st, double* e_os, dou
                            fc_stats* stats) {
     FC_TRY(set_smem_once());
     const int64_t nocc = d.nocc, nvir = d.nvir;
+    if (d.nshards == 1 && mod_energy_pays(d.naux, nocc * nvir, (nocc * nvir + 1) / 2)) {
+        bool ran = false;
+        FC_TRY(rimp2_energy_mod(d, st, e_os, e_ss, stats, &ran));
+        if (ran) return FC_OK;
+    }
     const int ntile = (int)((nvir + PR_T - 1) / PR_T);
     const int ntiles = ntile * (ntile + 1) / 2;  // tiles ta <= tb
     int64_t plo, phi;  // this shard's pairs (all of them unsharded)
@@ -388,9 +393,9 @@ fc_status rimp2_grad_f64(const Rimp2Dev& d, cudaStream_t st, double* e_os, doubl
     FC_TRY(set_smem_once());
     if (dens && d.nshards != 1) return fail(FC_ERR_INVALID, "RI-MP2 densities: no sharded form");
     // shards keep the DMMA form's partition of the chunk pairs (fc_rimp2_shard_pairs)
-    if (!dens && d.nshards == 1 && mod_grad_pays(d.naux, d.nocc, d.nvir)) {
+    if (d.nshards == 1 && mod_grad_pays(d.naux, d.nocc, d.nvir)) {
         bool ran = false;
-        FC_TRY(rimp2_grad_mod(d, st, e_os, e_ss, gamma, de_docc, de_dvir, stats, sink, &ran));
+        FC_TRY(rimp2_grad_mod(d, st, e_os, e_ss, gamma, de_docc, de_dvir, stats, sink, dens, &ran));
         if (ran) return FC_OK;
     }
     const int64_t nocc = d.nocc, nvir = d.nvir, naux = d.naux, nov = nocc * nvir;

@@ -14,6 +14,7 @@
 // (about 10 bytes per element beside 4 naux flops) are a tenth of the time.
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 #include "fc_internal.cuh"
@@ -24,8 +25,10 @@ namespace fc {
 
 namespace {
 
-constexpr int AT = 64;               // virtuals per side of an amplitude tile
+constexpr int AT = 32;               // virtuals per side of an amplitude tile
+constexpr int AN = 128;              // threads of its CTA
 constexpr int AP = AT + 1;           // pitch in shared memory
+constexpr int AE = AT * AT / AN;      // elements per thread
 constexpr int AMP_SMEM = 3 * AT * AP * 8;
 enum AmpMode { AMP_ENERGY, AMP_GRAD, AMP_CROSS };
 
@@ -46,9 +49,10 @@ struct AmpArgs {
 // One (pair, tile pair) per CTA: the tiles (a in ta, b in tb) and (b, a) of
 // the pair's block, so each element meets its exchange partner.  Gradient
 // mode writes Tt over G (and its transpose when I == J, whose lower part the
-// GEMM leaves out).  Bound by its reads and writes of g.
+// GEMM leaves out).  Bound by its reads and writes of g, given enough CTAs in
+// flight: tiles of 64 x 64 (two CTAs per SM) ran at 1.7 TB/s.
 template <int MODE>
-__global__ void __launch_bounds__(256) amp_kernel(const AmpArgs p) {
+__global__ void __launch_bounds__(AN) amp_kernel(const AmpArgs p) {
     extern __shared__ __align__(16) double sm[];
     __shared__ double red[32];
     double* X = sm;              // X[a][b] = (ia|jb), then Tt_ij[a, b]
@@ -65,7 +69,7 @@ __global__ void __launch_bounds__(256) amp_kernel(const AmpArgs p) {
     double* gy = p.g + ((int64_t)(i - p.i0) * nva + B0) * p.ld + (int64_t)(j - p.j0) * nvb + A0;
     // each thread keeps its columns' loads together
 #pragma unroll 4
-    for (int e = tid; e < AT * AT; e += 256) {
+    for (int e = tid; e < AT * AT; e += AN) {
         const int r = e / AT, c = e % AT;
         if (r < na && c < nb) X[r * AP + c] = gx[(int64_t)r * p.ld + c];
         if (MODE != AMP_CROSS && off && !dia && r < nb && c < na) Y[r * AP + c] = gy[(int64_t)r * p.ld + c];
@@ -78,10 +82,10 @@ __global__ void __launch_bounds__(256) amp_kernel(const AmpArgs p) {
     const int b = tid % AT;
     const bool vb = b < nb;
     const double eb = vb ? (MODE == AMP_CROSS ? p.ev2 : p.ev)[B0 + b] : 0.0;
-    double t1[AT / 4], t2[AT / 4];
+    double t1[AE], t2[AE];
 #pragma unroll
-    for (int k = 0; k < AT / 4; ++k) {
-        const int a = tid / AT + 4 * k;
+    for (int k = 0; k < AE; ++k) {
+        const int a = tid / AT + (AN / AT) * k;
         t1[k] = t2[k] = 0.0;
         double s = 0.0;
         if (vb && a < na) {
@@ -125,8 +129,8 @@ __global__ void __launch_bounds__(256) amp_kernel(const AmpArgs p) {
     }
     if constexpr (MODE == AMP_GRAD) {
 #pragma unroll
-        for (int k = 0; k < AT / 4; ++k) {
-            const int a = tid / AT + 4 * k;
+        for (int k = 0; k < AE; ++k) {
+            const int a = tid / AT + (AN / AT) * k;
             X[a * AP + b] = t1[k];
             if (off) Y[b * AP + a] = t2[k];
         }
@@ -146,7 +150,7 @@ __global__ void __launch_bounds__(256) amp_kernel(const AmpArgs p) {
         double* my = p.g + ((int64_t)(j - p.j0) * nva + A0) * p.ld + (int64_t)(i - p.i0) * nva + B0;
         const bool mir = p.same && i != j;
 #pragma unroll 4
-        for (int e = tid; e < AT * AT; e += 256) {
+        for (int e = tid; e < AT * AT; e += AN) {
             const int r = e / AT, c = e % AT;
             if (r < na && c < nb) {
                 gx[(int64_t)r * p.ld + c] = X[r * AP + c];
@@ -206,12 +210,13 @@ __global__ void __launch_bounds__(256) amp_fold_kernel(const double* __restrict_
 constexpr int VP = 32;
 __global__ void __launch_bounds__(256) amp_vir_part_kernel(const double* __restrict__ vir, int64_t npairs, int ntile,
                                                            double* __restrict__ out) {
-    __shared__ double sh[4][AT];
+    constexpr int G = 256 / AT;
+    __shared__ double sh[G][AT];
     const int t = blockIdx.x, r = threadIdx.x % AT, g = threadIdx.x / AT;
     const int ntiles = ntile * (ntile + 1) / 2;
     const int64_t x0 = (int64_t)blockIdx.y * VP, x1 = min(x0 + VP, npairs);
     KSum s;
-    for (int64_t x = x0 + g; x < x1; x += 4)
+    for (int64_t x = x0 + g; x < x1; x += G)
         for (int u = 0; u < ntile; ++u) {
             // tile (min, max) in the row-major list of ta <= tb
             const int lo = min(t, u), hi = max(t, u);
@@ -220,8 +225,11 @@ __global__ void __launch_bounds__(256) amp_vir_part_kernel(const double* __restr
         }
     sh[g][r] = s.value();
     __syncthreads();
-    if (g == 0)
-        out[((int64_t)blockIdx.y * ntile + t) * AT + r] = (sh[0][r] + sh[1][r]) + (sh[2][r] + sh[3][r]);
+    if (g == 0) {
+        double v = 0.0;
+        for (int k = 0; k < G; ++k) v += sh[k][r];
+        out[((int64_t)blockIdx.y * ntile + t) * AT + r] = v;
+    }
 }
 
 // de_dvir[a] += 2 sum over the chunks, one warp per 32 virtuals and eight
@@ -293,7 +301,8 @@ bool mod_grad_pays(int64_t naux, int64_t nocc, int64_t nvir) {
 // Returns FC_OK with *ran = false where the caller has to take the DMMA form
 // (no room for the residues, or operand rows out of range).
 fc_status rimp2_grad_mod(const Rimp2Dev& d, cudaStream_t st, double* e_os, double* e_ss, double* gamma,
-                         double* de_docc, double* de_dvir, fc_stats* stats, const GammaSink* sink, bool* ran) {
+                         double* de_docc, double* de_dvir, fc_stats* stats, const GammaSink* sink,
+                         const DensOut* dens, bool* ran) {
     *ran = false;
     FC_TRY(amp_attrs());
     const int64_t nocc = d.nocc, nvir = d.nvir, naux = d.naux, nov = nocc * nvir;
@@ -305,6 +314,8 @@ fc_status rimp2_grad_mod(const Rimp2Dev& d, cudaStream_t st, double* e_os, doubl
     if (cc * nvir > MG_KMAX) return FC_OK;
     cc = balanced(nocc, cc);
     const int64_t nch = (nocc + cc - 1) / cc, cv = cc * nvir;
+    // the densities contract whole rows of t and Tt: one chunk, both kept
+    if (dens && (nch > 1 || dens_chunk_f64(nocc, nvir, nocc, 4 * d.chunk_bytes) < nocc)) return FC_OK;
     const int ntile = (int)((nvir + AT - 1) / AT), ntiles = ntile * (ntile + 1) / 2;
 
     std::vector<ChunkPair> cps;
@@ -350,7 +361,13 @@ fc_status rimp2_grad_mod(const Rimp2Dev& d, cudaStream_t st, double* e_os, doubl
         *items = c.take<int4>(ht.size());
     };
     void *vT, *vpairs, *vpart, *vout;
-    FC_TRY(ws_get(WS_T, (size_t)cv * cv * 8, &vT));
+    DensF64 dx{};
+    if (dens) {
+        FC_TRY(dens_f64_alloc(nocc, nvir, nocc, st, &dx));
+        vT = dx.ts;
+    } else {
+        FC_TRY(ws_get(WS_T, (size_t)cv * cv * 8, &vT));
+    }
     FC_TRY(ws_get(WS_PAIRS, hp.size() * sizeof(int2), &vpairs));
     FC_TRY(ws_get(WS_PART, (np_items * (3 + 2 * AT) + (size_t)np_max * 3 + (size_t)nvch * ntile * AT) * 8, &vpart));
     FC_TRY(ws_get(WS_OUT, (size_t)(nocc + 2) * 8 + 64, &vout));
@@ -387,7 +404,8 @@ fc_status rimp2_grad_mod(const Rimp2Dev& d, cudaStream_t st, double* e_os, doubl
     }
     MgOperand bt{(int8_t*)mg[0], bts};
     FC_TRY(mg_convert_cols(d.b_ov, nov, nov, naux, &bt, cpart, flags, st));
-    int nl = 3, nadj = 0;
+    int64_t nl = 3;
+    int nadj = 0;
     double adj_flops = 0.0, adj_bytes = 0.0;
     size_t bq_off = 0;
     std::vector<char> seen((size_t)nch, 0);
@@ -433,7 +451,7 @@ fc_status rimp2_grad_mod(const Rimp2Dev& d, cudaStream_t st, double* e_os, doubl
         a.same = cp.same();
         a.part = part;
         a.vir = virp;
-        amp_kernel<AMP_GRAD><<<dim3((unsigned)ntiles, (unsigned)cp.np), 256, AMP_SMEM, st>>>(a);
+        amp_kernel<AMP_GRAD><<<dim3((unsigned)ntiles, (unsigned)cp.np), AN, AMP_SMEM, st>>>(a);
         amp_pair_sum_kernel<<<(unsigned)((cp.np + 7) / 8), 256, 0, st>>>(part, cp.np, ntiles, psum);
         amp_fold_kernel<<<(unsigned)(1 + cp.ni + (cp.same() ? 0 : cp.nj)), 256, 0, st>>>(
             psum, a.pairs, cp.np, (int)cp.i0, (int)cp.ni, (int)cp.j0, acc, acc_occ);
@@ -453,6 +471,11 @@ fc_status rimp2_grad_mod(const Rimp2Dev& d, cudaStream_t st, double* e_os, doubl
         }
         // row I of the chunk pairs is done: Gamma's columns of chunk I are final
         if (sink && cp.j0 + cp.nj == nocc) FC_TRY(gamma_sink_block(sink, gamma, naux, nov, nvir, cp.i0, cp.ni, st));
+    }
+    if (dens) {
+        FC_TRY(dens_f64_block(dx, 0, nocc, nocc, st, &nl));
+        FC_TRY(dens_f64_slab(dx, nocc, st, &nl));
+        FC_TRY(dens_f64_finish(dx, *dens, st, &nl));
     }
     scale_to_kernel<<<(unsigned)((nocc + 255) / 256), 256, 0, st>>>(acc_occ, nocc, -2.0, de_docc);
     FC_TRY(check_launch("scale_to_kernel"));
@@ -478,7 +501,7 @@ fc_status rimp2_grad_mod(const Rimp2Dev& d, cudaStream_t st, double* e_os, doubl
         stats->kernel_ms = ms;
         stats->flops = 2.0 * naux * (double)nvir * nvir * P + 2.0 * naux * (double)nov * nov;
         stats->precision = FC_PREC_F64;
-        stats->launches += nl + nadj + 1;
+        stats->launches += (int)(nl + nadj + 1);
         stats->tile_m = MG_BM;
         stats->tile_n = MG_BN;
         stats->k_panel = 0;
@@ -492,6 +515,209 @@ fc_status rimp2_grad_mod(const Rimp2Dev& d, cudaStream_t st, double* e_os, doubl
         FC_TRY(timing_sum2(nadj, &stats->aux_ms));
         stats->aux_flops = adj_flops;
         stats->aux_bytes = adj_bytes;
+    }
+    return FC_OK;
+}
+
+// ------------------------------------------------------------- energies --
+
+// Measured at the line (B200): see DESIGN's table.
+bool mod_energy_pays(int64_t naux, int64_t rows, int64_t cols) {
+    return naux <= MG_KMAX && 2.0 * naux * (double)rows * (double)cols >= 1e9;
+}
+
+namespace {
+
+// One pair sum: the pairs i <= j of one spin (b == a), or all (i, J) of two.
+struct EnergyPass {
+    int a, b;
+    AmpMode mode;
+    int64_t c0 = 0, nc = 0;      // its row chunks
+    int ntiles = 0;
+    int64_t tiles0 = 0;          // its virtual tiles in the pair table
+};
+struct EnergyChunk {
+    int64_t i0, ni, j0, nj, p0, np, t0, nt;
+};
+
+// e[2 k], e[2 k + 1]: E_os and E_ss of pass k (cross: E_ab, 0) of the spins'
+// b_ov, converted once each.  G of a chunk of rows is formed by the residue
+// GEMM and read once by amp_kernel; chunks of at most 2 GiB.
+fc_status energy_passes(const UmpSpin* spin, int nspin, std::vector<EnergyPass>& passes, int64_t naux, int has_kappa,
+                        double kappa, int64_t budget, cudaStream_t st, double* e, fc_stats* stats, bool* ran) {
+    *ran = false;
+    FC_TRY(amp_attrs());
+    budget = std::min(budget, int64_t(2) << 30);
+    std::vector<EnergyChunk> ch;
+    std::vector<int2> hp;
+    std::vector<int4> ht;
+    size_t g_max = 0, items_max = 0;
+    int64_t np_max = 0;
+    for (EnergyPass& ps : passes) {
+        const UmpSpin &A = spin[ps.a], &B = spin[ps.b];
+        const int nta = (int)((A.nvir + AT - 1) / AT), ntb = (int)((B.nvir + AT - 1) / AT);
+        const int64_t row = A.nvir * B.nocc * B.nvir * 8;  // bytes of G per orbital of the rows
+        const int64_t ci = balanced(A.nocc, std::min(budget / row, (int64_t)65535 / B.nocc));
+        if (row > budget || B.nocc > 65535) return FC_OK;  // (the amplitude kernel's grid)
+        ps.ntiles = ps.mode == AMP_CROSS ? nta * ntb : nta * (nta + 1) / 2;
+        ps.c0 = (int64_t)ch.size();
+        for (int64_t i0 = 0; i0 < A.nocc; i0 += ci) {
+            EnergyChunk x{};
+            x.i0 = i0;
+            x.ni = std::min(ci, A.nocc - i0);
+            x.j0 = ps.mode == AMP_CROSS ? 0 : i0;
+            x.nj = B.nocc - x.j0;
+            x.p0 = (int64_t)hp.size();
+            for (int64_t i = i0; i < i0 + x.ni; ++i)
+                for (int64_t j = ps.mode == AMP_CROSS ? 0 : i; j < B.nocc; ++j)
+                    hp.push_back(make_int2((int)i, (int)j));
+            x.np = (int64_t)hp.size() - x.p0;
+            x.t0 = (int64_t)ht.size();
+            x.nt = mg_tiles(x.nj * B.nvir, x.ni * A.nvir, naux, ps.mode != AMP_CROSS, 1, &ht);
+            g_max = std::max(g_max, (size_t)(x.ni * A.nvir * x.nj * B.nvir));
+            items_max = std::max(items_max, (size_t)x.np * ps.ntiles);
+            np_max = std::max(np_max, x.np);
+            ch.push_back(x);
+        }
+        ps.nc = (int64_t)ch.size() - ps.c0;
+        ps.tiles0 = (int64_t)hp.size();
+        for (int ta = 0; ta < nta; ++ta)
+            for (int tb = ps.mode == AMP_CROSS ? 0 : ta; tb < ntb; ++tb) hp.push_back(make_int2(ta, tb));
+    }
+    int64_t rows[2] = {0, 0}, rmax = 0;
+    for (int s = 0; s < nspin; ++s) {
+        rows[s] = spin[s].nocc * spin[s].nvir;
+        rmax = std::max(rmax, rows[s]);
+    }
+    const int64_t npass = (int64_t)passes.size();
+    void *vG, *vpairs, *vpart, *vout;
+    FC_TRY(ws_get(WS_T, g_max * 8, &vG));
+    FC_TRY(ws_get(WS_PAIRS, hp.size() * sizeof(int2), &vpairs));
+    FC_TRY(ws_get(WS_PART, (items_max * 3 + (size_t)np_max * 3) * 8, &vpart));
+    FC_TRY(ws_get(WS_OUT, 256, &vout));
+    double *sc[2], *cpart;
+    int4* items;
+    auto misc = [&](Carver& c) {
+        for (int s = 0; s < 2; ++s) sc[s] = c.take<double>(rows[s]);
+        cpart = c.take<double>(mg_colpart(rmax, naux));
+        items = c.take<int4>(ht.size());
+    };
+    Carver cm;
+    misc(cm);
+    void* mg[WS_MG_SLOTS];
+    if (!ws_get_mg({mg_bytes(rows[0], naux), nspin > 1 ? mg_bytes(rows[1], naux) : 0, 0, mg_scratch_bytes(), cm.off},
+                   mg))
+        return FC_OK;
+    cm = Carver{(char*)mg[4], 0};
+    misc(cm);
+    double* G = (double*)vG;
+    double* part = (double*)vpart;
+    double* psum = part + 3 * items_max;
+    double* acc = (double*)vout;
+    int* flags = (int*)(acc + 2 * npass);
+    FC_CUDA(cudaMemcpyAsync(vpairs, hp.data(), hp.size() * sizeof(int2), cudaMemcpyHostToDevice, st));
+    FC_CUDA(cudaMemcpyAsync(items, ht.data(), ht.size() * sizeof(int4), cudaMemcpyHostToDevice, st));
+    FC_CUDA(cudaMemsetAsync(vout, 0, 256, st));
+    Context& c = ctx();
+    if (stats) FC_CUDA(cudaEventRecord(c.ev0, st));
+    MgOperand op[2] = {{(int8_t*)mg[0], sc[0]}, {(int8_t*)mg[1], sc[1]}};
+    for (int s = 0; s < nspin; ++s)
+        FC_TRY(mg_convert_cols(spin[s].b_ov, rows[s], rows[s], naux, &op[s], cpart, flags, st));
+    int nl = 3 * nspin;
+    double flops = 0.0;
+    for (int64_t k = 0; k < npass; ++k) {
+        const EnergyPass& ps = passes[(size_t)k];
+        const UmpSpin &A = spin[ps.a], &B = spin[ps.b];
+        for (int64_t q = ps.c0; q < ps.c0 + ps.nc; ++q) {
+            const EnergyChunk& x = ch[(size_t)q];
+            const int64_t ld = x.nj * B.nvir;
+            FC_TRY(mg_gemm(op[ps.b].slice(x.j0 * B.nvir, ld), op[ps.a].slice(x.i0 * A.nvir, x.ni * A.nvir),
+                           MgOut{G, ld, 0, 1.0, 0}, items + x.t0, x.nt, mg[3], flags + 1, st));
+            AmpArgs a{};
+            a.g = G;
+            a.ld = ld;
+            a.pairs = (const int2*)vpairs + x.p0;
+            a.tiles = (const int2*)vpairs + ps.tiles0;
+            a.ntiles = ps.ntiles;
+            a.i0 = (int)x.i0;
+            a.j0 = (int)x.j0;
+            a.nvir = (int)A.nvir;
+            a.nvir2 = (int)B.nvir;
+            a.eo = A.eps_occ;
+            a.ev = A.eps_vir;
+            a.eo2 = B.eps_occ;
+            a.ev2 = B.eps_vir;
+            a.same = ps.mode != AMP_CROSS;
+            a.has_kappa = has_kappa;
+            a.kappa = kappa;
+            a.part = part;
+            const dim3 grid((unsigned)ps.ntiles, (unsigned)x.np);
+            if (ps.mode == AMP_CROSS) amp_kernel<AMP_CROSS><<<grid, AN, AMP_SMEM, st>>>(a);
+            else amp_kernel<AMP_ENERGY><<<grid, AN, AMP_SMEM, st>>>(a);
+            amp_pair_sum_kernel<<<(unsigned)((x.np + 7) / 8), 256, 0, st>>>(part, x.np, ps.ntiles, psum);
+            amp_fold_kernel<<<1, 256, 0, st>>>(psum, a.pairs, x.np, 0, 0, 0, acc + 2 * k, nullptr);
+            FC_TRY(check_launch("residue energy"));
+            nl += 4;
+        }
+        const double P = ps.mode == AMP_CROSS ? (double)A.nocc * B.nocc : (double)A.nocc * (A.nocc + 1) / 2.0;
+        flops += 2.0 * naux * (double)A.nvir * B.nvir * P;
+    }
+    if (stats) FC_CUDA(cudaEventRecord(c.ev1, st));
+    double h[8];  // the sums, then the flags
+    FC_CUDA(cudaMemcpyAsync(h, acc, (2 * npass + 1) * 8, cudaMemcpyDeviceToHost, st));
+    FC_CUDA(cudaStreamSynchronize(st));
+    int hf[2];
+    std::memcpy(hf, h + 2 * npass, sizeof(hf));
+    if (hf[1]) return fail(FC_ERR_TIMEOUT, "RI-MP2 energy: a pipeline wait ran out");
+    if (hf[0]) return FC_OK;
+    *ran = true;
+    for (int64_t k = 0; k < 2 * npass; ++k) e[k] = h[k];
+    if (stats) {
+        float ms = 0.f;
+        FC_CUDA(cudaEventElapsedTime(&ms, c.ev0, c.ev1));
+        stats->kernel_ms = ms;
+        stats->flops = flops;
+        stats->precision = FC_PREC_F64;
+        stats->launches += nl;
+        stats->tile_m = MG_BM;
+        stats->tile_n = MG_BN;
+        stats->k_panel = 0;
+        stats->d2h_bytes += (2 * npass + 1) * 8;
+        stats->h2d_bytes += hp.size() * sizeof(int2) + ht.size() * sizeof(int4);
+        stats->main_launches = (int)ch.size();
+        stats->main_ms = ms;
+        stats->main_flops = flops;
+        stats->main_bytes = (double)MG_N * naux * (rows[0] + rows[1]);
+    }
+    return FC_OK;
+}
+
+}  // namespace
+
+fc_status rimp2_energy_mod(const Rimp2Dev& d, cudaStream_t st, double* e_os, double* e_ss, fc_stats* stats,
+                           bool* ran) {
+    const UmpSpin s{d.b_ov, d.eps_occ, d.eps_vir, d.nocc, d.nvir};
+    std::vector<EnergyPass> ps{{0, 0, AMP_ENERGY}};
+    double e[2] = {0.0, 0.0};
+    FC_TRY(energy_passes(&s, 1, ps, d.naux, d.has_kappa, d.kappa, d.chunk_bytes, st, e, stats, ran));
+    if (*ran) {
+        *e_os = e[0];
+        *e_ss = e[1];
+    }
+    return FC_OK;
+}
+
+fc_status ump2_energy_mod(const UmpSpin& a, const UmpSpin& b, int64_t naux, int64_t budget, cudaStream_t st,
+                          double* e_aa, double* e_bb, double* e_ab, fc_stats* stats, bool* ran) {
+    const UmpSpin s[2] = {a, b};
+    std::vector<EnergyPass> ps{{0, 0, AMP_ENERGY}, {1, 1, AMP_ENERGY}, {0, 1, AMP_CROSS}};
+    double e[6] = {};
+    FC_TRY(energy_passes(s, 2, ps, naux, 0, 0.0, budget, st, e, stats, ran));
+    if (*ran) {
+        // one spin's E_ss = 2 E_sigma-sigma (no pair where it has one orbital)
+        *e_aa = a.nocc < 2 ? 0.0 : 0.5 * e[1];
+        *e_bb = b.nocc < 2 ? 0.0 : 0.5 * e[3];
+        *e_ab = e[4];
     }
     return FC_OK;
 }

@@ -50,3 +50,46 @@ def test_gradient_rows_out_of_range(fc):
     b[3, 5] = np.inf
     sc, g, go, gv = rimp2.rimp2_energy_grad(b, eo, ev, stats=st)
     assert st["tile_n"] == 64 and not np.isfinite(sc.e_total)
+
+
+@pytest.mark.parametrize("naux,nocc,nvir,kappa", [(640, 12, 129, None), (1153, 16, 65, 1.1), (700, 1, 1300, None)])
+def test_energy_matches_oracle(fc, naux, nocc, nvir, kappa):
+    from ferric_b200 import rimp2
+    b, eo, ev = synthetic.rimp2_inputs(naux, nocc, nvir)
+    ref = orc.spin_components(b, np.concatenate([eo, ev]), nocc, nvir, kappa=kappa)
+    st = {}
+    e_os, e_ss = rimp2.rimp2_energy(b, eo, ev, kappa=kappa, stats=st)
+    assert st["tile_n"] == 256
+    # E_ss is a difference of sums of the size of E_os
+    assert abs(e_os - ref[0]) <= 1e-13 * abs(ref[0]) and abs(e_ss - ref[1]) <= 1e-13 * abs(ref[0])
+
+
+@pytest.mark.parametrize("naux,na,nva,nb,nvb", [(640, 17, 129, 15, 131), (500, 40, 66, 1, 105)])
+def test_ump2_matches_oracle(fc, naux, na, nva, nb, nvb):
+    from ferric_b200 import rimp2
+    ba, oa, va = synthetic.rimp2_inputs(naux, na, nva)
+    bb, ob, vb = synthetic.rimp2_inputs(naux, nb, nvb, seed_b=5, seed_eps=50)
+    st = {}
+    got = rimp2.ump2_energy(ba, oa, va, bb, ob, vb, stats=st)
+    assert st["tile_n"] == 256
+    # the same-spin sum is half of one spin's closed-shell E_ss
+    e_aa = 0.5 * orc.spin_components(ba, np.concatenate([oa, va]), na, nva)[1]
+    e_bb = 0.5 * orc.spin_components(bb, np.concatenate([ob, vb]), nb, nvb)[1]
+    g = (ba.T @ bb).reshape(na, nva, nb, nvb)
+    d = oa[:, None, None, None] + ob[None, None, :, None] - va[None, :, None, None] - vb[None, None, None, :]
+    e_ab = float((g * g / d).sum())
+    for x, y in zip(got, (e_aa, e_bb, e_ab)):
+        assert abs(x - y) <= 1e-13 * abs(e_ab)
+
+
+@pytest.mark.parametrize("naux,nocc,nvir", [(640, 10, 129), (513, 33, 64)])
+def test_densities_match_oracle(fc, naux, nocc, nvir):
+    from ferric_b200 import rimp2
+    b, eo, ev = synthetic.rimp2_inputs(naux, nocc, nvir)
+    st = {}
+    got = rimp2.rimp2_energy_grad_dens(b, eo, ev, stats=st)
+    assert st["tile_n"] == 256
+    _check(got[:4], orc.energy_gamma_deps(b, eo, ev))
+    t2, _ = orc.t2_and_integrals(b, eo, ev)
+    for x, y in zip(got[4:], orc.mp2_density(t2, nocc, nvir)):
+        assert np.abs(x - y).max() <= 1e-12 * np.abs(y).max()
