@@ -13,6 +13,7 @@
 #include "fc_internal.cuh"
 #include "dgemm_tn.cuh"
 #include "dfjk.cuh"
+#include "mgemm.cuh"
 
 #include <vector>
 
@@ -88,11 +89,17 @@ __global__ void __launch_bounds__(256) dfj_pass2_kernel(const TB* __restrict__ b
     if (k >= pair) return;
     double s0 = 0.0, s1 = 0.0;
     int64_t p = p0;
-    for (; p + 1 < p1; p += 2) {
-        s0 += (double)bp[p * pair + k] * c[p];
-        s1 += (double)bp[(p + 1) * pair + k] * c[p + 1];
+    for (; p + 7 < p1; p += 8) {  // eight rows' loads in flight
+        double v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = (double)bp[(p + u) * pair + k];
+#pragma unroll
+        for (int u = 0; u < 8; u += 2) {
+            s0 += v[u] * c[p + u];
+            s1 += v[u + 1] * c[p + u + 1];
+        }
     }
-    if (p < p1) s0 += (double)bp[p * pair + k] * c[p];
+    for (; p < p1; ++p) s0 += (double)bp[p * pair + k] * c[p];
     part[(int64_t)blockIdx.y * pair + k] = s0 + s1;
 }
 
@@ -323,14 +330,26 @@ struct EpiScatterW {
     }
 };
 
-__global__ void dfk_fold_kernel(const double* __restrict__ part, int nsplit, int64_t n,
-                                double* __restrict__ k) {
+// mg (optional): the residue GEMM's flags; nsplit_mg of its partials count
+// unless one is raised.
+__global__ void dfk_fold_kernel(const double* __restrict__ part, int nsplit, int64_t n, double* __restrict__ k,
+                                const int* __restrict__ mg, int nsplit_mg) {
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= n * n) return;
+    if (mg && !(mg[0] | mg[1])) nsplit = nsplit_mg;
     const int64_t r = idx / n, c = idx % n;
     const int64_t lo = r < c ? r : c, hi = r < c ? c : r;
+    const double* x = part + lo * n + hi;
     double s = 0.0;
-    for (int sp = 0; sp < nsplit; ++sp) s += part[(int64_t)sp * n * n + lo * n + hi];
+    int sp = 0;
+    for (; sp + 8 <= nsplit; sp += 8) {  // eight loads in flight, added in order
+        double v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = x[(int64_t)(sp + u) * n * n];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) s += v[u];
+    }
+    for (; sp < nsplit; ++sp) s += x[(int64_t)sp * n * n];
     k[idx] = s;
 }
 
@@ -368,6 +387,25 @@ static fc_status dfj_solve_pass2(fc_dfjk* h, const TB* bp, double* dp, double* p
     return check_launch("DF-J pass 2");
 }
 
+// Statistics of a J build whose first event has been recorded.
+static fc_status dfj_stats(const fc_dfjk* h, int prec, size_t elem, int launches, cudaStream_t st, fc_stats* stats) {
+    if (!stats) return FC_OK;
+    Context& c = ctx();
+    FC_CUDA(cudaEventRecord(c.ev1, st));
+    FC_CUDA(cudaEventSynchronize(c.ev1));
+    float ms = 0.f;
+    FC_CUDA(cudaEventElapsedTime(&ms, c.ev0, c.ev1));
+    stats->kernel_ms = ms;
+    stats->flops = 4.0 * (double)h->naux * (double)h->pair;
+    stats->precision = prec;
+    stats->launches += launches;
+    stats->main_launches = launches > 1 ? 2 : 1;
+    stats->main_ms = ms;
+    stats->main_flops = stats->flops;
+    stats->main_bytes = 2.0 * (double)elem * (double)h->naux * (double)h->pair;
+    return FC_OK;
+}
+
 template <typename TB>
 static fc_status dfj_build_t(fc_dfjk* h, const TB* bp, int prec, const double* d, double* j, cudaStream_t st,
                              fc_stats* stats) {
@@ -399,21 +437,7 @@ static fc_status dfj_build_t(fc_dfjk* h, const TB* bp, int prec, const double* d
     dfj_seg_sum_kernel<<<(unsigned)((naux + 255) / 256), 256, 0, st>>>(segp, (int)nseg, naux, dp);
     FC_TRY(dfj_solve_pass2<TB>(h, bp, dp, (double*)vpart, nsplit, j, st));
     FC_TRY(check_launch("DF-J kernels"));
-    if (stats) {
-        FC_CUDA(cudaEventRecord(c.ev1, st));
-        FC_CUDA(cudaEventSynchronize(c.ev1));
-        float ms = 0.f;
-        FC_CUDA(cudaEventElapsedTime(&ms, c.ev0, c.ev1));
-        stats->kernel_ms = ms;
-        stats->flops = 4.0 * (double)naux * (double)pair;
-        stats->precision = prec;
-        stats->launches += 5 + (h->l_chol ? 1 : 0);
-        stats->main_launches = 2;
-        stats->main_ms = ms;
-        stats->main_flops = stats->flops;
-        stats->main_bytes = 2.0 * sizeof(TB) * (double)naux * (double)pair;
-    }
-    return FC_OK;
+    return dfj_stats(h, prec, sizeof(TB), 5 + (h->l_chol ? 1 : 0), st, stats);
 }
 
 fc_status dfj_build_f64(fc_dfjk* h, const double* d, double* j, cudaStream_t st, fc_stats* stats) {
@@ -456,6 +480,28 @@ void dfjk_free_mixed(fc_dfjk* h) {
     h->sq_scale = nullptr;
 }
 
+// Statistics of an FP64 K build whose first event has been recorded.
+static fc_status dfk_stats(const fc_dfjk* h, int64_t nocc, int launches, int tile_m, int tile_n, cudaStream_t st,
+                           fc_stats* stats) {
+    if (!stats) return FC_OK;
+    Context& c = ctx();
+    FC_CUDA(cudaEventRecord(c.ev1, st));
+    FC_CUDA(cudaEventSynchronize(c.ev1));
+    float ms = 0.f;
+    FC_CUDA(cudaEventElapsedTime(&ms, c.ev0, c.ev1));
+    stats->kernel_ms = ms;
+    stats->flops = 4.0 * (double)h->naux * (double)h->n * (double)h->n * (double)nocc;
+    stats->precision = FC_PREC_F64;
+    stats->launches += launches;
+    stats->main_launches = launches > 1 ? 2 : 1;
+    stats->main_ms = ms;
+    stats->main_flops = stats->flops;
+    stats->main_bytes = 8.0 * (double)h->naux * (double)h->n * (double)h->n;
+    stats->tile_m = tile_m;
+    stats->tile_n = tile_n;
+    return FC_OK;
+}
+
 fc_status dfk_build_f64(fc_dfjk* h, const double* c_occ, int64_t nocc, double* k, cudaStream_t st,
                         fc_stats* stats, const JFork* jf) {
     FC_TRY(dfjk_smem_once());
@@ -478,7 +524,16 @@ fc_status dfk_build_f64(fc_dfjk* h, const double* c_occ, int64_t nocc, double* k
     void *vct, *vw, *vpart;
     FC_TRY(ws_get(WS_MISC, nocc * n * 8, &vct));
     FC_TRY(ws_get(WS_T, n * kdim * 8, &vw));
-    FC_TRY(ws_get(WS_PART, (int64_t)nsplit * n * n * 8, &vpart));
+    // K = W W^T through residues (mgemm.cuh) where the product is worth W's
+    // conversion: n = 600, kdim = 144000: 2.50 -> 0.95 ms; even at n = 400, kdim = 64000.
+    const bool residues = (double)n * n * kdim >= 8e9 && n <= 65535;
+    const int nsplit_mg = residues ? mg_splits(n, n, kdim, true) : 0;
+    void* vflags = nullptr;
+    FC_TRY(ws_get(WS_PART, (int64_t)std::max(nsplit, nsplit_mg) * n * n * 8, &vpart));
+    if (residues) {
+        FC_TRY(ws_get(WS_OUT, 256, &vflags));
+        FC_CUDA(cudaMemsetAsync(vflags, 0, 256, st));
+    }
     Context& c = ctx();
     if (stats) FC_CUDA(cudaEventRecord(c.ev0, st));
     transpose_kernel<<<(unsigned)((n * nocc + 255) / 256), 256, 0, st>>>(c_occ, n, nocc, (double*)vct);
@@ -502,35 +557,27 @@ fc_status dfk_build_f64(fc_dfjk* h, const double* c_occ, int64_t nocc, double* k
         dfj_d_sum_kernel<<<(unsigned)((naux + 255) / 256), 256, 0, st>>>(jf->dpart, naux, jf->dp);
         FC_TRY(dfj_fork_pass2(h, *jf, st));
     }
-    {
+    bool room = false;
+    if (residues) {
+        const MgSrc w{(const double*)vw, kdim, n, false};
+        FC_TRY(mg_multiply(w, w, kdim, MgOut{(double*)vpart, n, n * n, 1.0, 0}, true, nsplit_mg, (int*)vflags, st,
+                           &room));
+    }
+    const int* mg = room ? (const int*)vflags : nullptr;
+    {  // every CTA leaves at once where the residue product stands
         dim3 g(tn, tm, nsplit);
         EpiSplit epi{(double*)vpart, n * n, (int)n};
         dgemm_tn_kernel<EpiSplit><<<g, 256, DG_SMEM, st>>>((const double*)vw, kdim, (const double*)vw, kdim,
-                                                            (int)n, (int)n, kdim, kps, 1, epi);
+                                                            (int)n, (int)n, kdim, kps, 1, epi, mg);
     }
-    dfk_fold_kernel<<<(unsigned)((n * n + 255) / 256), 256, 0, st>>>((const double*)vpart, nsplit, n, k);
+    dfk_fold_kernel<<<(unsigned)((n * n + 255) / 256), 256, 0, st>>>((const double*)vpart, nsplit, n, k, mg,
+                                                                     nsplit_mg);
     FC_TRY(check_launch("DF-K kernels"));
     if (jf) {  // join J's second pass
         FC_CUDA(cudaEventRecord(c.join, c.side));
         FC_CUDA(cudaStreamWaitEvent(st, c.join, 0));
     }
-    if (stats) {
-        FC_CUDA(cudaEventRecord(c.ev1, st));
-        FC_CUDA(cudaEventSynchronize(c.ev1));
-        float ms = 0.f;
-        FC_CUDA(cudaEventElapsedTime(&ms, c.ev0, c.ev1));
-        stats->kernel_ms = ms;
-        stats->flops = 4.0 * (double)naux * (double)n * (double)n * (double)nocc;
-        stats->precision = FC_PREC_F64;
-        stats->launches += 4;
-        stats->main_launches = 2;
-        stats->main_ms = ms;
-        stats->main_flops = stats->flops;
-        stats->main_bytes = 8.0 * (double)naux * (double)n * (double)n;
-        stats->tile_m = DG_BM;
-        stats->tile_n = DG_BN;
-    }
-    return FC_OK;
+    return dfk_stats(h, nocc, room ? 10 : 4, room ? MG_BM : DG_BM, room ? MG_BN : DG_BN, st, stats);
 }
 
 // J's second pass on the side stream, after everything `st` holds so far.

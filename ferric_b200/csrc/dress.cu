@@ -22,6 +22,7 @@
 #include "dgemm_tn.cuh"
 #include "fc_internal.cuh"
 #include "fx_split.cuh"
+#include "mgemm.cuh"
 #include "tmap.cuh"
 #include "xgemm.cuh"
 
@@ -95,11 +96,20 @@ struct EpiDress {
     }
 };
 
+// Column tile of the half transform: C_left's columns are few, and each CTA's
+// time is that of its padded tile (nl 81: one tile of 96 instead of two of 64).
+constexpr int HALF_M = 64, HALF_N = 96;
+bool half_wide(int64_t nl) { return rup(nl, HALF_N) < rup(nl, DG_BN); }
+
 bool g_dress_attr = false;
 
 fc_status dress_attrs() {
     if (g_dress_attr) return FC_OK;
     FC_CUDA(cudaFuncSetAttribute(dgemm_tn_kernel<EpiHalf>, cudaFuncAttributeMaxDynamicSharedMemorySize, DG_SMEM));
+    FC_CUDA(cudaFuncSetAttribute(dgemm_tn_kernel<EpiHalf, false, false, HALF_M, HALF_N>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, dg_smem(HALF_M, HALF_N)));
+    FC_CUDA(cudaFuncSetAttribute(dgemm_tn_kernel<EpiStore, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 DG_SMEM));
     FC_CUDA(cudaFuncSetAttribute(dgemm_tn_kernel<EpiMoT>, cudaFuncAttributeMaxDynamicSharedMemorySize, DG_SMEM));
     FC_CUDA(cudaFuncSetAttribute(dgemm_tn_kernel<EpiStore>, cudaFuncAttributeMaxDynamicSharedMemorySize, DG_SMEM));
     FC_CUDA(cudaFuncSetAttribute(xgemm_kernel<128, EpiDress>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -129,6 +139,18 @@ fc_status mo_dress(const double* eri3, bool host, int64_t naux, int64_t n, const
     FC_TRY(ws_get(WS_TS, (size_t)qc * nl * n * 8, &vh));
     FC_TRY(ws_get(WS_T, (size_t)width * naux * 8, &vmot));
     if (host) FC_TRY(ws_get(WS_SPLIT, (size_t)qc * n * n * 8, &vchunk));
+    // FP64 through residues (mgemm.cuh) where the products outweigh their
+    // operands' conversion: the MO step per chunk (K = n) and the dressing
+    // (K = naux).  The MO tensor then stays in its natural order (Q, l, r).
+    const bool residues = precision == FC_PREC_F64 && 2.0 * naux * (double)naux * width >= 1e10 && naux <= MG_KMAX &&
+                          n <= MG_KMAX && n >= 256;
+    int* mg_flags = nullptr;
+    if (residues) {
+        void* v;
+        FC_TRY(ws_get(WS_OUT, 256, &v));
+        mg_flags = (int*)v;
+        FC_CUDA(cudaMemsetAsync(v, 0, 256, st));
+    }
     double* clt = (double*)vct;  // C_left^T (nl x n)
     double* crt = clt + nl * n;  // C_right^T (nr x n)
     double* H = (double*)vh;
@@ -148,11 +170,27 @@ fc_status mo_dress(const double* eri3, bool host, int64_t naux, int64_t n, const
         }
         {  // H[(q, nu)][l] = sum_mu (Q|nu mu) C_left[mu, l]
             const int M = (int)(qn * n);
-            dim3 g((unsigned)((nl + DG_BN - 1) / DG_BN), (unsigned)((M + DG_BM - 1) / DG_BM), 1);
             EpiHalf epi{H, n, (int)nl};
-            dgemm_tn_kernel<EpiHalf><<<g, 256, DG_SMEM, st>>>(t3, n, clt, n, M, (int)nl, n, n, 0, epi);
+            if (half_wide(nl) && (M + HALF_M - 1) / HALF_M <= 65535) {
+                dim3 g((unsigned)((nl + HALF_N - 1) / HALF_N), (unsigned)((M + HALF_M - 1) / HALF_M), 1);
+                dgemm_tn_kernel<EpiHalf, false, false, HALF_M, HALF_N>
+                    <<<g, 256, dg_smem(HALF_M, HALF_N), st>>>(t3, n, clt, n, M, (int)nl, n, n, 0, epi);
+            } else {
+                dim3 g((unsigned)((nl + DG_BN - 1) / DG_BN), (unsigned)((M + DG_BM - 1) / DG_BM), 1);
+                dgemm_tn_kernel<EpiHalf><<<g, 256, DG_SMEM, st>>>(t3, n, clt, n, M, (int)nl, n, n, 0, epi);
+            }
         }
-        {  // (Q|lr) = sum_nu H[(q, l)][nu] C_right[nu, r] -> MOt[l*nr + r][Q]
+        if (residues) {  // (Q|lr) = sum_nu H[(q, l)][nu] C_right[nu, r]
+            const MgOut o{mot + q0 * width, nr, 0, 1.0, 0};
+            bool room = false;
+            FC_TRY(mg_multiply({c_right, nr, nr, true}, {H, n, qn * nl, false}, n, o, false, 1, mg_flags, st, &room));
+            const int M = (int)(qn * nl);
+            dim3 g((unsigned)((nr + DG_BN - 1) / DG_BN), (unsigned)((M + DG_BM - 1) / DG_BM), 1);
+            EpiStore epi{o.out, nr, 1.0, 0};
+            dgemm_tn_kernel<EpiStore><<<g, 256, DG_SMEM, st>>>(H, n, crt, n, M, (int)nr, n, n, 0, epi,
+                                                                room ? mg_flags : nullptr);
+            launches += 4;
+        } else {  // the same, stored as MOt[l*nr + r][Q]
             const int M = (int)(qn * nl);
             dim3 g((unsigned)((nr + DG_BN - 1) / DG_BN), (unsigned)((M + DG_BM - 1) / DG_BM), 1);
             EpiMoT epi{mot, naux, (int)nl, (int)nr, (int)q0};
@@ -166,7 +204,18 @@ fc_status mo_dress(const double* eri3, bool host, int64_t naux, int64_t n, const
         FC_TRY(timing_events(1, &ev));
         FC_CUDA(cudaEventRecord(ev[0], st));
     }
-    if (precision == FC_PREC_F64) {
+    if (residues) {
+        // B[P][w] = sum_Q M[P][Q] MO[Q][w]
+        bool room = false;
+        FC_TRY(mg_multiply({mot, width, width, true}, {m, naux, naux, false}, naux, MgOut{b, width, 0, 1.0, 0}, false, 1,
+                           mg_flags, st, &room));
+        dim3 g((unsigned)((width + DG_BN - 1) / DG_BN), (unsigned)((naux + DG_BM - 1) / DG_BM), 1);
+        EpiStore epi{b, width, 1.0, 0};
+        dgemm_tn_kernel<EpiStore, false, true><<<g, 256, DG_SMEM, st>>>(
+            m, naux, mot, width, (int)naux, (int)width, naux, naux, 0, epi, room ? mg_flags : nullptr);
+        FC_TRY(check_launch("dressing GEMM (FP64, residues)"));
+        launches += 8;
+    } else if (precision == FC_PREC_F64) {
         // B[P][w] = sum_Q M[P][Q] MOt[w][Q]
         dim3 g((unsigned)((width + DG_BN - 1) / DG_BN), (unsigned)((naux + DG_BM - 1) / DG_BM), 1);
         if (g.x > 2147483647u) return fail(FC_ERR_LAYOUT, "MO dressing: width too large");
@@ -228,7 +277,7 @@ fc_status mo_dress(const double* eri3, bool host, int64_t naux, int64_t n, const
         stats->precision = precision == FC_PREC_F64 ? FC_PREC_F64 : FC_PREC_MIXED;
         stats->launches += launches;
         stats->tile_m = 128;
-        stats->tile_n = precision == FC_PREC_F64 ? DG_BN : 128;
+        stats->tile_n = residues ? MG_BN : precision == FC_PREC_F64 ? DG_BN : 128;
         stats->k_panel = precision == FC_PREC_F64 ? 0 : xg::KP * xg::KT;
         stats->main_launches = 1;
         stats->main_ms = m4;

@@ -507,19 +507,64 @@ fc_status mg_convert_cols(const double* src, int64_t ld, int64_t R, int64_t K, M
     return check_launch("residue conversion (columns)");
 }
 
+// Tile c of the product in launch order: split-major, then groups of GM m-tiles,
+// n-major within a group (16 x 9 tiles in flight: 2048 x 2304 of the product,
+// whose operands the CTAs share in L2).
+struct TileGrid {
+    static constexpr int GM = 16;
+    int ntm, ntn, nks, kps, upper;
+    __host__ __device__ int64_t count() const { return (int64_t)ntm * ntn * ((nks + kps - 1) / kps); }
+    __host__ __device__ bool at(int64_t c, int4* it) const {
+        const int s = (int)(c / ((int64_t)ntm * ntn));
+        const int64_t r = c % ((int64_t)ntm * ntn);
+        const int g = (int)(r / ((int64_t)GM * ntn)), q = (int)(r % ((int64_t)GM * ntn));
+        const int gm = ntm - g * GM < GM ? ntm - g * GM : GM;
+        const int tm = g * GM + q % gm, tn = q / gm;
+        const int nk = nks - s * kps < kps ? nks - s * kps : kps;
+        *it = make_int4(tm, tn, s * kps, nk | (s << 20));
+        return !upper || (int64_t)tm * MG_BM + MG_BM - 1 >= (int64_t)tn * MG_BN;
+    }
+};
+
+static TileGrid tile_grid(int64_t M, int64_t N, int64_t K, bool upper, int splits) {
+    const int nks = (int)(mg_kp(K) / MG_KT);
+    return {(int)((M + MG_BM - 1) / MG_BM), (int)((N + MG_BN - 1) / MG_BN), nks, (nks + splits - 1) / splits, upper};
+}
+
 int64_t mg_tiles(int64_t M, int64_t N, int64_t K, bool upper, int splits, std::vector<int4>* items) {
-    const int ntm = (int)((M + MG_BM - 1) / MG_BM), ntn = (int)((N + MG_BN - 1) / MG_BN);
-    const int nks = (int)(mg_kp(K) / MG_KT), kps = (nks + splits - 1) / splits;
-    constexpr int GM = 16;  // 16 x 9 tiles in flight: 2048 x 2304 of the product
-    const size_t n0 = items->size();
-    for (int s = 0; s * kps < nks; ++s)
-        for (int g = 0; g < ntm; g += GM)
-            for (int tn = 0; tn < ntn; ++tn)
-                for (int tm = g; tm < std::min(ntm, g + GM); ++tm) {
-                    if (upper && (int64_t)tm * MG_BM + MG_BM - 1 < (int64_t)tn * MG_BN) continue;
-                    items->push_back(make_int4(tm, tn, s * kps, std::min(kps, nks - s * kps) | (s << 20)));
-                }
-    return (int64_t)(items->size() - n0);
+    const TileGrid g = tile_grid(M, N, K, upper, splits);
+    if (!items && !upper) return g.count();
+    int64_t n = 0;
+    int4 it;
+    for (int64_t c = 0; c < g.count(); ++c)
+        if (g.at(c, &it)) {
+            if (items) items->push_back(it);
+            ++n;
+        }
+    return n;
+}
+
+// The same list written on the device: calls that return before their work is
+// done copy nothing from the host.
+__global__ void __launch_bounds__(1024) mg_tiles_kernel(TileGrid g, int4* __restrict__ items) {
+    __shared__ int cnt[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int64_t base = 0;
+    for (int64_t c0 = 0; c0 < g.count(); c0 += 1024) {
+        int4 it;
+        const bool in = c0 + threadIdx.x < g.count() && g.at(c0 + threadIdx.x, &it);
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        if (lane == 0) cnt[warp] = __popc(m);
+        __syncthreads();
+        int before = 0, all = 0;
+        for (int w = 0; w < 32; ++w) {
+            before += w < warp ? cnt[w] : 0;
+            all += cnt[w];
+        }
+        if (in) items[base + before + __popc(m & ((1u << lane) - 1))] = it;
+        base += all;
+        __syncthreads();
+    }
 }
 
 size_t mg_scratch_bytes() { return CTA_SCRATCH * (size_t)ctx().sm_count; }
@@ -532,7 +577,7 @@ fc_status mg_gemm(const MgOperand& A, const MgOperand& B, const MgOut& out, cons
         FC_CUDA(cudaFuncSetAttribute(mg_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
         done.fetch_or(bit);
     }
-    if (A.kp != B.kp || A.K > MG_KMAX || MG_N * std::max(A.plane, B.plane) + MG_BN > INT32_MAX) return fail(FC_ERR_LAYOUT, "residue GEMM: K differs or is too large");
+    if (A.kp != B.kp || MG_N * std::max(A.plane, B.plane) + MG_BN > INT32_MAX) return fail(FC_ERR_LAYOUT, "residue GEMM: K differs or is too large");
     CUtensorMap ta, tb;
     FC_TRY(make_tmap_i8_2d(&ta, A.r, A.kp, (uint64_t)(MG_N - 1) * A.plane + A.rows, A.kp, MG_KT, MG_BM));
     FC_TRY(make_tmap_i8_2d(&tb, B.r, B.kp, (uint64_t)(MG_N - 1) * B.plane + B.rows, B.kp, MG_KT, MG_BN));
@@ -542,6 +587,74 @@ fc_status mg_gemm(const MgOperand& A, const MgOperand& B, const MgOut& out, cons
     if (grid > 0)
         mg_gemm_kernel<<<grid, THREADS, SMEM, st>>>(ta, tb, a);
     return check_launch("mg_gemm_kernel");
+}
+
+__global__ void mg_fold_kernel(const double* __restrict__ part, int splits, int64_t M, int64_t N, double alpha,
+                               double* __restrict__ out, int64_t ld) {
+    const int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    if (e >= M * N) return;
+    double s = 0.0;
+    for (int k = 0; k < splits; ++k) s += part[(int64_t)k * M * N + e];
+    out[e / M * ld + e % M] = alpha * s;
+}
+
+fc_status mg_fold(const double* part, int splits, int64_t M, int64_t N, double alpha, double* out, int64_t ld,
+                  cudaStream_t st) {
+    mg_fold_kernel<<<(unsigned)((M * N + 255) / 256), 256, 0, st>>>(part, splits, M, N, alpha, out, ld);
+    return check_launch("mg_fold_kernel");
+}
+
+int mg_splits(int64_t M, int64_t N, int64_t K, bool upper) {
+    const int64_t tiles = std::max<int64_t>(1, mg_tiles(M, N, 1, upper, 1, nullptr)), nks = mg_kp(K) / MG_KT;
+    int64_t s = std::max<int64_t>(1, std::min(ctx().sm_count / tiles, nks / 4));
+    s = std::max(s, (K + MG_KMAX - 1) / MG_KMAX);  // the ranges' sums stay exact
+    const int64_t kps = (nks + s - 1) / s;
+    return (int)((nks + kps - 1) / kps);
+}
+
+fc_status mg_multiply(const MgSrc& a, const MgSrc& b, int64_t K, const MgOut& out, bool upper, int splits, int* flags,
+                      cudaStream_t st, bool* room) {
+    *room = false;
+    const bool same = a.p == b.p && a.ld == b.ld && a.rows == b.rows && a.cols == b.cols;
+    const int64_t seg = splits > 1 ? K : std::min<int64_t>(K, MG_KMAX / MG_KT * MG_KT);
+    const int64_t rmax = std::max(a.rows, b.rows);
+    if (MG_N * rmax + MG_BN > INT32_MAX || K > INT32_MAX) return FC_OK;
+    const TileGrid gf = tile_grid(a.rows, b.rows, seg, upper, splits);
+    const TileGrid gl = tile_grid(a.rows, b.rows, K % seg ? K % seg : seg, upper, splits);
+    const int64_t nfull = mg_tiles(a.rows, b.rows, seg, upper, splits, nullptr);
+    size_t off = 0;
+    auto take = [&](size_t bytes) {
+        const size_t o = off;
+        off += (bytes + 255) & ~size_t(255);
+        return o;
+    };
+    const size_t osa = take(a.rows * 8), osb = take(b.rows * 8);
+    const size_t opart = take((a.cols || b.cols) ? mg_colpart(rmax, seg) * 8 : 0);
+    const size_t ofull = take(nfull * sizeof(int4)), olast = take(nfull * sizeof(int4));
+    void* mg[WS_MG_SLOTS];
+    if (!ws_get_mg({mg_bytes(a.rows, seg), same ? 0 : mg_bytes(b.rows, seg), 0, mg_scratch_bytes(), off}, mg))
+        return FC_OK;
+    *room = true;
+    char* m = (char*)mg[4];
+    mg_tiles_kernel<<<1, 1024, 0, st>>>(gf, (int4*)(m + ofull));
+    if (K % seg) mg_tiles_kernel<<<1, 1024, 0, st>>>(gl, (int4*)(m + olast));
+    auto convert = [&](const MgSrc& s, void* r, size_t os, int64_t k0, int64_t k, MgOperand* o) {
+        *o = MgOperand{(int8_t*)r, (double*)(m + os)};
+        return s.cols ? mg_convert_cols(s.p + k0 * s.ld, s.ld, s.rows, k, o, (double*)(m + opart), flags, st)
+                      : mg_convert_rows(s.p + k0, s.ld, s.rows, k, o, flags, st);
+    };
+    for (int64_t k0 = 0; k0 < K; k0 += seg) {
+        const int64_t k = std::min(seg, K - k0);
+        MgOperand A, B;
+        FC_TRY(convert(a, mg[0], osa, k0, k, &A));
+        if (same) B = A;
+        else FC_TRY(convert(b, mg[1], osb, k0, k, &B));
+        MgOut o = out;
+        if (k0) o.accumulate = 1;
+        const bool part = k != seg;
+        FC_TRY(mg_gemm(A, B, o, (const int4*)(m + (part ? olast : ofull)), nfull, mg[3], flags + 1, st));
+    }
+    return FC_OK;
 }
 
 }  // namespace fc

@@ -65,11 +65,31 @@ struct MgOut {
 };
 
 // Tiles (tm, tn) of the product, `splits` ranges of K each; upper: only tiles
-// that reach m >= n.  Grouped so that the tiles in flight share operands.
+// that reach m >= n.  Appended to items (or only counted: nullptr).
 int64_t mg_tiles(int64_t M, int64_t N, int64_t K, bool upper, int splits, std::vector<int4>* items);
 size_t mg_scratch_bytes();  // residues of the tiles in flight
 // items: device copy of mg_tiles' list.  *err (device) takes a wait's timeout.
 fc_status mg_gemm(const MgOperand& A, const MgOperand& B, const MgOut& out, const int4* items, int64_t nitems,
                   void* scratch, int* err, cudaStream_t st);
+
+// A whole product of two FP64 matrices in device memory, converted here:
+// operand rows are the rows of p, or its columns (cols).  Uses every residue
+// slot but WS_MG_T.  K beyond MG_KMAX runs in ranges that accumulate (splits
+// must be 1).  *room = false, and nothing is launched, where the residues do
+// not fit.  flags (two device ints, zeroed by the caller): rows out of range,
+// a wait's timeout; the product is valid where both stay 0.
+struct MgSrc {
+    const double* p;
+    int64_t ld, rows;
+    bool cols;
+};
+fc_status mg_multiply(const MgSrc& a, const MgSrc& b, int64_t K, const MgOut& out, bool upper, int splits, int* flags,
+                      cudaStream_t st, bool* room);
+// out[n * ld + m] = alpha * sum of the splits' partials, in order.
+fc_status mg_fold(const double* part, int splits, int64_t M, int64_t N, double alpha, double* out, int64_t ld,
+                  cudaStream_t st);
+// Splits of K that give the tiles of an M x N product about one wave, at least
+// four k-steps each.
+int mg_splits(int64_t M, int64_t N, int64_t K, bool upper);
 
 }  // namespace fc

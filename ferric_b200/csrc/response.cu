@@ -20,6 +20,7 @@
 
 #include "dgemm_tn.cuh"
 #include "fc_internal.cuh"
+#include "mgemm.cuh"
 
 namespace fc {
 
@@ -58,15 +59,45 @@ fc_status response_2c(const double* x_ov, const double* b_ov, const double* vis,
     void* vc;
     FC_TRY(ws_get(WS_PART, (size_t)naux * nov * 8, &vc));
     double* cfit = (double*)vc;
+    const bool residues = 2.0 * naux * (double)naux * nov >= 4e9 && naux <= MG_KMAX;
+    const int splits = residues && nov <= INT32_MAX / 2 ? mg_splits(naux, naux, nov, false) : 1;
+    int* flags = nullptr;
+    double* gpart = nullptr;
+    if (residues) {
+        void *vf, *vp;
+        FC_TRY(ws_get(WS_OUT, 256, &vf));
+        FC_TRY(ws_get(WS_T, splits > 1 ? (size_t)splits * naux * naux * 8 : 0, &vp));
+        flags = (int*)vf;
+        gpart = (double*)vp;
+        FC_CUDA(cudaMemsetAsync(vf, 0, 256, st));
+    }
     if (stats) FC_CUDA(cudaEventRecord(c.ev0, st));
     // y[P, ia] = sum_Q V[Q, P] x[Q, ia];  C[P, ia] = sum_Q V[Q, P] b[Q, ia]
-    dgemm_tn_kernel<EpiStore, true, true><<<tiles(naux, nov), 256, DG_SMEM, st>>>(
-        vis, naux, x_ov, nov, (int)naux, (int)nov, naux, naux, 0, EpiStore{y_ov, nov, 1.0, 0});
-    dgemm_tn_kernel<EpiStore, true, true><<<tiles(naux, nov), 256, DG_SMEM, st>>>(
-        vis, naux, b_ov, nov, (int)naux, (int)nov, naux, naux, 0, EpiStore{cfit, nov, 1.0, 0});
     // gamma_2c[P, Q] = -w sum_ia C[P, ia] y[Q, ia]
+    // Through residues (mgemm.cuh) where the products outweigh their operands'
+    // conversion; the DMMA launches then only run where its flags ask for it.
+    const int* mg = nullptr;
+    if (residues) {
+        const MgSrc v{vis, naux, naux, true};
+        bool room = false;
+        FC_TRY(mg_multiply({x_ov, nov, nov, true}, v, naux, MgOut{y_ov, nov, 0, 1.0, 0}, false, 1, flags, st, &room));
+        if (room)
+            FC_TRY(mg_multiply({b_ov, nov, nov, true}, v, naux, MgOut{cfit, nov, 0, 1.0, 0}, false, 1, flags, st,
+                               &room));
+        if (room)
+            FC_TRY(mg_multiply({y_ov, nov, naux, false}, {cfit, nov, naux, false}, nov,
+                               splits > 1 ? MgOut{gpart, naux, naux * naux, 1.0, 0}
+                                          : MgOut{gamma_2c, naux, 0, -w, 0},
+                               false, splits, flags, st, &room));
+        if (room && splits > 1) FC_TRY(mg_fold(gpart, splits, naux, naux, -w, gamma_2c, naux, st));
+        mg = room ? flags : nullptr;
+    }
+    dgemm_tn_kernel<EpiStore, true, true><<<tiles(naux, nov), 256, DG_SMEM, st>>>(
+        vis, naux, x_ov, nov, (int)naux, (int)nov, naux, naux, 0, EpiStore{y_ov, nov, 1.0, 0}, mg);
+    dgemm_tn_kernel<EpiStore, true, true><<<tiles(naux, nov), 256, DG_SMEM, st>>>(
+        vis, naux, b_ov, nov, (int)naux, (int)nov, naux, naux, 0, EpiStore{cfit, nov, 1.0, 0}, mg);
     dgemm_tn_kernel<EpiStore><<<tiles(naux, naux), 256, DG_SMEM, st>>>(
-        cfit, nov, y_ov, nov, (int)naux, (int)naux, nov, nov, 0, EpiStore{gamma_2c, naux, -w, 0});
+        cfit, nov, y_ov, nov, (int)naux, (int)naux, nov, nov, 0, EpiStore{gamma_2c, naux, -w, 0}, mg);
     FC_TRY(check_launch("RI response 2c GEMMs"));
     if (stats) {
         FC_CUDA(cudaEventRecord(c.ev1, st));
@@ -76,7 +107,7 @@ fc_status response_2c(const double* x_ov, const double* b_ov, const double* vis,
         stats->kernel_ms = ms;
         stats->flops = 6.0 * (double)naux * naux * nov;
         stats->precision = FC_PREC_F64;
-        stats->launches += 3;
+        stats->launches += mg ? 26 : 3;  // conversions, tile lists, residue GEMMs, fold
         stats->main_launches = 3;
         stats->main_ms = ms;
         stats->main_flops = stats->flops;

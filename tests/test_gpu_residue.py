@@ -93,3 +93,74 @@ def test_densities_match_oracle(fc, naux, nocc, nvir):
     t2, _ = orc.t2_and_integrals(b, eo, ev)
     for x, y in zip(got[4:], orc.mp2_density(t2, nocc, nvir)):
         assert np.abs(x - y).max() <= 1e-12 * np.abs(y).max()
+
+
+def _rand(seed, *shape):
+    import torch
+    return torch.randn(shape, generator=torch.Generator("cuda").manual_seed(seed), device="cuda", dtype=torch.float64)
+
+
+def _close(x, y, tol=1e-13):
+    assert float((x - y).abs().max()) <= tol * float(y.abs().max())
+
+
+@pytest.mark.parametrize("n,naux,nocc", [(257, 640, 192), (513, 401, 77)])
+def test_dfk_rank_update(fc, n, naux, nocc):
+    """K = W W^T through residues, split over (Q, i); non-finite C takes the DMMA form."""
+    import torch
+    from ferric_b200.dfjk import DfJK
+    b = _rand(1, naux, n, n) / n
+    b = b + b.transpose(1, 2)
+    c = torch.linalg.qr(_rand(2, n, nocc))[0].contiguous()
+    torch.cuda.synchronize()
+    w = (b @ c).permute(1, 0, 2).reshape(n, -1)
+    jk = DfJK(b)
+    st = {}
+    j, k = jk.jk_from_occ(c, stats=st)
+    assert st["tile_n"] == 256
+    torch.cuda.synchronize()
+    _close(k, w @ w.T)
+    _close(j, torch.einsum("q,qmn->mn", torch.einsum("qmn,mn->q", b, c @ c.T), b))
+    assert torch.equal(k, k.T)
+    c[3, 2] = float("nan")
+    torch.cuda.synchronize()
+    k = jk.k_from_occ(c)
+    torch.cuda.synchronize()
+    assert bool(torch.isnan(k).all())
+    jk.close()
+
+
+@pytest.mark.parametrize("naux,n,nl,nr", [(640, 257, 17, 769), (1025, 256, 90, 64)])
+def test_dressing(fc, naux, n, nl, nr):
+    import torch
+    from ferric_b200 import dress
+    t = _rand(3, naux, n, n)
+    t = t + t.transpose(1, 2)
+    m, cl, cr = _rand(4, naux, naux), _rand(5, n, nl), _rand(6, n, nr)
+    torch.cuda.synchronize()
+    st = {}
+    b = dress.mo_dress(t, m, cl, cr, stats=st)
+    assert st["tile_n"] == 256
+    ref = m @ (cl.T @ t @ cr).reshape(naux, nl * nr)
+    _close(b, ref)
+    m[5, 7] = float("inf")  # its row takes the DMMA form: not finite there, the others as before
+    torch.cuda.synchronize()
+    b = dress.mo_dress(t, m, cl, cr)
+    torch.cuda.synchronize()
+    assert not bool(torch.isfinite(b[5]).any())
+    _close(torch.cat([b[:5], b[6:]]), torch.cat([ref[:5], ref[6:]]))
+
+
+@pytest.mark.parametrize("naux,nov", [(513, 8193), (300, 66000)])
+def test_response_2c(fc, naux, nov):
+    """Few tiles over a long K (split), and a K past one range of exact sums."""
+    import torch
+    from ferric_b200 import rimp2
+    x, b, v = _rand(7, naux, nov), _rand(8, naux, nov), _rand(9, naux, naux)
+    torch.cuda.synchronize()
+    st = {}
+    y, g = rimp2.rimp2_response_2c(x, b, v, stats=st)
+    assert st["launches"] > 3
+    yr = v.T @ x
+    _close(y, yr)
+    _close(g, -2.0 * (v.T @ b) @ yr.T)
