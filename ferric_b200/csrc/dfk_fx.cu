@@ -138,7 +138,11 @@ __global__ void __launch_bounds__(256) dfk_split_w_kernel(const float* __restric
 
 // Stage 1 store: row r = (Q, mu) of B, column i: W[mu * ldw + Q * nocc_p + i].
 // Also, per thread, the max |W| of its values (atomicMax into wmax[mu]: the
-// order-free maximum of non-negative FP32 bits), so W's split reads W once.
+// order-free maximum of non-negative FP32 bits), so W's split reads W once; and
+// (e: optional) J's pass-1 terms e[col0 / 32][r] = sum_i W[mu, (Q, i)] C[mu, i]
+// over its 32 columns, of the FP32 W, so that pass reads W not at all (a pass of
+// its own over W, 637 MB at n 872, naux 2256, nocc 81, took 237 us).
+template <int BN>
 struct EpiW {
     const double* sa;  // [naux*n] B row scales
     const double* sc;  // [npad] C^T row scales
@@ -146,30 +150,51 @@ struct EpiW {
     int64_t ldw, rows;
     int n, nocc, nocc_p;
     unsigned* wmax;     // [n]
+    const double* c;    // (n x nocc)
+    double* e;          // [ceil(nocc_p / 32)][rows]
     __device__ void operator()(int64_t, int4 it, int row, int col0, const double (&acc)[32]) const {
         const int64_t r = (int64_t)it.x * xg::BM + row;
         if (r >= rows) return;
         const int64_t q = r / n, mu = r % n;
-        const int i0 = it.y * 64 + col0;
+        const int i0 = it.y * BN + col0;
         if (i0 >= nocc_p) return;
         const double s = sa[r];
         float* dst = w + mu * ldw + q * nocc_p + i0;
+        const double* cr = c + mu * nocc + i0;
         float m = 0.f;
+        double d = 0.0;
 #pragma unroll
         for (int c4 = 0; c4 < 32; c4 += 4) {
             if (i0 + c4 >= nocc_p) break;  // nocc_p is a multiple of 16
             float v[4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int i = i0 + c4 + e;
-                v[e] = i < nocc ? (float)(s * sc[i] * acc[c4 + e]) : 0.f;
-                m = fmaxf(m, fabsf(v[e]));
+            for (int u = 0; u < 4; ++u) {
+                const int i = i0 + c4 + u;
+                v[u] = i < nocc ? (float)(s * sc[i] * acc[c4 + u]) : 0.f;
+                m = fmaxf(m, fabsf(v[u]));
+            }
+            if (e) {
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (i0 + c4 + u < nocc) d += (double)v[u] * cr[c4 + u];
             }
             *reinterpret_cast<float4*>(dst + c4) = make_float4(v[0], v[1], v[2], v[3]);
         }
         atomicMax(wmax + mu, __float_as_uint(m));
+        if (e) e[(int64_t)(i0 / 32) * rows + r] = d;
     }
 };
+
+// d[Q] = sum over the column groups g and mu of e[g][Q n + mu], one CTA per Q.
+__global__ void __launch_bounds__(128) dfk_d_sum_kernel(const double* __restrict__ e, int ng, int64_t rows, int64_t n,
+                                                        double* __restrict__ d) {
+    __shared__ double red[32];
+    double s = 0.0;
+    for (int g = 0; g < ng; ++g)
+        for (int64_t mu = threadIdx.x; mu < n; mu += 128) s += e[(int64_t)g * rows + blockIdx.x * n + mu];
+    s = block_sum(s, red);
+    if (threadIdx.x == 0) d[blockIdx.x] = s;
+}
 
 // Stage 2 store: the item's FP64 partial tile [128][128], zero outside n x n.
 struct EpiPart {
@@ -208,10 +233,32 @@ __global__ void __launch_bounds__(256) dfk_fold_fx_kernel(const double* __restri
 
 bool g_attr_done = false;
 
+template <int BN>
+fc_status stage1_attr() {
+    FC_CUDA(cudaFuncSetAttribute(xgemm_kernel<BN, EpiW<BN>, true, LdKBlocksA>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, xg::Cfg<BN, true>::SMEM));
+    return FC_OK;
+}
+
+// W = B C: every column tile reads all of B's slices, so the stage, HBM-bound,
+// takes the narrowest tile that holds all columns (with two tiles of 64 for
+// nocc 81 it ran 1.77 ms, B's slices alone are 0.79 at the copy rate).  Up to 64
+// columns two accumulator sets overlap the drain with the next item.
+int stage1_bn(int64_t nocc) { return nocc <= 64 ? 64 : nocc <= 96 ? 96 : nocc <= 128 ? 128 : 64; }
+
+template <int BN>
+void stage1(const CUtensorMap& tb, const CUtensorMap& tc, const XArgs& a, const EpiW<64>& p, int grid,
+            cudaStream_t st) {
+    const EpiW<BN> epi{p.sa, p.sc, p.w, p.ldw, p.rows, p.n, p.nocc, p.nocc_p, p.wmax, p.c, p.e};
+    xgemm_kernel<BN, EpiW<BN>, true, LdKBlocksA>
+        <<<grid, xg::Cfg<BN, true>::THREADS, xg::Cfg<BN, true>::SMEM, st>>>(tb, tc, a, epi);
+}
+
 fc_status xg_attrs() {
     if (g_attr_done) return FC_OK;
-    FC_CUDA(cudaFuncSetAttribute(xgemm_kernel<64, EpiW, true, LdKBlocksA>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, xg::Cfg<64, true>::SMEM));
+    FC_TRY((stage1_attr<64>()));
+    FC_TRY((stage1_attr<96>()));
+    FC_TRY((stage1_attr<128>()));
     FC_CUDA(cudaFuncSetAttribute(xgemm_kernel<128, EpiPart, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  xg::Cfg<128, true>::SMEM));
     g_attr_done = true;
@@ -245,16 +292,15 @@ fc_status dfk_build_mixed(fc_dfjk* h, const double* c_occ, int64_t nocc, double*
     const int64_t n = h->n, naux = h->naux, ldk = rup(n, 16);
     const int64_t rows = naux * n;
     // nocc_p a multiple of 16: W's rows (ldw = naux nocc_p bytes as int8 slices) stay 16-byte aligned
-    const int64_t nocc_p = rup(nocc, 16), npad = rup(nocc, 64), ldw = naux * nocc_p, mp = rup(n, 128);
+    const int bn1 = stage1_bn(nocc);
+    const int64_t nocc_p = rup(nocc, 16), npad = rup(nocc, bn1), ldw = naux * nocc_p, mp = rup(n, 128);
 
     if (rows > INT32_MAX || 3 * rows > (int64_t)UINT32_MAX || mp > 65536 || ldw > INT32_MAX)
         return fail(FC_ERR_LAYOUT, "DF-K mixed: shape too large");
-    // stage-1 and stage-2 work items
+    // stage-1 items are numbered by the kernel; stage-2 work items
+    const int ntn1 = (int)(npad / bn1);
+    const int64_t n1 = (rows + 127) / 128 * ntn1;
     std::vector<int4> items;
-    const int ntm1 = (int)((rows + 127) / 128), ntn1 = (int)(npad / 64), nks1 = (int)((n + 127) / 128);
-    for (int tm = 0; tm < ntm1; ++tm)
-        for (int tn = 0; tn < ntn1; ++tn) items.push_back(make_int4(tm, tn, 0, nks1));
-    const int64_t n1 = (int64_t)items.size();
     const int nt = (int)(mp / 128);
     const int ntile = nt * (nt + 1) / 2;
     const int nks2 = (int)((ldw + 127) / 128);  // k-steps of 128 int8
@@ -271,7 +317,7 @@ fc_status dfk_build_mixed(fc_dfjk* h, const double* c_occ, int64_t nocc, double*
                 items.push_back(make_int4(tm, tn, k0, std::min(kps, nks2 - k0)));
             }
         }
-    const int64_t n2 = (int64_t)items.size() - n1;
+    const int64_t n2 = (int64_t)items.size();
 
     void *vc, *vout, *vw, *vws, *vsw, *vpart, *vtab;
     const size_t cs_bytes = (size_t)3 * npad * ldk;
@@ -283,6 +329,9 @@ fc_status dfk_build_mixed(fc_dfjk* h, const double* c_occ, int64_t nocc, double*
     unsigned* wmax = (unsigned*)((double*)vsw + mp);  // [n] row maxima of |W| (FP32 bits)
 
     FC_TRY(ws_get(WS_PART, (size_t)n2 * 128 * 128 * 8, &vpart));
+    // J's row terms use the space of W's slices, which are written after the terms are read
+    const int nej = (int)((nocc_p + 31) / 32);
+    double* jterm = jf ? (double*)vws : nullptr;
     FC_TRY(ws_get(WS_PAIRS, items.size() * sizeof(int4) + tix.size() * sizeof(int), &vtab));
     int* flags = (int*)vout;  // [0] range, [1] timeout
     double* sc = (double*)((char*)vc + rup((int64_t)cs_bytes, 256));
@@ -295,7 +344,7 @@ fc_status dfk_build_mixed(fc_dfjk* h, const double* c_occ, int64_t nocc, double*
     CUtensorMap tb, tcm, tw;
     const int64_t nkb = (n + 127) / 128;  // k-blocks of the B slices
     FC_TRY(make_tmap_i8_2d(&tb, h->sq_split, 128, 3 * nkb * rows, 128, 128, 128));
-    FC_TRY(make_tmap_i8_2d(&tcm, vc, n, 3 * npad, ldk, 128, 64));
+    FC_TRY(make_tmap_i8_2d(&tcm, vc, n, 3 * npad, ldk, 128, bn1));
     FC_TRY(make_tmap_i8_2d(&tw, vws, ldw, 3 * mp, ldw, 128, 128));
 
     if (stats) FC_CUDA(cudaEventRecord(cx.ev0, st));
@@ -307,25 +356,24 @@ fc_status dfk_build_mixed(fc_dfjk* h, const double* c_occ, int64_t nocc, double*
         FC_CUDA(cudaEventRecord(ev[0], st));
     }
     {
-        XArgs a{(const int4*)vtab, n1, (int)rows, (int)npad, flags + 1, (int)nkb};
-        EpiW epi{h->sq_scale, sc, (float*)vw, ldw, rows, (int)n, (int)nocc, (int)nocc_p, wmax};
+        const XArgs a{nullptr, n1, (int)rows, (int)npad, flags + 1, (int)nkb, ntn1};
+        const EpiW<64> epi{h->sq_scale, sc,       (float*)vw, ldw,  rows,   (int)n, (int)nocc,
+                           (int)nocc_p, wmax,     c_occ,      jterm};
         const int grid = (int)std::min<int64_t>(n1, cx.sm_count);
-        xgemm_kernel<64, EpiW, true, LdKBlocksA>
-            <<<grid, xg::Cfg<64, true>::THREADS, xg::Cfg<64, true>::SMEM, st>>>(tb, tcm, a, epi);
+        if (bn1 == 64) stage1<64>(tb, tcm, a, epi, grid, st);
+        else if (bn1 == 96) stage1<96>(tb, tcm, a, epi, grid, st);
+        else stage1<128>(tb, tcm, a, epi, grid, st);
     }
     if (stats) FC_CUDA(cudaEventRecord(ev[1], st));
-    if (jf) {  // J: pass-1 vector from the FP32 W (each element rounded once), second pass forked off
-        const int64_t dq = dfj_d_rows(nocc, 4);  // nocc_p: a multiple of 16 floats
-        dfj_d_from_w_kernel<float, 4><<<dim3((unsigned)((naux + dq - 1) / dq), DFJ_DY), 256, 0, st>>>(
-            (const float*)vw, ldw, nocc_p, n, nocc, naux, dq, c_occ, jf->dpart);
-        dfj_d_sum_kernel<<<(unsigned)((naux + 255) / 256), 256, 0, st>>>(jf->dpart, naux, jf->dp);
+    if (jf) {  // J: pass-1 vector from the stage's row terms, second pass forked off
+        dfk_d_sum_kernel<<<(unsigned)naux, 128, 0, st>>>(jterm, nej, rows, n, jf->dp);
         FC_TRY(dfj_fork_pass2(h, *jf, st));
     }
     dfk_split_w_kernel<<<dim3((unsigned)n, 4), 256, 0, st>>>((const float*)vw, ldw, mp, (double*)vsw, (int8_t*)vws,
                                                               wmax);
     if (stats) FC_CUDA(cudaEventRecord(ev[2], st));
     {
-        XArgs a{(const int4*)vtab + n1, n2, (int)mp, (int)mp, flags + 1};
+        XArgs a{(const int4*)vtab, n2, (int)mp, (int)mp, flags + 1};
         EpiPart epi{(const double*)vsw, (double*)vpart, (int)n};
         const int grid = (int)std::min<int64_t>(n2, cx.sm_count);
         xgemm_kernel<128, EpiPart, true><<<grid, xg::Cfg<128, true>::THREADS, xg::Cfg<128, true>::SMEM, st>>>(
@@ -355,7 +403,7 @@ fc_status dfk_build_mixed(fc_dfjk* h, const double* c_occ, int64_t nocc, double*
         stats->precision = FC_PREC_MIXED;
         stats->launches += 5;
         stats->tile_m = 128;
-        stats->tile_n = 64;
+        stats->tile_n = bn1;
         stats->k_panel = xg::KP * xg::KT;
         stats->main_launches = 2;
         stats->main_ms = (double)m1 + (double)m2;

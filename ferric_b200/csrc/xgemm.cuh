@@ -50,12 +50,12 @@ constexpr double I8L1W = 1.0 / 254.0, I8L2W = 1.0 / (254.0 * 254.0);
 
 template <int BN, bool I8 = false>
 struct Cfg {
-    static_assert(BN == 64 || BN == 128, "BN is 64 or 128");
+    static_assert(BN == 64 || BN == 96 || BN == 128, "BN is 64, 96 or 128");
     static constexpr int KTE = I8 ? 2 * KT : KT;   // elements of K per k-step (128 bytes)
     static constexpr int A_BYTES = BM * KT * 2;
     static constexpr int B_BYTES = BN * KT * 2;
     static constexpr int STAGE = 3 * (A_BYTES + B_BYTES);
-    static constexpr int STAGES = BN == 128 ? 2 : 3;
+    static constexpr int STAGES = BN == 64 ? 3 : 2;
     static constexpr int NEW = BN / 8;             // epilogue warps
     static constexpr int THREADS = 64 + 32 * NEW;
     static constexpr int NSET = BN == 64 ? 2 : 1;  // TMEM accumulator sets
@@ -73,10 +73,12 @@ struct XArgs {
     int Ma, Nb;  // rows (LdPlanes: planes) between the slices of the A and B tensor maps
     int* err;
     int nka;     // LdKBlocksA: k-blocks of A per slice
+    int ntn;     // LdKBlocksA: n-tiles (its items are numbered, not listed)
 };
 
 struct LdTiles {
     static constexpr int KP = xg::KP;
+    __device__ static int4 item(const XArgs& p, int64_t t) { return p.items[t]; }
     __device__ static int k0(int4 it) { return it.z; }
     template <int BN, int KTE>
     __device__ static void load(void* da, void* db, const CUtensorMap* ta, const CUtensorMap* tb, uint64_t* bar,
@@ -87,9 +89,12 @@ struct LdTiles {
 };
 
 // A in 128-byte column blocks ([slice][k-block][Ma rows][128 B], a 2-D map
-// 128 bytes wide), B as LdTiles.
+// 128 bytes wide), B as LdTiles; item t is (t / ntn, t % ntn) over all of K.
 struct LdKBlocksA {
     static constexpr int KP = xg::KP;
+    __device__ static int4 item(const XArgs& p, int64_t t) {
+        return make_int4((int)(t / p.ntn), (int)(t % p.ntn), 0, p.nka);
+    }
     __device__ static int k0(int4 it) { return it.z; }
     template <int BN, int KTE>
     __device__ static void load(void* da, void* db, const CUtensorMap* ta, const CUtensorMap* tb, uint64_t* bar,
@@ -101,6 +106,7 @@ struct LdKBlocksA {
 
 struct LdRows {  // item (A row, B row, first k-step, k-steps)
     static constexpr int KP = 256;
+    __device__ static int4 item(const XArgs& p, int64_t t) { return p.items[t]; }
     __device__ static int k0(int4 it) { return it.z; }
     template <int BN, int KTE>
     __device__ static void load(void* da, void* db, const CUtensorMap* ta, const CUtensorMap* tb, uint64_t* bar,
@@ -112,6 +118,7 @@ struct LdRows {  // item (A row, B row, first k-step, k-steps)
 
 struct LdPlanes {  // item (A plane tile, B plane tile, row in every plane, k-steps from 0)
     static constexpr int KP = 256;
+    __device__ static int4 item(const XArgs& p, int64_t t) { return p.items[t]; }
     __device__ static int k0(int4) { return 0; }
     template <int BN, int KTE>
     __device__ static void load(void* da, void* db, const CUtensorMap* ta, const CUtensorMap* tb, uint64_t* bar,
@@ -177,7 +184,7 @@ __global__ void __launch_bounds__(xg::Cfg<BN, I8>::THREADS, 1)
         if (lane == 0) {
             uint32_t g = 0;
             for (int64_t t = blockIdx.x; t < p.nitems && !*abort_flag; t += gridDim.x) {
-                const int4 it = p.items[t];
+                const int4 it = Ld::item(p, t);
                 const int kb = Ld::k0(it);
                 for (int kt = kb; kt < kb + it.w; ++kt, ++g) {
                     const int s = g % S;
@@ -201,7 +208,7 @@ __global__ void __launch_bounds__(xg::Cfg<BN, I8>::THREADS, 1)
         if (lane == 0) {
             uint32_t g = 0, pc = 0;  // k-steps consumed, panels issued
             for (int64_t t = blockIdx.x; t < p.nitems && !*abort_flag; t += gridDim.x) {
-                const int4 it = p.items[t];
+                const int4 it = Ld::item(p, t);
                 for (int k0 = 0; k0 < it.w; k0 += KP, ++pc) {
                     const int b = (int)(pc % NS);
                     const uint32_t u = pc / NS;
@@ -254,7 +261,7 @@ __global__ void __launch_bounds__(xg::Cfg<BN, I8>::THREADS, 1)
         uint32_t pc = 0;
         bool ok = true;
         for (int64_t t = blockIdx.x; t < p.nitems && ok; t += gridDim.x) {
-            const int4 it = p.items[t];
+            const int4 it = Ld::item(p, t);
             double acc[32];
 #pragma unroll
             for (int c = 0; c < 32; ++c) acc[c] = 0.0;
