@@ -10,8 +10,9 @@ namespace fc {
 
 namespace {
 
-// The largest 15 pairwise coprime integers up to 256 (greedily).
-constexpr int MOD[MG_N] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 197};
+// 15 pairwise coprime integers up to 256 (the largest ones but for the last,
+// which makes their product P = 2^117.75 an FP64 number within 2^-56.7).
+constexpr int MOD[MG_N] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 193};
 
 constexpr int symmod(int64_t x, int p) {
     int64_t r = x % p;
@@ -48,39 +49,51 @@ constexpr int crt_inv(int l) {
     return 0;
 }
 
-// The remainder theorem in fractions: x / P = sum_l s_l / p_l (mod 1), s_l =
-// r_l inv_l.  Two moduli a, b at a time: (s_a p_b + s_b p_a) / (p_a p_b) with
-// an integer numerator below 2^25; 1 / (p_a p_b) = fh + fl, fh a multiple of
-// 2^-40, so the sum of the numerators times fh is exact in FP64 and loses its
-// integer part exactly.  MG_N is odd: the last one stands alone.
-constexpr int NPAIR = (MG_N + 1) / 2;
+// The remainder theorem in fractions: x / P = sum_l r_l inv_l / p_l (mod 1).
+// F_l = inv_l / p_l rounded to 72 bits: the sum's error, 2^-64 on average, is a
+// sixteenth of the operands' rounding.  Byte b of four F_l is a word, so four
+// terms of the sum's byte b are one dp4a, and the sum is nine 20-bit integers.
+// (In FP64, on pairs of moduli, the same took 30 FP64 instructions per element,
+// which share their pipe with the tensor core: at K = 700 as long as a third of
+// its products.)
+constexpr int FB = 9;                      // bytes of F_l
+constexpr int NG = (MG_N + 3) / 4;         // groups of four moduli
 struct Crt {
-    uint32_t wa[NPAIR], wb[NPAIR];
-    double fh[NPAIR], fl[NPAIR];
-    double ph, pl;  // P = ph + pl
+    uint32_t f[FB][NG];
+    double p64;  // P / 2^64
 };
 constexpr Crt make_crt() {
     Crt c{};
-    for (int k = 0; k < NPAIR; ++k) {
-        const int a = 2 * k, b = 2 * k + 1;
-        const int64_t pa = MOD[a], pb = b < MG_N ? MOD[b] : 1;
-        c.wa[k] = (uint32_t)(crt_inv(a) * pb);
-        c.wb[k] = b < MG_N ? (uint32_t)(crt_inv(b) * pa) : 0u;
-        const int64_t q = (int64_t(1) << 40) / (pa * pb), r = (int64_t(1) << 40) % (pa * pb);
-        c.fh[k] = (double)q / 1099511627776.0;
-        c.fl[k] = (double)r / (double)(pa * pb) / 1099511627776.0;
+    for (int l = 0; l < MG_N; ++l) {
+        const unsigned __int128 f = (((unsigned __int128)crt_inv(l) << (8 * FB)) + MOD[l] / 2) / (unsigned)MOD[l];
+        for (int b = 0; b < FB; ++b) c.f[b][l / 4] |= (uint32_t)(uint8_t)(f >> (8 * b)) << (8 * (l % 4));
     }
     unsigned __int128 P = 1;
     for (int l = 0; l < MG_N; ++l) P *= (unsigned)MOD[l];
-    // top 53 bits and the rest
-    const unsigned __int128 top = (P >> 65) << 65;
-    c.ph = (double)(uint64_t)(P >> 65) * 36893488147419103232.0;  // 2^65; P < 2^118: 53 bits
-    const unsigned __int128 rest = P - top;
-    c.pl = (double)(uint64_t)(rest >> 33) * 8589934592.0;  // 2^33 (what is left is below 2^-85 P)
+    c.p64 = (double)(uint64_t)(P >> 64) + (double)(uint64_t)P / 18446744073709551616.0;
     return c;
 }
-static_assert(make_crt().ph > 1.6615e35 && make_crt().ph < 3.3231e35, "P lies in [2^117, 2^118)");
+static_assert(make_crt().p64 > 0.83 * 18014398509481984.0 && make_crt().p64 < 0.85 * 18014398509481984.0,
+              "P = 0.84 2^118: |x| <= 2^116.7 < P / 2");
 __constant__ Crt c_crt = make_crt();
+
+// The element whose residues (unsigned bytes, any representatives) are the
+// bytes of r[0..NG-1], as x / P * 2^64.
+__device__ __forceinline__ double crt_element(const uint32_t (&r)[NG]) {
+    uint32_t a[FB];
+#pragma unroll
+    for (int b = 0; b < FB; ++b) {
+        a[b] = 0;
+#pragma unroll
+        for (int g = 0; g < NG; ++g) a[b] = __dp4a(r[g], c_crt.f[b][g], a[b]);
+    }
+    // (sum_b a_b 2^(8 b)) / 2^8 modulo 2^64
+    const uint32_t g0 = (a[0] >> 8) + a[1] + (a[2] << 8), g1 = a[3] + (a[4] << 8);
+    const uint32_t g2 = a[5] + (a[6] << 8), g3 = a[7] + (a[8] << 8);
+    const uint64_t t = (uint64_t)g1 * 65536u + g0;
+    const uint32_t lo = (uint32_t)t, hi = (uint32_t)(t >> 32) + g2 + (g3 << 16);
+    return tc::i64_to_f64((int)hi, lo);
+}
 
 // floor(c / p) = (c * m) >> 38 with m = floor(2^38 / p) + 1 for 0 <= c < 2^30;
 // for -2^30 < c < 0 it is one less where p divides c, which leaves the residue
@@ -167,27 +180,32 @@ __device__ __forceinline__ double mg_scale(double n2, int* bad) {
     return ldexp(1.0, -e);
 }
 
-constexpr int ROWS_PER_CTA = 8;
-
-// One warp per row: its 2-norm, in a fixed order, and its scale.
+// Scales of the rows from their 2-norms, summed in a fixed order: one warp per
+// row, or with WIDE a CTA of eight (few long rows: 700 x 5577 took 26 us with a
+// warp each, 88 CTAs of dependent loads).
+template <bool WIDE>
 __global__ void __launch_bounds__(256) mg_row_scale_kernel(const double* __restrict__ x, int64_t ld, int64_t R,
                                                            int64_t K, double* __restrict__ scale, int* bad) {
-    const int64_t r = (int64_t)blockIdx.x * ROWS_PER_CTA + (threadIdx.x >> 5);
+    __shared__ double red[32];
+    constexpr int T = WIDE ? 256 : 32;  // threads per row
+    const int64_t r = WIDE ? blockIdx.x : (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (r >= R) return;
-    const int lane = threadIdx.x & 31;
+    const int t = threadIdx.x % T;
     const double* row = x + r * ld;
     double s[4] = {0.0, 0.0, 0.0, 0.0};
-    int64_t k = lane;
-    for (; k + 96 < K; k += 128) {
+    int64_t k = t;
+    for (; k + 3 * T < K; k += 4 * T) {
         double v[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) v[u] = row[k + 32 * u];
+        for (int u = 0; u < 4; ++u) v[u] = row[k + T * u];
 #pragma unroll
         for (int u = 0; u < 4; ++u) s[u] += v[u] * v[u];
     }
-    for (; k < K; k += 32) s[0] += row[k] * row[k];
-    const double n2 = warp_sum((s[0] + s[1]) + (s[2] + s[3]));
-    if (lane == 0) scale[r] = mg_scale(n2, bad);
+    for (; k < K; k += T) s[0] += row[k] * row[k];
+    double n2 = (s[0] + s[1]) + (s[2] + s[3]);
+    if constexpr (WIDE) n2 = block_sum(n2, red);
+    else n2 = warp_sum(n2);
+    if (t == 0) scale[r] = mg_scale(n2, bad);
 }
 
 // Partial squared norms of the columns over 256 rows each.
@@ -222,7 +240,7 @@ __global__ void __launch_bounds__(256) mg_col_scale_kernel(const double* __restr
 // its shared-memory strip (one double of padding per 16, so the 16 k a lane
 // then reads lie in other banks than its neighbours'), 16 bytes of each plane
 // per lane.  Bound by the integer pipes: about 100 instructions per element.
-__global__ void __launch_bounds__(256) mg_rows_kernel(const double* __restrict__ x, int64_t ld, int64_t R, int64_t K,
+__global__ void __launch_bounds__(256, 4) mg_rows_kernel(const double* __restrict__ x, int64_t ld, int64_t R, int64_t K,
                                                       int64_t kp, const double* __restrict__ scale,
                                                       int8_t* __restrict__ out) {
     __shared__ double sm[8][512 + 32];
@@ -247,7 +265,7 @@ __global__ void __launch_bounds__(256) mg_rows_kernel(const double* __restrict__
 
 // Columns of x (K x R) -> residues: a CTA takes 32 columns by 128 k through
 // shared memory (columns rotated by 4 per 16 k against bank conflicts).
-__global__ void __launch_bounds__(256) mg_cols_kernel(const double* __restrict__ x, int64_t ld, int64_t R, int64_t K,
+__global__ void __launch_bounds__(256, 4) mg_cols_kernel(const double* __restrict__ x, int64_t ld, int64_t R, int64_t K,
                                                       int64_t kp, const double* __restrict__ scale,
                                                       int8_t* __restrict__ out) {
     __shared__ double sm[128 * 32];
@@ -270,8 +288,9 @@ constexpr int S = 4;
 constexpr int A_BYTES = MG_BM * MG_KT, B_BYTES = MG_BN * MG_KT;  // 16 + 32 KiB
 constexpr int STAGE = A_BYTES + B_BYTES;
 constexpr int SMEM = S * STAGE + 1024 + 256;
-constexpr int EPI_WARPS = 8;
+constexpr int EPI_WARPS = 16;
 constexpr int EPI_THREADS = 32 * EPI_WARPS;
+constexpr int EPI_COLS = MG_BN / (EPI_WARPS / 4);  // columns per thread
 constexpr int THREADS = 64 + EPI_THREADS;
 constexpr uint32_t IDESC = tc::idesc_i8_s32(MG_BM, MG_BN);
 constexpr size_t CTA_SCRATCH = (size_t)MG_N * MG_BM * MG_BN;
@@ -283,17 +302,23 @@ struct MgArgs {
     const double* sm;  // scales of the rows of A, B
     const double* sn;
     MgOut o;
-    uint4* scratch;
+    uint32_t* scratch;
     int* err;
 };
 
 // Persistent: a CTA takes tiles of 128 x 256; per tile it runs the 15 moduli
 // one after another, each over all of K, into one of two 256-column TMEM
-// accumulators, so the epilogue of one modulus overlaps the products of the
-// next.  The epilogue reduces the int32 sums modulo p and parks the residue
-// bytes of the tile (480 KiB per CTA, in L2) until the last modulus is done;
-// then each thread reads its own bytes back and forms the FP64 results.
-// Lanes are consecutive m, so stores to out[n * ld + m] are coalesced.
+// accumulators, so the reduction of one modulus overlaps the products of the
+// next.  Sixteen warps reduce the int32 sums modulo p and park the residue
+// bytes of the tile (480 KiB per CTA: 71 MB in all, which L2 holds; twice that,
+// to form a tile's results under the next one's reductions, cost 23% at K =
+// 4800) until the last modulus is done; then each thread reads its own bytes
+// back and forms the FP64 results.  Lanes are consecutive m, so stores to
+// out[n * ld + m] are coalesced.
+// Bound by the int8 products at large K (16611^2 x 4800: 15.8 ms, 168 TFLOP/s
+// FP64-equivalent) and by the epilogue below K ~ 1000.  Sixteen epilogue warps
+// with the dp4a remainder theorem instead of eight with the FP64 one: 5577^2 x
+// 700 0.54 -> 0.48 ms, 16384^2 x 2150 8.0 -> 7.55.
 __global__ void __launch_bounds__(THREADS, 1)
     mg_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const MgArgs p) {
     extern __shared__ uint8_t smem_raw[];
@@ -390,11 +415,12 @@ __global__ void __launch_bounds__(THREADS, 1)
         }
         __syncwarp();
     } else {
+        // thread = TMEM lane (row) and a range of 64 columns; the bytes of four
+        // columns are a word, a warp's words are consecutive
         const int q = warp & 3, h = (warp - 2) >> 2;
         const int row = q * 32 + lane;
-        const int et = tid - 64;
-        uint4* scr = p.scratch + (int64_t)blockIdx.x * (CTA_SCRATCH / 16) + et;
-        const uint32_t tl0 = tmem_base + ((uint32_t)(q * 32) << 16) + h * 128;
+        uint32_t* scr = p.scratch + (int64_t)blockIdx.x * (CTA_SCRATCH / 4) + (tid - 64);
+        const uint32_t tl0 = tmem_base + ((uint32_t)(q * 32) << 16) + h * EPI_COLS;
         uint32_t c = 0;
         bool ok = true;
         for (int64_t t = blockIdx.x; t < p.nitems && ok; t += gridDim.x) {
@@ -406,25 +432,26 @@ __global__ void __launch_bounds__(THREADS, 1)
                     break;
                 }
                 tc::fence_after_sync();
-                const int m = c_mod.m[l], pp = c_mod.p[l];
+                const int mm = c_mod.m[l], pp = c_mod.p[l];
+                // 16 columns at a time, the next ones on their way meanwhile
+                float v[2][16];
+                tc::tmem_ld16(tl0 + b * 256, v[0]);
+                tc::tmem_wait_ld();
 #pragma unroll
-                for (int cg = 0; cg < 4; ++cg) {
-                    float v[32];
-                    tc::tmem_ld32(tl0 + b * 256 + cg * 32, v);
-                    tc::tmem_wait_ld();
-                    uint32_t w[8];
+                for (int cg = 0; cg < EPI_COLS / 16; ++cg) {
+                    if (cg + 1 < EPI_COLS / 16) tc::tmem_ld16(tl0 + b * 256 + (cg + 1) * 16, v[(cg + 1) & 1]);
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
+                    for (int j = 0; j < 4; ++j) {
                         uint32_t r[4];
 #pragma unroll
                         for (int u = 0; u < 4; ++u) {
-                            const int x = __float_as_int(v[4 * j + u]);
-                            r[u] = (uint32_t)(x - (__mulhi(x, m) >> 6) * pp);
+                            const int x = __float_as_int(v[cg & 1][4 * j + u]);
+                            r[u] = (uint32_t)(x - (__mulhi(x, mm) >> 6) * pp);
                         }
-                        w[j] = __byte_perm(__byte_perm(r[0], r[1], 0x0040), __byte_perm(r[2], r[3], 0x0040), 0x5410);
+                        __stcg(scr + (l * (EPI_COLS / 4) + 4 * cg + j) * EPI_THREADS,
+                               __byte_perm(__byte_perm(r[0], r[1], 0x0040), __byte_perm(r[2], r[3], 0x0040), 0x5410));
                     }
-                    __stcg(scr + (l * 8 + 2 * cg) * EPI_THREADS, make_uint4(w[0], w[1], w[2], w[3]));
-                    __stcg(scr + (l * 8 + 2 * cg + 1) * EPI_THREADS, make_uint4(w[4], w[5], w[6], w[7]));
+                    if (cg + 1 < EPI_COLS / 16) tc::tmem_wait_ld();
                 }
                 tc::fence_before_sync();
                 tc::mbar_arrive(&tempty[b]);
@@ -432,42 +459,47 @@ __global__ void __launch_bounds__(THREADS, 1)
             if (!ok) break;
             const int m = it.x * MG_BM + row;
             const bool vm = m < p.M;
-            const double sr = vm ? p.o.alpha * p.sm[m] : 0.0;
-            double* o = p.o.out + (int64_t)(it.w >> 20) * p.o.split_stride + m;
+            const double sr = vm ? p.o.alpha * c_crt.p64 * p.sm[m] : 0.0;
+            const int n00 = it.y * MG_BN + h * EPI_COLS, left = p.N - n00;
+            double* o = p.o.out + (int64_t)(it.w >> 20) * p.o.split_stride + (int64_t)n00 * p.o.ld + m;
+            const int ng = left >= EPI_COLS ? EPI_COLS / 4 : left > 0 ? (left + 3) / 4 : 0;
+            uint32_t w[MG_N];
+            if (ng > 0) {
+#pragma unroll
+                for (int l = 0; l < MG_N; ++l) w[l] = __ldcg(scr + l * (EPI_COLS / 4) * EPI_THREADS);
+            }
 #pragma unroll 1
-            for (int cg = 0; cg < 8; ++cg) {
-                const int n0 = it.y * MG_BN + h * 128 + cg * 16;
-                if (n0 >= p.N) break;
-                uint32_t w[MG_N][4];
+            for (int cg = 0; cg < ng; ++cg) {
+                uint32_t x[MG_N];
+                const int nx = cg + 1 < ng ? cg + 1 : cg;
 #pragma unroll
                 for (int l = 0; l < MG_N; ++l) {
-                    const uint4 x = __ldcg(scr + (l * 8 + cg) * EPI_THREADS);
-                    w[l][0] = x.x;
-                    w[l][1] = x.y;
-                    w[l][2] = x.z;
-                    w[l][3] = x.w;
+                    x[l] = w[l];
+                    w[l] = __ldcg(scr + (l * (EPI_COLS / 4) + nx) * EPI_THREADS);
+                }
+                double old[4], sc[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const bool vn = vm && cg * 4 + j < left;
+                    old[j] = p.o.accumulate && vn ? o[(int64_t)(cg * 4 + j) * p.o.ld] : 0.0;
+                    sc[j] = vn ? sr * p.sn[n00 + cg * 4 + j] : 0.0;
+                }
+                // byte j of four moduli's words -> the words of element j
+                uint32_t e[4][NG];
+#pragma unroll
+                for (int g = 0; g < NG; ++g) {
+                    const uint32_t a0 = x[4 * g], a1 = 4 * g + 1 < MG_N ? x[4 * g + 1] : 0u;
+                    const uint32_t a2 = 4 * g + 2 < MG_N ? x[4 * g + 2] : 0u, a3 = 4 * g + 3 < MG_N ? x[4 * g + 3] : 0u;
+                    const uint32_t t0 = __byte_perm(a0, a1, 0x5140), t1 = __byte_perm(a0, a1, 0x7362);
+                    const uint32_t u0 = __byte_perm(a2, a3, 0x5140), u1 = __byte_perm(a2, a3, 0x7362);
+                    e[0][g] = __byte_perm(t0, u0, 0x5410);
+                    e[1][g] = __byte_perm(t0, u0, 0x7632);
+                    e[2][g] = __byte_perm(t1, u1, 0x5410);
+                    e[3][g] = __byte_perm(t1, u1, 0x7632);
                 }
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    double hi = 0.0, lo = 0.0;
-#pragma unroll
-                    for (int k = 0; k < NPAIR; ++k) {
-                        const uint32_t ra = __byte_perm(w[2 * k][j / 4], 0, 0x4440 + j % 4);
-                        uint32_t v = ra * c_crt.wa[k];
-                        if (2 * k + 1 < MG_N) v += __byte_perm(w[2 * k + 1][j / 4], 0, 0x4440 + j % 4) * c_crt.wb[k];
-                        const double d = __hiloint2double(0x43300000, (int)v) - 4503599627370496.0;
-                        hi = __fma_rn(d, c_crt.fh[k], hi);
-                        lo = __fma_rn(d, c_crt.fl[k], lo);
-                    }
-                    const double t0 = (hi - ((hi + 6755399441055744.0) - 6755399441055744.0)) + lo;
-                    const double x = __fma_rn(t0, c_crt.pl, t0 * c_crt.ph);
-                    const int n = n0 + j;
-                    if (vm && n < p.N) {
-                        const double y = x * sr * p.sn[n];
-                        double* d = o + (int64_t)n * p.o.ld;
-                        *d = p.o.accumulate ? *d + y : y;
-                    }
-                }
+                for (int j = 0; j < 4; ++j)
+                    if (vm && cg * 4 + j < left) o[(int64_t)(cg * 4 + j) * p.o.ld] = __fma_rn(crt_element(e[j]), sc[j], old[j]);
             }
         }
     }
@@ -487,8 +519,11 @@ fc_status mg_convert_rows(const double* src, int64_t ld, int64_t R, int64_t K, M
     o->rows = o->plane = R;
     o->K = K;
     o->kp = mg_kp(K);
-    mg_row_scale_kernel<<<(unsigned)((R + ROWS_PER_CTA - 1) / ROWS_PER_CTA), 256, 0, st>>>(src, ld, R, K, o->scale,
-                                                                                           bad);
+    // one warp per row where that alone fills the chip's 64 warps per SM
+    if (R < 64 * ctx().sm_count && K >= 1024)
+        mg_row_scale_kernel<true><<<(unsigned)R, 256, 0, st>>>(src, ld, R, K, o->scale, bad);
+    else
+        mg_row_scale_kernel<false><<<(unsigned)((R + 7) / 8), 256, 0, st>>>(src, ld, R, K, o->scale, bad);
     const int64_t work = R * ((o->kp + 511) / 512);
     mg_rows_kernel<<<(unsigned)((work + 7) / 8), 256, 0, st>>>(src, ld, R, K, o->kp, o->scale, o->r);
     return check_launch("residue conversion (rows)");
@@ -582,7 +617,7 @@ fc_status mg_gemm(const MgOperand& A, const MgOperand& B, const MgOut& out, cons
     FC_TRY(make_tmap_i8_2d(&ta, A.r, A.kp, (uint64_t)(MG_N - 1) * A.plane + A.rows, A.kp, MG_KT, MG_BM));
     FC_TRY(make_tmap_i8_2d(&tb, B.r, B.kp, (uint64_t)(MG_N - 1) * B.plane + B.rows, B.kp, MG_KT, MG_BN));
     const MgArgs a{items,   nitems,  (int)A.rows, (int)B.rows, (int)A.plane, (int)B.plane,
-                   A.scale, B.scale, out, (uint4*)scratch, err};
+                   A.scale, B.scale, out, (uint32_t*)scratch, err};
     const int grid = (int)std::min<int64_t>(nitems, ctx().sm_count);
     if (grid > 0)
         mg_gemm_kernel<<<grid, THREADS, SMEM, st>>>(ta, tb, a);

@@ -256,6 +256,13 @@ __device__ __forceinline__ double i32_to_f64(float word) {
     return __hiloint2double(0x43300000, __float_as_int(word) ^ (int)0x80000000) - 4503601774854144.0;
 }
 
+// Signed 64-bit integer hi:lo -> double (rounded once) with two FP64 adds:
+// ((2^84 + 2^63 + hi 2^32) - (2^84 + 2^63 + 2^52)) + (2^52 + lo).
+__device__ __forceinline__ double i64_to_f64(int hi, uint32_t lo) {
+    return (__hiloint2double(0x45300000, hi ^ (int)0x80000000) - 19342822341709703277445120.0) +
+           __hiloint2double(0x43300000, (int)lo);
+}
+
 __device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                           uint32_t accumulate) {
     asm volatile(
