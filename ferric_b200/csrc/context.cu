@@ -233,6 +233,7 @@ fc_status fc_init(int32_t device, uint64_t pool_bytes) {
     FC_CUDA(cudaEventCreateWithFlags(&c.join, cudaEventDisableTiming));
     FC_CUDA(cudaEventCreate(&c.ev0));
     FC_CUDA(cudaEventCreate(&c.ev1));
+    FC_CUDA(cudaHostAlloc(&c.host_sum, 2 * sizeof(double), cudaHostAllocMapped | cudaHostAllocPortable));
     c.sm_count = p.multiProcessorCount;
     c.device = device;
     c.pool_cap = pool_bytes;

@@ -97,6 +97,7 @@ struct Context {
     cudaStream_t side = nullptr;   // a call's second stream (work that overlaps its main stream)
     cudaEvent_t fork = nullptr, join = nullptr;
     int sm_count = 0;
+    double* host_sum = nullptr;  // two sums of a call that ends with a synchronisation (under mu), mapped host memory
     std::mutex mu;
     Workspace ws[WS_COUNT];
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;

@@ -60,7 +60,22 @@ struct PairArgs {
     int nvir2;
     const double* eo2;
     const double* ev2;
+    // without tables (pairs == nullptr): the pairs i <= j of nocc orbitals in
+    // row-major order from number p0; the tiles ta <= tb of ntile (energy) or
+    // all of them (gradient)
+    int nocc, ntile;
+    int64_t p0;
 };
+
+// Number k of the pairs (i, j), i <= j < n, in row-major order.
+__device__ __forceinline__ int2 nth_pair(int64_t k, int64_t n) {
+    const double h = (double)(2 * n + 1);
+    int64_t i = (int64_t)((h - sqrt(h * h - 8.0 * (double)k)) * 0.5);
+    i = i < 0 ? 0 : i >= n ? n - 1 : i;
+    while (i > 0 && i * n - i * (i - 1) / 2 > k) --i;
+    while ((i + 1) * n - (i + 1) * i / 2 <= k) ++i;
+    return make_int2((int)i, (int)(i + k - (i * n - i * (i - 1) / 2)));
+}
 
 // GRAD: 0 energy (unique pairs, X and Y = G_ji), 1 gradient, 2 cross-spin
 // energy (X = G_iJ of B_alpha and B_beta only, E_ab += X^2 / D).
@@ -76,9 +91,11 @@ __global__ void __launch_bounds__(256, 2) pair_f64_kernel(PairArgs p) {
     const int wr = warp & 3, wc = warp >> 2;
     const int64_t item = blockIdx.x;
     const int64_t pidx = item / p.ntiles;
-    const int2 tt = p.tiles[item % p.ntiles];
+    const bool table = CROSS || p.pairs;
+    const int ti = (int)(item % p.ntiles);
+    const int2 tt = table ? p.tiles[ti] : GRAD ? make_int2(ti / p.ntile, ti % p.ntile) : nth_pair(ti, p.ntile);
     const int ta = tt.x, tb = tt.y;
-    const int2 ij = p.pairs[pidx];
+    const int2 ij = table ? p.pairs[pidx] : nth_pair(p.p0 + pidx, p.nocc);
     const int i = ij.x, j = ij.y;
     const int A0 = ta * PR_T, B0 = tb * PR_T;
     const int nvir = p.nvir, naux = p.naux;
@@ -294,6 +311,53 @@ __global__ void __launch_bounds__(256) reduce_vir_kernel(const double* __restric
     if (lane == 0) acc_vir[a] += 2.0 * v;
 }
 
+// The sums of a gradient whose occupied orbitals are one chunk, in one launch:
+// block 0 the energies, one block per occupied orbital, one per eight
+// virtuals.  A small molecule's gradient is three launches this way (naux 84,
+// nocc 5, nvir 19: 97 us, with four sum kernels, four fills and copies in and
+// out 175; naux 357, nocc 13, nvir 118: 403 -> 338).
+__global__ void __launch_bounds__(256) grad_sums_kernel(const double* __restrict__ part,
+                                                        const double* __restrict__ occ_part,
+                                                        const double* __restrict__ vir_part, int nocc, int ntile,
+                                                        int nvir, double* e, double* __restrict__ de_docc,
+                                                        double* __restrict__ de_dvir) {
+    __shared__ double2 sh[32];
+    const int ntile2 = ntile * ntile;
+    const int64_t npairs = (int64_t)nocc * (nocc + 1) / 2;
+    if (blockIdx.x == 0) {
+        KSum a, b;
+        for (int64_t k = threadIdx.x; k < npairs * ntile2; k += 256) {
+            a.add(part[2 * k]);
+            b.add(part[2 * k + 1]);
+        }
+        const double va = block_ksum(a, sh), vb = block_ksum(b, sh);
+        if (threadIdx.x == 0) {
+            e[0] = va;
+            e[1] = vb;
+        }
+    } else if ((int)blockIdx.x <= nocc) {
+        // the ordering (o, s) of every partner s: slot 0 of pair (o, s >= o), slot 1 of (s < o, o)
+        const int64_t o = blockIdx.x - 1;
+        KSum a;
+        for (int64_t u = threadIdx.x; u < (int64_t)nocc * ntile2; u += 256) {
+            const int64_t s = u / ntile2, i = s < o ? s : o, j = s < o ? o : s;
+            const int64_t k = (i * nocc - i * (i - 1) / 2 + (j - i)) * ntile2 + u % ntile2;
+            a.add(occ_part[2 * k + (s < o)]);
+        }
+        const double v = block_ksum(a, sh);
+        if (threadIdx.x == 0) de_docc[o] = -2.0 * v;
+    } else {
+        const int a = ((int)blockIdx.x - nocc - 1) * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+        if (a >= nvir) return;
+        const int ta = a / PR_T, ar = a % PR_T;
+        KSum s;
+        for (int64_t k = lane; k < npairs * ntile; k += 32)
+            s.add(vir_part[(((k / ntile) * ntile + ta) * ntile + k % ntile) * PR_T + ar]);
+        const double v = warp_sum(s.value());
+        if (lane == 0) de_dvir[a] = 2.0 * v;
+    }
+}
+
 static fc_status set_smem_once() {
     static std::atomic<uint64_t> done{0};
     uint64_t bit = 0;
@@ -329,17 +393,12 @@ fc_status rimp2_energy_f64(const Rimp2Dev& d, cudaStream_t st, double* e_os, dou
         return FC_OK;
     }
 
-    void *vpairs, *vpart, *vout;
-    FC_TRY(ws_get(WS_PAIRS, (npairs + ntiles) * sizeof(int2), &vpairs));
+    // The CTAs number their pairs themselves and the sum goes to the host's own
+    // memory: with a table to copy in and two doubles to copy out a call at
+    // naux 84, nocc 5, nvir 19 took 12 us more (66 -> 54).
+    Context& c = ctx();
+    void* vpart;
     FC_TRY(ws_get(WS_PART, items * 2 * sizeof(double), &vpart));
-    FC_TRY(ws_get(WS_OUT, 64 * sizeof(double), &vout));
-    std::vector<int2> hp;
-    for (int64_t i = 0, k = 0; i < nocc; ++i)
-        for (int64_t j = i; j < nocc; ++j, ++k)
-            if (k >= plo && k < phi) hp.push_back(make_int2((int)i, (int)j));
-    for (int ta = 0; ta < ntile; ++ta)
-        for (int tb = ta; tb < ntile; ++tb) hp.push_back(make_int2(ta, tb));
-    FC_CUDA(cudaMemcpyAsync(vpairs, hp.data(), hp.size() * sizeof(int2), cudaMemcpyHostToDevice, st));
 
     PairArgs a{};
     a.B = d.b_ov;
@@ -348,23 +407,22 @@ fc_status rimp2_energy_f64(const Rimp2Dev& d, cudaStream_t st, double* e_os, dou
     a.nvir = (int)nvir;
     a.eo = d.eps_occ;
     a.ev = d.eps_vir;
-    a.pairs = (const int2*)vpairs;
-    a.tiles = (const int2*)vpairs + npairs;
+    a.nocc = (int)nocc;
+    a.ntile = ntile;
+    a.p0 = plo;
     a.ntiles = ntiles;
     a.has_kappa = d.has_kappa;
     a.kappa = d.kappa;
     a.part = (double*)vpart;
 
-    Context& c = ctx();
     if (stats) FC_CUDA(cudaEventRecord(c.ev0, st));
     pair_f64_kernel<0><<<(unsigned)items, 256, PR_SMEM, st>>>(a);
     FC_TRY(check_launch("pair_f64_kernel<energy>"));
     if (stats) FC_CUDA(cudaEventRecord(c.ev1, st));
-    reduce_pairs_kernel<<<1, 1024, 0, st>>>((const double*)vpart, items, (double*)vout);
+    reduce_pairs_kernel<<<1, 1024, 0, st>>>((const double*)vpart, items, c.host_sum);
     FC_TRY(check_launch("reduce_pairs_kernel"));
-    double h[2];
-    FC_CUDA(cudaMemcpyAsync(h, vout, sizeof(h), cudaMemcpyDeviceToHost, st));
     FC_CUDA(cudaStreamSynchronize(st));
+    const double h[2] = {c.host_sum[0], c.host_sum[1]};
     *e_os = h[0];
     *e_ss = h[1];
     if (stats) {
@@ -378,7 +436,6 @@ fc_status rimp2_energy_f64(const Rimp2Dev& d, cudaStream_t st, double* e_os, dou
         stats->tile_n = PR_T;
         stats->k_panel = 0;
         stats->d2h_bytes += sizeof(h);
-        stats->h2d_bytes += hp.size() * sizeof(int2);
         stats->main_launches = 1;
         stats->main_ms = ms;
         stats->main_flops = stats->flops;
@@ -458,6 +515,7 @@ fc_status rimp2_grad_f64(const Rimp2Dev& d, cudaStream_t st, double* e_os, doubl
                                  I == nch - 1});
     }
     const int64_t nsteps = (int64_t)steps.size();
+    const bool single = nch == 1 && !dens && d.nshards == 1;  // no tables, no running sums
     DensF64 dx{};
 
     void *vpairs, *vpart, *vT, *vout;
@@ -473,11 +531,13 @@ fc_status rimp2_grad_f64(const Rimp2Dev& d, cudaStream_t st, double* e_os, doubl
     double* T2 = T1 + blk;
     double* e_cp = (double*)vout;     // [ncp][2]
     double* acc_occ = e_cp + 2 * ncp;  // [nocc]
-    FC_CUDA(cudaMemcpyAsync(vpairs, hp.data(), hp.size() * sizeof(int2), cudaMemcpyHostToDevice, st));
-    FC_CUDA(cudaMemsetAsync(de_dvir, 0, nvir * sizeof(double), st));
-    FC_CUDA(cudaMemsetAsync(acc_occ, 0, nocc * sizeof(double), st));
-    FC_CUDA(cudaMemsetAsync(e_cp, 0, 2 * ncp * sizeof(double), st));  // chunk pairs of other shards add nothing
-    FC_CUDA(cudaMemsetAsync(gamma, 0, (size_t)naux * nov * sizeof(double), st));
+    if (!single) {
+        FC_CUDA(cudaMemcpyAsync(vpairs, hp.data(), hp.size() * sizeof(int2), cudaMemcpyHostToDevice, st));
+        FC_CUDA(cudaMemsetAsync(de_dvir, 0, nvir * sizeof(double), st));
+        FC_CUDA(cudaMemsetAsync(acc_occ, 0, nocc * sizeof(double), st));
+        FC_CUDA(cudaMemsetAsync(e_cp, 0, 2 * ncp * sizeof(double), st));  // chunk pairs of other shards add nothing
+        FC_CUDA(cudaMemsetAsync(gamma, 0, (size_t)naux * nov * sizeof(double), st));
+    }
     const int2* dpairs = (const int2*)vpairs;
 
     Context& c = ctx();
@@ -494,7 +554,7 @@ fc_status rimp2_grad_f64(const Rimp2Dev& d, cudaStream_t st, double* e_os, doubl
     auto adjoint = [&](const double* T, int64_t r0, int64_t nr, int64_t k0, int64_t nk) -> fc_status {
         const int N = (int)(nr * nvir);
         dim3 grid((N + DG_BN - 1) / DG_BN, (unsigned)((naux + DG_BM - 1) / DG_BM), 1);
-        EpiStore epi{gamma + r0 * nvir, nov, 4.0, 1};
+        EpiStore epi{gamma + r0 * nvir, nov, 4.0, !single};
         const int64_t K = nk * nvir;
         if (stats) FC_CUDA(cudaEventRecord(ev2[2 * nadj], st));
         dgemm_tn_kernel<EpiStore><<<grid, 256, DG_SMEM, st>>>(d.b_ov + k0 * nvir, nov, T, K, (int)naux, N, K, K, 0,
@@ -524,9 +584,11 @@ fc_status rimp2_grad_f64(const Rimp2Dev& d, cudaStream_t st, double* e_os, doubl
         a.nvir = (int)nvir;
         a.eo = d.eps_occ;
         a.ev = d.eps_vir;
-        a.pairs = dpairs + cp.p0;
+        a.pairs = single ? nullptr : dpairs + cp.p0;
         a.tiles = dpairs + npairs_all;
         a.ntiles = ntile2;
+        a.nocc = (int)nocc;
+        a.ntile = ntile;
         a.part = part;
         a.T = T1;
         a.ldt = cp.nj * nvir;
@@ -554,7 +616,12 @@ fc_status rimp2_grad_f64(const Rimp2Dev& d, cudaStream_t st, double* e_os, doubl
         FC_TRY(check_launch("pair_f64_kernel<grad>"));
         if (stats) FC_CUDA(cudaEventRecord(ev[2 * sx + 1], st));
         ++npair_launch;
-        if (step.sums) {
+        if (single) {
+            grad_sums_kernel<<<(unsigned)(1 + nocc + (nvir + 7) / 8), 256, 0, st>>>(
+                part, occ, vir, (int)nocc, ntile, (int)nvir, c.host_sum, de_docc, de_dvir);
+            FC_TRY(check_launch("grad_sums_kernel"));
+            ++nl;
+        } else if (step.sums) {
             reduce_pairs_kernel<<<1, 1024, 0, st>>>(part, nit, e_cp + 2 * x);
             reduce_occ_kernel<<<(unsigned)(same ? cp.ni : cp.ni + cp.nj), 256, 0, st>>>(
                 occ, dpairs + cp.p0, cp.np, ntile2, (int)cp.i0, (int)cp.ni, (int)cp.j0, acc_occ);
@@ -579,12 +646,19 @@ fc_status rimp2_grad_f64(const Rimp2Dev& d, cudaStream_t st, double* e_os, doubl
         FC_TRY(dens_f64_finish(dx, *dens, st, &nl));
         if (sink) FC_TRY(gamma_sink_block(sink, gamma, naux, nov, nvir, 0, nocc, st));
     }
-    scale_copy_f64_kernel<<<(unsigned)((nocc + 255) / 256), 256, 0, st>>>(acc_occ, nocc, -2.0, de_docc);
-    FC_TRY(check_launch("scale_copy_f64_kernel"));
+    if (!single) {
+        scale_copy_f64_kernel<<<(unsigned)((nocc + 255) / 256), 256, 0, st>>>(acc_occ, nocc, -2.0, de_docc);
+        FC_TRY(check_launch("scale_copy_f64_kernel"));
+        ++nl;
+    }
     if (stats) FC_CUDA(cudaEventRecord(c.ev1, st));
     std::vector<double> h((size_t)(2 * ncp));
-    FC_CUDA(cudaMemcpyAsync(h.data(), e_cp, h.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
+    if (!single) FC_CUDA(cudaMemcpyAsync(h.data(), e_cp, h.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
     FC_CUDA(cudaStreamSynchronize(st));
+    if (single) {
+        h[0] = c.host_sum[0];
+        h[1] = c.host_sum[1];
+    }
     double eo = 0.0, co = 0.0, es = 0.0, cs = 0.0;
     for (int64_t x = 0; x < ncp; ++x) {  // chunk-pair order, compensated
         double v = h[2 * x], tt = eo + v;
@@ -604,12 +678,12 @@ fc_status rimp2_grad_f64(const Rimp2Dev& d, cudaStream_t st, double* e_os, doubl
         const double P = (double)nocc * (nocc + 1) / 2.0;
         stats->flops = 2.0 * naux * (double)nvir * nvir * P + 2.0 * naux * (double)nov * nov;
         stats->precision = FC_PREC_F64;
-        stats->launches += (int)(nl + nadj + 1);
+        stats->launches += (int)(nl + nadj);
         stats->tile_m = PR_T;
         stats->tile_n = PR_T;
         stats->k_panel = 0;
         stats->d2h_bytes += h.size() * sizeof(double);
-        stats->h2d_bytes += hp.size() * sizeof(int2);
+        stats->h2d_bytes += single ? 0 : hp.size() * sizeof(int2);
         // dominant kernel: the fused pair kernel, one launch per chunk pair,
         // forming G_ij and G_ji of every unordered pair
         stats->main_launches = (int)npair_launch;

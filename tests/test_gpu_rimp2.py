@@ -140,3 +140,16 @@ def test_pool_cap_refuses_before_transfer(fc):
         assert rimp2.try_spin_components_on_device(b, np.concatenate([eo, ev]), 5, 23) is None
     finally:
         L.init(0, 0)
+
+
+# one-chunk gradients, whose CTAs number pairs and tiles themselves: one pair,
+# one to nine tiles per pair, more orbitals than a block of the sums has warps
+@pytest.mark.parametrize("naux,nocc,nvir", [(17, 1, 1), (40, 2, 128), (21, 3, 129), (33, 40, 9)])
+def test_small_gradient_matches_oracle(fc, naux, nocc, nvir):
+    from ferric_b200 import rimp2
+    b, eo, ev = synthetic.rimp2_inputs(naux, nocc, nvir)
+    e_os, e_ss, *grads = orc.energy_gamma_deps(b, eo, ev)
+    sc, *got = rimp2.rimp2_energy_grad(b, eo, ev, precision="f64")
+    assert abs(sc.e_os - e_os) < _tol(e_os) and abs(sc.e_ss - e_ss) < _tol(e_ss)
+    for x, y in zip(got, grads):  # sums of at most nocc nvir = 387 terms in another order
+        assert np.abs(x - y).max() <= 1e-12 * np.abs(y).max()
