@@ -357,8 +357,8 @@ static fc_status dfjk_smem_once() {
     static std::atomic<uint64_t> done{0};
     uint64_t bit = 0;
     if (!attrs_needed(done, &bit)) return FC_OK;
-    FC_CUDA(cudaFuncSetAttribute(dgemm_tn_kernel<EpiScatterW>, cudaFuncAttributeMaxDynamicSharedMemorySize, DG_SMEM));
-    FC_CUDA(cudaFuncSetAttribute(dgemm_tn_kernel<EpiSplit>, cudaFuncAttributeMaxDynamicSharedMemorySize, DG_SMEM));
+    FC_CUDA(dgemm_tn_smem<EpiScatterW>());
+    FC_CUDA(dgemm_tn_smem<EpiSplit>());
     done.fetch_or(bit);
     return FC_OK;
 }
@@ -540,8 +540,7 @@ fc_status dfk_build_f64(fc_dfjk* h, const double* c_occ, int64_t nocc, double* k
     {
         dim3 g((unsigned)((nocc + DG_BN - 1) / DG_BN), (unsigned)((M1 + DG_BM - 1) / DG_BM), 1);
         EpiScatterW epi{(double*)vw, n, naux, nocc};
-        dgemm_tn_kernel<EpiScatterW><<<g, 256, DG_SMEM, st>>>(h->b_sq, n, (const double*)vct, n, (int)M1,
-                                                               (int)nocc, n, n, 0, epi);
+        dgemm_tn_launch(g, st, h->b_sq, n, (const double*)vct, n, (int)M1, (int)nocc, n, n, 0, epi);
     }
     if (jf) {  // J: pass-1 vector from W = B C, second pass forked off
         // W rows of nocc doubles: 16-byte vectors when nocc is even (and W's base is)
@@ -567,8 +566,7 @@ fc_status dfk_build_f64(fc_dfjk* h, const double* c_occ, int64_t nocc, double* k
     {  // every CTA leaves at once where the residue product stands
         dim3 g(tn, tm, nsplit);
         EpiSplit epi{(double*)vpart, n * n, (int)n};
-        dgemm_tn_kernel<EpiSplit><<<g, 256, DG_SMEM, st>>>((const double*)vw, kdim, (const double*)vw, kdim,
-                                                            (int)n, (int)n, kdim, kps, 1, epi, mg);
+        dgemm_tn_launch(g, st, (const double*)vw, kdim, (const double*)vw, kdim, (int)n, (int)n, kdim, kps, 1, epi, mg);
     }
     dfk_fold_kernel<<<(unsigned)((n * n + 255) / 256), 256, 0, st>>>((const double*)vpart, nsplit, n, k, mg,
                                                                      nsplit_mg);

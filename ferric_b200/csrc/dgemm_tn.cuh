@@ -10,8 +10,8 @@
 // products whose M or N would leave most of that empty), 8 warps (4 x 2);
 // 3-stage cp.async pipeline; split-K over blockIdx.z.  Shared-memory rows are
 // padded to 20 doubles so the fragment reads (g*20 + t) hit distinct banks.
-// A K-major operand whose rows start on 16 bytes is copied 16 bytes at a time
-// (half the copy instructions), any other 8.
+// V16 copies 16 bytes at a time, half the copy instructions; it needs both
+// operands K-major with rows on 16 bytes (dgemm_tn_launch looks).
 #pragma once
 #include <type_traits>
 
@@ -27,11 +27,12 @@ constexpr int DG_SMEM = dg_smem(DG_BM, DG_BN);
 // same with TB: a transposed (MN-major) operand is read with consecutive
 // threads on consecutive m (n), so its global loads stay coalesced.  The
 // epilogue gets `z` (the split or the batch index).
-template <class Epi, bool TA, bool TB, int BM = DG_BM, int BN = DG_BN>
+template <class Epi, bool TA, bool TB, int BM = DG_BM, int BN = DG_BN, bool V16 = false>
 __device__ __forceinline__ void dgemm_tile(const double* __restrict__ A, int64_t lda, const double* __restrict__ B,
                                            int64_t ldb, int M, int N, int64_t kbeg, int64_t kend, int upper_only,
                                            const Epi& epi, int z) {
     static_assert(BM % 32 == 0 && BN % 16 == 0, "4 x 2 warps of 8 x 8 DMMA tiles");
+    static_assert(!V16 || (!TA && !TB), "16-byte copies: K-major operands");
     constexpr int MT = BM / 32, NT = BN / 16;  // DMMA tiles per warp
     extern __shared__ __align__(16) double dg_smem_buf[];
     double* sA = dg_smem_buf;                               // [STAGES][BM][LDK]
@@ -44,8 +45,6 @@ __device__ __forceinline__ void dgemm_tile(const double* __restrict__ A, int64_t
     if (upper_only && m0 > n0 + BN - 1) return;  // tile strictly below the diagonal
     if (kbeg >= kend) return;
     const int nk = (int)((kend - kbeg + DG_BK - 1) / DG_BK);
-    const bool va = !TA && !(((uintptr_t)A & 15) | (uintptr_t)(lda & 1) | (uintptr_t)(kbeg & 1));
-    const bool vb = !TB && !(((uintptr_t)B & 15) | (uintptr_t)(ldb & 1) | (uintptr_t)(kbeg & 1));
 
     // rows [r0, r0 + ROWS) of a K-major operand (R rows), 16 bytes a copy
     auto load16 = [&](double* s, const double* X, int64_t ld, int r0, int R, int64_t kb, auto rows) {
@@ -78,10 +77,13 @@ __device__ __forceinline__ void dgemm_tile(const double* __restrict__ A, int64_t
         using RB = std::integral_constant<int, BN>;
         double* a = sA + stage * BM * DG_LDK;
         double* b = sB + stage * BN * DG_LDK;
-        if (va) load16(a, A, lda, m0, M, kb, RA{});
-        else load8(a, A, lda, m0, M, kb, RA{}, std::integral_constant<bool, TA>{});
-        if (vb) load16(b, B, ldb, n0, N, kb, RB{});
-        else load8(b, B, ldb, n0, N, kb, RB{}, std::integral_constant<bool, TB>{});
+        if constexpr (V16) {
+            load16(a, A, lda, m0, M, kb, RA{});
+            load16(b, B, ldb, n0, N, kb, RB{});
+        } else {
+            load8(a, A, lda, m0, M, kb, RA{}, std::integral_constant<bool, TA>{});
+            load8(b, B, ldb, n0, N, kb, RB{}, std::integral_constant<bool, TB>{});
+        }
     };
 
     double acc[MT][NT][2];
@@ -130,7 +132,7 @@ __device__ __forceinline__ void dgemm_tile(const double* __restrict__ A, int64_t
             }
 }
 
-template <class Epi, bool TA = false, bool TB = false, int BM = DG_BM, int BN = DG_BN>
+template <class Epi, bool TA = false, bool TB = false, int BM = DG_BM, int BN = DG_BN, bool V16 = false>
 __global__ void __launch_bounds__(256) dgemm_tn_kernel(const double* __restrict__ A, int64_t lda,
                                                        const double* __restrict__ B, int64_t ldb,
                                                        int M, int N, int64_t K, int64_t k_per_split,
@@ -138,7 +140,34 @@ __global__ void __launch_bounds__(256) dgemm_tn_kernel(const double* __restrict_
     if (run_if && !(run_if[0] | run_if[1])) return;  // the residue form's result stands (mgemm.cuh)
     const int64_t kbeg = (int64_t)blockIdx.z * k_per_split;
     const int64_t kend = kbeg + k_per_split < K ? kbeg + k_per_split : K;
-    dgemm_tile<Epi, TA, TB, BM, BN>(A, lda, B, ldb, M, N, kbeg, kend, upper_only, epi, (int)blockIdx.z);
+    dgemm_tile<Epi, TA, TB, BM, BN, V16>(A, lda, B, ldb, M, N, kbeg, kend, upper_only, epi, (int)blockIdx.z);
+}
+
+// K-major product with the copies that its operands allow (k_per_split a
+// multiple of DG_BK unless there is one split).  16-byte copies: the DF-K half
+// transform at n 600, naux 2400, nocc 60 (and with it the JK build) 4% faster,
+// the MO dressing at naux 600, n 180 5%; below eight k-steps there is nothing
+// to gain (JK at n 80: 110 -> 115 us with them).
+template <class Epi, int BM = DG_BM, int BN = DG_BN>
+void dgemm_tn_launch(dim3 grid, cudaStream_t st, const double* A, int64_t lda, const double* B, int64_t ldb, int M,
+                     int N, int64_t K, int64_t k_per_split, int upper_only, const Epi& epi,
+                     const int* run_if = nullptr) {
+    constexpr int smem = dg_smem(BM, BN);
+    const bool aligned = !(((uintptr_t)A | (uintptr_t)B | (uintptr_t)(lda * 8) | (uintptr_t)(ldb * 8)) & 15);
+    if (!aligned || K < 8 * DG_BK || k_per_split < 8 * DG_BK)
+        dgemm_tn_kernel<Epi, false, false, BM, BN>
+            <<<grid, 256, smem, st>>>(A, lda, B, ldb, M, N, K, k_per_split, upper_only, epi, run_if);
+    else
+        dgemm_tn_kernel<Epi, false, false, BM, BN, true>
+            <<<grid, 256, smem, st>>>(A, lda, B, ldb, M, N, K, k_per_split, upper_only, epi, run_if);
+}
+template <class Epi, int BM = DG_BM, int BN = DG_BN>
+cudaError_t dgemm_tn_smem() {
+    const cudaError_t e = cudaFuncSetAttribute(dgemm_tn_kernel<Epi, false, false, BM, BN>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, dg_smem(BM, BN));
+    return e != cudaSuccess ? e
+                            : cudaFuncSetAttribute(dgemm_tn_kernel<Epi, false, false, BM, BN, true>,
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, dg_smem(BM, BN));
 }
 
 // Batched over blockIdx.z: operands z * sa and z * sb elements on, all of K.

@@ -105,13 +105,12 @@ bool g_dress_attr = false;
 
 fc_status dress_attrs() {
     if (g_dress_attr) return FC_OK;
-    FC_CUDA(cudaFuncSetAttribute(dgemm_tn_kernel<EpiHalf>, cudaFuncAttributeMaxDynamicSharedMemorySize, DG_SMEM));
-    FC_CUDA(cudaFuncSetAttribute(dgemm_tn_kernel<EpiHalf, false, false, HALF_M, HALF_N>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, dg_smem(HALF_M, HALF_N)));
+    FC_CUDA(dgemm_tn_smem<EpiHalf>());
+    FC_CUDA((dgemm_tn_smem<EpiHalf, HALF_M, HALF_N>()));
     FC_CUDA(cudaFuncSetAttribute(dgemm_tn_kernel<EpiStore, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  DG_SMEM));
-    FC_CUDA(cudaFuncSetAttribute(dgemm_tn_kernel<EpiMoT>, cudaFuncAttributeMaxDynamicSharedMemorySize, DG_SMEM));
-    FC_CUDA(cudaFuncSetAttribute(dgemm_tn_kernel<EpiStore>, cudaFuncAttributeMaxDynamicSharedMemorySize, DG_SMEM));
+    FC_CUDA(dgemm_tn_smem<EpiMoT>());
+    FC_CUDA(dgemm_tn_smem<EpiStore>());
     FC_CUDA(cudaFuncSetAttribute(xgemm_kernel<128, EpiDress>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  xg::Cfg<128>::SMEM));
     g_dress_attr = true;
@@ -173,11 +172,10 @@ fc_status mo_dress(const double* eri3, bool host, int64_t naux, int64_t n, const
             EpiHalf epi{H, n, (int)nl};
             if (half_wide(nl) && (M + HALF_M - 1) / HALF_M <= 65535) {
                 dim3 g((unsigned)((nl + HALF_N - 1) / HALF_N), (unsigned)((M + HALF_M - 1) / HALF_M), 1);
-                dgemm_tn_kernel<EpiHalf, false, false, HALF_M, HALF_N>
-                    <<<g, 256, dg_smem(HALF_M, HALF_N), st>>>(t3, n, clt, n, M, (int)nl, n, n, 0, epi);
+                dgemm_tn_launch<EpiHalf, HALF_M, HALF_N>(g, st, t3, n, clt, n, M, (int)nl, n, n, 0, epi);
             } else {
                 dim3 g((unsigned)((nl + DG_BN - 1) / DG_BN), (unsigned)((M + DG_BM - 1) / DG_BM), 1);
-                dgemm_tn_kernel<EpiHalf><<<g, 256, DG_SMEM, st>>>(t3, n, clt, n, M, (int)nl, n, n, 0, epi);
+                dgemm_tn_launch(g, st, t3, n, clt, n, M, (int)nl, n, n, 0, epi);
             }
         }
         if (residues) {  // (Q|lr) = sum_nu H[(q, l)][nu] C_right[nu, r]
@@ -187,14 +185,13 @@ fc_status mo_dress(const double* eri3, bool host, int64_t naux, int64_t n, const
             const int M = (int)(qn * nl);
             dim3 g((unsigned)((nr + DG_BN - 1) / DG_BN), (unsigned)((M + DG_BM - 1) / DG_BM), 1);
             EpiStore epi{o.out, nr, 1.0, 0};
-            dgemm_tn_kernel<EpiStore><<<g, 256, DG_SMEM, st>>>(H, n, crt, n, M, (int)nr, n, n, 0, epi,
-                                                                room ? mg_flags : nullptr);
+            dgemm_tn_launch(g, st, H, n, crt, n, M, (int)nr, n, n, 0, epi, room ? mg_flags : nullptr);
             launches += 4;
         } else {  // the same, stored as MOt[l*nr + r][Q]
             const int M = (int)(qn * nl);
             dim3 g((unsigned)((nr + DG_BN - 1) / DG_BN), (unsigned)((M + DG_BM - 1) / DG_BM), 1);
             EpiMoT epi{mot, naux, (int)nl, (int)nr, (int)q0};
-            dgemm_tn_kernel<EpiMoT><<<g, 256, DG_SMEM, st>>>(H, n, crt, n, M, (int)nr, n, n, 0, epi);
+            dgemm_tn_launch(g, st, H, n, crt, n, M, (int)nr, n, n, 0, epi);
         }
         FC_TRY(check_launch("MO transform GEMMs"));
         launches += 2;
@@ -220,8 +217,7 @@ fc_status mo_dress(const double* eri3, bool host, int64_t naux, int64_t n, const
         dim3 g((unsigned)((width + DG_BN - 1) / DG_BN), (unsigned)((naux + DG_BM - 1) / DG_BM), 1);
         if (g.x > 2147483647u) return fail(FC_ERR_LAYOUT, "MO dressing: width too large");
         EpiStore epi{b, width, 1.0, 0};
-        dgemm_tn_kernel<EpiStore><<<g, 256, DG_SMEM, st>>>(m, naux, mot, naux, (int)naux, (int)width, naux, naux,
-                                                            0, epi);
+        dgemm_tn_launch(g, st, m, naux, mot, naux, (int)naux, (int)width, naux, naux, 0, epi);
         FC_TRY(check_launch("dressing GEMM (FP64)"));
         launches += 1;
     } else {
