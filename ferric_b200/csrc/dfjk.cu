@@ -412,6 +412,14 @@ static fc_status dfj_build_t(fc_dfjk* h, const TB* bp, int prec, const double* d
     const int64_t naux = h->naux, n = h->n, pair = h->pair;
     constexpr bool F32 = sizeof(TB) == 4;
     const int64_t ld = F32 ? h->ld32 : pair;  // row pitch of bp
+    if constexpr (!F32) {
+        if (dfj_small_fits(h)) {
+            Context& c = ctx();
+            if (stats) FC_CUDA(cudaEventRecord(c.ev0, st));
+            FC_TRY(dfj_small(h, d, j, st));
+            return dfj_stats(h, prec, sizeof(TB), 1, st, stats);
+        }
+    }
     void *vw, *vpart;
     const int nsplit = 4;
     const int64_t seg = F32 ? DFJ_SEG_BYTES / 2 / 16 : DFJ_SEG_BYTES / (int64_t)sizeof(TB);  // float4 or TB units
@@ -509,6 +517,14 @@ fc_status dfk_build_f64(fc_dfjk* h, const double* c_occ, int64_t nocc, double* k
     const int64_t M1 = naux * n;
     if (M1 > INT32_MAX || (M1 + DG_BM - 1) / DG_BM > 65535)
         return fail(FC_ERR_LAYOUT, "DF-K: naux*n too large for one stage-1 launch");
+    if (dfk_small_fits(h, nocc) && !(jf && h->l_chol)) {
+        Context& c = ctx();
+        if (stats) FC_CUDA(cudaEventRecord(c.ev0, st));
+        if (jf && jf->ev[0]) FC_CUDA(cudaEventRecord(jf->ev[0], st));
+        FC_TRY(dfk_small(h, c_occ, nocc, k, jf ? jf->j : nullptr, st));
+        if (jf && jf->ev[1]) FC_CUDA(cudaEventRecord(jf->ev[1], st));
+        return dfk_stats(h, nocc, 1, (int)n, (int)n, st, stats);
+    }
     const int64_t kdim = naux * nocc;
     const int tm = (int)((n + DG_BM - 1) / DG_BM), tn = (int)((n + DG_BN - 1) / DG_BN);
     int upper = 0;

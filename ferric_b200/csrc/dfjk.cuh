@@ -45,6 +45,13 @@ fc_status dfj_build_mixed(fc_dfjk* h, const double* d, double* j, cudaStream_t s
 fc_status dfk_build_mixed(fc_dfjk* h, const double* c_occ, int64_t nocc, double* k, cudaStream_t st,
                           fc_stats* stats, const JFork* jf = nullptr);
 
+// One-launch builds of small molecules (dfjk_small.cu): where they apply, J of
+// a density, and K (with j also J of C C^T).
+bool dfj_small_fits(const fc_dfjk* h);
+bool dfk_small_fits(const fc_dfjk* h, int64_t nocc);
+fc_status dfj_small(const fc_dfjk* h, const double* d, double* j, cudaStream_t st);
+fc_status dfk_small(const fc_dfjk* h, const double* c_occ, int64_t nocc, double* k, double* j, cudaStream_t st);
+
 // d[Q] = sum_{mu, i < nocc} W[mu * ldw + Q * ldq + i] C[mu * nocc + i], in a
 // fixed order: the J pass-1 vector d_Q = <B_Q, C C^T> = sum_mu (B_Q C)[mu, :] . C[mu, :]
 // from the DF-K stage-1 product.  A CTA takes dq consecutive aux rows and one

@@ -231,3 +231,23 @@ def test_fused_jk_empty_channel(fc):
     jk = DfJK(b)
     j, k = jk.jk_from_occ(np.zeros((20, 0)))
     assert not j.any() and not k.any()
+
+
+# the one-launch builds: edges of their 8 x 8 tiles and of eight and sixteen
+# orbitals, aux rows fewer than CTAs, not a multiple of eight, past one
+# shared-memory group, and K past the line where only J stays one launch
+@pytest.mark.parametrize("n,naux,nocc", [(44, 83, 16), (45, 7, 5), (64, 64, 9), (64, 61, 8), (57, 77, 1),
+                                         (7, 4000, 3), (1, 9, 1), (64, 250, 16)])
+def test_small_builds_match_oracle(fc, n, naux, nocc):
+    from ferric_b200.dfjk import DfJK
+    b, c, d = synthetic.dfjk_inputs(n, naux, nocc)
+    jk = DfJK(b)
+    st = {}
+    j, k = jk.j(d), jk.k_from_occ(c, stats=st)
+    assert (st["launches"] == 1) == (naux * n * n * 8 <= 2 << 20)
+    j2, k2 = jk.jk_from_occ(c)
+    # sums of up to naux n^2 terms in another order: 1e-13 of the largest element
+    for x, y in ((j, orc.df_j_square(b, d)), (k, orc.df_k_occ(b, c))):
+        assert np.abs(x - y).max() <= 1e-13 * np.abs(y).max() and np.array_equal(x, x.T)
+    assert np.array_equal(k2, k) and np.abs(j2 - j).max() <= 1e-13 * np.abs(j).max()
+    jk.close()
