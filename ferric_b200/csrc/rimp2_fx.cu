@@ -621,19 +621,29 @@ __device__ __forceinline__ ItemView item_view(const PairFxArgs& p, int64_t k) {
     return v;
 }
 
-// This thread's HC columns of a phase's four level accumulators -> FP64
+// Columns per thread of the epilogue on tile column tb: the valid columns in
+// four groups (with HC each, the 41 columns of a last tile were one warp's 32
+// and another's 9, and a narrow tile took as long as a full one).
+__device__ __forceinline__ int thread_columns(int nvir, int tb) {
+    using namespace fx;
+    const int c = min(BN, nvir - tb * BN);
+    return (c + 8 * NCG - 1) / (8 * NCG) * 8;
+}
+
+// This thread's hc columns of a phase's four level accumulators -> FP64
 // values s_r s_c (L0 + L1/254 + L2/254^2 + L3/254^3), stored at dst + c BM
 // for its column c (the CTA's column-major tile in global scratch, L2 only;
 // dst is its row of the first of its columns).  gdv >= 0 is the column (of
-// these HC) on the tile diagonal a == b of an i == j block: it takes the
+// these hc) on the tile diagonal a == b of an i == j block: it takes the
 // exact (ia|ia) instead, whose dropped level-4 products (the slice c3 c3' of
 // a row with itself) are one-signed.
 __device__ __forceinline__ void drain_levels(uint32_t tl, double sr, const double* __restrict__ sc, double* dst,
-                                             int gdv, double gval) {
+                                             int hc, int gdv, double gval) {
     using namespace fx;
     const double sr3 = sr * LW3INV;
 #pragma unroll
     for (int c0 = 0; c0 < HC; c0 += 8) {
+        if (c0 >= hc) break;
         float l0[8], l1[8], l2[8], l3[8];
         tc::tmem_ld8(tl + c0, l0);
         tc::tmem_ld8(tl + BN + c0, l1);
@@ -791,7 +801,7 @@ __global__ void __launch_bounds__(fx::PAIR_THREADS, 1)
         // ---------------------------------------------------------- epilogue
         // EPI_WARPS warps: lane quadrant q = warp % 4 (TMEM lanes 32q..32q+31),
         // column group h = (warp - 2) / 4; each thread owns row `row`, columns
-        // [HC h, HC h + HC).  A phase's four level accumulators fill TMEM, so
+        // [hc h, hc h + hc) with hc = thread_columns(), HC on a full tile.  A phase's four level accumulators fill TMEM, so
         // each phase is drained at once into the CTA's FP64 tiles in global
         // scratch (X, then Y), which hands TMEM back to the MMA warp.  The FP64
         // terms of an item run in two halves of its columns, software-pipelined
@@ -805,22 +815,22 @@ __global__ void __launch_bounds__(fx::PAIR_THREADS, 1)
         const int h = (warp - 2) >> 2;
         const int row = q * 32 + lane;  // a within the tile
         const int et = tid - 64;        // 0 .. EPI_THREADS - 1
-        const uint32_t tl = tmem_base + ((uint32_t)(q * 32) << 16) + h * HC;
+        const uint32_t tl = tmem_base + ((uint32_t)(q * 32) << 16);
         // X tiles [2][col][row], Y tile [col][row]: column-major, so a warp's
         // stores and loads of one column cover its 32 consecutive rows
         double* const scr0 = p.scr + (int64_t)blockIdx.x * (3 * BM * BN);
         double* const syt = scr0 + 2 * BM * BN;
-        double* const ycol = syt + h * HC * BM + row;  // this thread's first column, its row
-        constexpr int HH = HC / 2;  // columns per half
+        constexpr int HH = HC / 2;  // columns per half, at most
         // carried from an item's first half of terms to its second
         double os = 0.0, ss = 0.0, oc = 0.0, rowc = 0.0;
 
         // FP64 terms of columns [c_lo, c_lo + HH) of this thread's HC, item k
-        // (li parity lk): energy sums, derivative sums, amplitude stores, and the
+        // (li parity lk; HH is its view's hc / 2): energy sums, derivative sums, amplitude stores, and the
         // column terms of the mirrored tile reduced over the warp's 32 rows into
         // colsh[q][h][c_lo ..].
-        auto terms = [&](int64_t k, uint32_t lk, int c_lo) {
+        auto terms = [&](int64_t k, uint32_t lk, int second) {
             const ItemView v = item_view<BATCH>(p, k);
+            const int hc = thread_columns(v.nvir, v.tb), hh = hc / 2, c_lo = second * hh;
             const int i = v.i, j = v.j;
             const bool diag = i == j;
             const int ta = v.ta, tb = v.tb;
@@ -829,17 +839,23 @@ __global__ void __launch_bounds__(fx::PAIR_THREADS, 1)
             const int a = ta * BM + row;
             const bool va = a < v.nvir;
             const double dA = v.eo[i] + v.eo[j] - (va ? v.ev[a] : 0.0);
-            const int b0 = tb * BN + h * HC;  // first column of this thread
-            const double* evb = colb + (lk & 1) * 3 * BN + h * HC;
+            const int b0 = tb * BN + h * hc;  // first column of this thread
+            const double* evb = colb + (lk & 1) * 3 * BN + h * hc;
             const int bmax = v.nvir - b0;  // columns c < bmax are real virtuals
             const bool xt = v.xt;
             const bool two = !diag && !xt;
             double* const sxt = scr0 + (lk & 1) * BM * BN;
-            const double* const xcol = sxt + h * HC * BM + row;
+            const double* const xcol = sxt + h * hc * BM + row;
+            const double* const ycol = syt + h * hc * BM + row;
             constexpr int CW = 4;  // columns per step of the FP64 terms
             float ck[HH];          // column terms of this half's columns (gradient)
 #pragma unroll
             for (int cs = 0; cs < HH; cs += CW) {
+                if (cs >= hh) {
+#pragma unroll
+                    for (int cc = 0; cc < CW; ++cc) ck[cs + cc] = 0.f;
+                    continue;
+                }
                 const int c0 = c_lo + cs;
                 double xv[CW] = {}, yv[CW] = {};
                 // rows and columns past the last virtual read nothing (those tile
@@ -852,7 +868,7 @@ __global__ void __launch_bounds__(fx::PAIR_THREADS, 1)
                         for (int cc = 0; cc < CW; ++cc) yv[cc] = __ldcg(ycol + (c0 + cc) * BM);
                     } else if (xt) {
                         // Y[a, b] = X[b, a]: column a of X, this thread's columns b as rows
-                        const double2* x2 = reinterpret_cast<const double2*>(sxt + row * BM + h * HC + c0);
+                        const double2* x2 = reinterpret_cast<const double2*>(sxt + row * BM + h * hc + c0);
 #pragma unroll
                         for (int u = 0; u < CW / 2; ++u) {
                             const double2 t = __ldcg(x2 + u);
@@ -973,7 +989,7 @@ __global__ void __launch_bounds__(fx::PAIR_THREADS, 1)
                     }
                 }
                 const float tot = ck[0] + __shfl_xor_sync(0xffffffffu, ck[0], 1);
-                if ((lane & 1) == 0) colsh[(q * NCG + h) * HC + c_lo + (lane >> 1)] = (double)tot;
+                if ((lane & 1) == 0 && (lane >> 1) < hh) colsh[(q * NCG + h) * HC + c_lo + (lane >> 1)] = (double)tot;
             }
         };
 
@@ -1002,10 +1018,11 @@ __global__ void __launch_bounds__(fx::PAIR_THREADS, 1)
                 p.vir_part[k * 2 * BM + row] = rs;
             }
             if ((mir || both) && et < BM) {  // an exchanged tile put its column terms on the rows
-                const int hh = et / HC, c = et % HC;
+                const int hc = thread_columns(v.nvir, v.tb), hh = et / hc, c = et % hc;
                 double cs = 0.0;
+                if (hh < NCG)
 #pragma unroll
-                for (int qq = 0; qq < 4; ++qq) cs += colsh[(qq * NCG + hh) * HC + c];
+                    for (int qq = 0; qq < 4; ++qq) cs += colsh[(qq * NCG + hh) * HC + c];
                 p.vir_part[k * 2 * BM + BM + et] = xt ? 0.0 : cs;
             }
             if (et == 0) {
@@ -1053,8 +1070,8 @@ __global__ void __launch_bounds__(fx::PAIR_THREADS, 1)
                     }
                 }
                 asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory");
-                const double* sxb = cb_ + BN + h * HC;
-                const double* syb = cb_ + 2 * BN + h * HC;
+                const int hc = thread_columns(v.nvir, tb);
+                const double* sxb = cb_ + BN + h * hc;
                 xt = v.xt;
                 two = !diag && !xt;  // a Y phase follows in TMEM
                 // X phase -> X tile.  One thread waits (bounded); the epilogue
@@ -1064,21 +1081,20 @@ __global__ void __launch_bounds__(fx::PAIR_THREADS, 1)
                 tc::fence_after_sync();
                 {
                     // (ia|ia) on the diagonal of an i == j block's diagonal tile
-                    const int gdv = (diag && ta == tb && va) ? row - h * HC : -1;
+                    const int gdv = (diag && ta == tb && va) ? row - h * hc : -1;
                     const double gval = gdv >= 0 ? v.gd[(int64_t)i * v.a_pad + a] : 0.0;
-                    double* const xcol = scr0 + (li & 1) * BM * BN + h * HC * BM + row;
+                    double* const xcol = scr0 + (li & 1) * BM * BN + h * hc * BM + row;
                     // a warp whose columns or rows lie wholly past the last virtual
                     // drains nothing: those tile entries are never read
-                    if (h * HC < v.nvir - tb * BN && q * 32 < v.nvir - ta * BM)
-                        drain_levels(tl, sxa, sxb, xcol, (gdv >= 0 && gdv < HC) ? gdv : -1, gval);
+                    if (h * hc < v.nvir - tb * BN && q * 32 < v.nvir - ta * BM)
+                        drain_levels(tl + h * hc, sxa, sxb, xcol, hc, (gdv >= 0 && gdv < hc) ? gdv : -1, gval);
                 }
                 tc::fence_before_sync();
                 tc::mbar_arrive(tempty);
                 ++pc;
-                (void)syb;
             }
             if (kprev >= 0) {
-                terms(kprev, lprev, HH);
+                terms(kprev, lprev, 1);
                 finish(kprev, lprev);
                 kprev = -1;
             }
@@ -1086,13 +1102,14 @@ __global__ void __launch_bounds__(fx::PAIR_THREADS, 1)
             if (two) {
                 const ItemView v = item_view<BATCH>(p, k);
                 const double sya = v.scl[(int64_t)v.j * v.a_pad + v.ta * BM + row];
-                const double* syb = colb + (li & 1) * 3 * BN + 2 * BN + h * HC;
+                const int hc = thread_columns(v.nvir, v.tb);
+                const double* syb = colb + (li & 1) * 3 * BN + 2 * BN + h * hc;
                 // Y phase: (ib|ja) = G_ji[a, b] -> Y tile
                 if (!tc::bar_and<1, EPI_THREADS>(et != 0 || tc::mbar_wait(tfull, pc & 1, abort_flag, p.err))) break;
                 if (et != 0) tc::mbar_wait(tfull, pc & 1, abort_flag, p.err);
                 tc::fence_after_sync();
-                if (h * HC < v.nvir - v.tb * BN && q * 32 < v.nvir - v.ta * BM)
-                    drain_levels(tl, sya, syb, ycol, -1, 0.0);
+                if (h * hc < v.nvir - v.tb * BN && q * 32 < v.nvir - v.ta * BM)
+                    drain_levels(tl + h * hc, sya, syb, syt + h * hc * BM + row, hc, -1, 0.0);
                 tc::fence_before_sync();
                 tc::mbar_arrive(tempty);  // the level columns are free for the next item
                 ++pc;
