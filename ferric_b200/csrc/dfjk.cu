@@ -339,18 +339,7 @@ __global__ void dfk_fold_kernel(const double* __restrict__ part, int nsplit, int
     if (mg && !(mg[0] | mg[1])) nsplit = nsplit_mg;
     const int64_t r = idx / n, c = idx % n;
     const int64_t lo = r < c ? r : c, hi = r < c ? c : r;
-    const double* x = part + lo * n + hi;
-    double s = 0.0;
-    int sp = 0;
-    for (; sp + 8 <= nsplit; sp += 8) {  // eight loads in flight, added in order
-        double v[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) v[u] = x[(int64_t)(sp + u) * n * n];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) s += v[u];
-    }
-    for (; sp < nsplit; ++sp) s += x[(int64_t)sp * n * n];
-    k[idx] = s;
+    k[idx] = fold_in_order(part + lo * n + hi, nsplit, n * n);
 }
 
 static fc_status dfjk_smem_once() {

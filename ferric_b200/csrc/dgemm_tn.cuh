@@ -30,7 +30,7 @@ constexpr int DG_SMEM = dg_smem(DG_BM, DG_BN);
 template <class Epi, bool TA, bool TB, int BM = DG_BM, int BN = DG_BN, bool V16 = false>
 __device__ __forceinline__ void dgemm_tile(const double* __restrict__ A, int64_t lda, const double* __restrict__ B,
                                            int64_t ldb, int M, int N, int64_t kbeg, int64_t kend, int upper_only,
-                                           const Epi& epi, int z) {
+                                           const Epi& epi, int z, int bx, int by) {
     static_assert(BM % 32 == 0 && BN % 16 == 0, "4 x 2 warps of 8 x 8 DMMA tiles");
     static_assert(!V16 || (!TA && !TB), "16-byte copies: K-major operands");
     constexpr int MT = BM / 32, NT = BN / 16;  // DMMA tiles per warp
@@ -41,7 +41,7 @@ __device__ __forceinline__ void dgemm_tile(const double* __restrict__ A, int64_t
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
     const int wm = warp & 3, wn = warp >> 2;
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    const int m0 = by * BM, n0 = bx * BN;
     if (upper_only && m0 > n0 + BN - 1) return;  // tile strictly below the diagonal
     if (kbeg >= kend) return;
     const int nk = (int)((kend - kbeg + DG_BK - 1) / DG_BK);
@@ -140,7 +140,8 @@ __global__ void __launch_bounds__(256) dgemm_tn_kernel(const double* __restrict_
     if (run_if && !(run_if[0] | run_if[1])) return;  // the residue form's result stands (mgemm.cuh)
     const int64_t kbeg = (int64_t)blockIdx.z * k_per_split;
     const int64_t kend = kbeg + k_per_split < K ? kbeg + k_per_split : K;
-    dgemm_tile<Epi, TA, TB, BM, BN, V16>(A, lda, B, ldb, M, N, kbeg, kend, upper_only, epi, (int)blockIdx.z);
+    dgemm_tile<Epi, TA, TB, BM, BN, V16>(A, lda, B, ldb, M, N, kbeg, kend, upper_only, epi, (int)blockIdx.z,
+                                         (int)blockIdx.x, (int)blockIdx.y);
 }
 
 // K-major product with the copies that its operands allow (k_per_split a
@@ -174,9 +175,35 @@ cudaError_t dgemm_tn_smem() {
 template <class Epi, bool TA = false, bool TB = false>
 __global__ void __launch_bounds__(256) dgemm_batched_kernel(const double* __restrict__ A, int64_t lda, int64_t sa,
                                                             const double* __restrict__ B, int64_t ldb, int64_t sb,
-                                                            int M, int N, int64_t K, Epi epi, int upper_only = 0) {
+                                                            int M, int N, int64_t K, Epi epi) {
     const int z = (int)blockIdx.z;
-    dgemm_tile<Epi, TA, TB>(A + z * sa, lda, B + z * sb, ldb, M, N, 0, K, upper_only, epi, z);
+    dgemm_tile<Epi, TA, TB>(A + z * sa, lda, B + z * sb, ldb, M, N, 0, K, 0, epi, z, (int)blockIdx.x,
+                            (int)blockIdx.y);
+}
+
+// The tiles of an M x M product that reach the upper triangle, numbered by rows.
+template <int BM, int BN>
+int dgemm_upper_tiles(int64_t M) {
+    const int tn = (int)((M + BN - 1) / BN);
+    int t = 0;
+    for (int y = 0; y * BM < M; ++y) t += tn - y * BM / BN;
+    return t;
+}
+
+// Batched as above, only those tiles (blockIdx.x), each in `splits` ranges of K:
+// the epilogue's z is batch * splits + range.  A grid with the tiles below the
+// diagonal in it leaves the SMs that got those idle.
+template <class Epi, int BM, int BN>
+__global__ void __launch_bounds__(256) dgemm_upper_kernel(const double* __restrict__ A, const double* __restrict__ B,
+                                                          int64_t ld, int64_t stride, int M, int64_t K, int splits,
+                                                          int64_t k_per_split, Epi epi) {
+    const int z = (int)blockIdx.z, b = z / splits, tn = (M + BN - 1) / BN;
+    int x = (int)blockIdx.x, y = 0;
+    while (x >= tn - y * BM / BN) x -= tn - y++ * BM / BN;
+    const int64_t kbeg = (int64_t)(z % splits) * k_per_split;
+    const int64_t kend = kbeg + k_per_split < K ? kbeg + k_per_split : K;
+    dgemm_tile<Epi, false, false, BM, BN>(A + b * stride, ld, B + b * stride, ld, M, M, kbeg, kend, 0, epi, z,
+                                          x + y * BM / BN, y);
 }
 
 // value * alpha -> C[m*ldc + n]
@@ -199,6 +226,20 @@ struct EpiBatchStore {
         C[(int64_t)z * stride + (int64_t)m * ldc + n] = v;
     }
 };
+
+// s + x[0] + x[stride] + ... (n terms, in order), eight loads in flight.
+__device__ __forceinline__ double fold_in_order(const double* __restrict__ x, int n, int64_t stride, double s = 0.0) {
+    int i = 0;
+    for (; i + 8 <= n; i += 8) {
+        double v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = x[(int64_t)(i + u) * stride];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) s += v[u];
+    }
+    for (; i < n; ++i) s += x[(int64_t)i * stride];
+    return s;
+}
 
 // split-K partial -> P[split][m*N + n]
 struct EpiSplit {

@@ -121,10 +121,10 @@ struct DensF64 {
     double* ts;       // [nocc nvir][ld]
     double* as;       // [nocc nvir][ld]
     double* part_oo;  // [splits][nocc x nocc]
-    double* part_vv;  // [gvv][nvir x nvir]
+    double* part_vv;  // [gvv][kvv][nvir x nvir]
     double* acc_vv;   // [nvir x nvir] running P_vv (upper tiles)
     double* acc_oo;   // [nocc x nocc] running P_oo
-    int splits, gvv;
+    int splits, gvv, kvv;  // P_oo's ranges of K; P_vv's orbitals per launch, ranges of K
 };
 int64_t dens_chunk_f64(int64_t nocc, int64_t nvir, int64_t cc, int64_t budget);
 fc_status dens_f64_alloc(int64_t nocc, int64_t nvir, int64_t cc, cudaStream_t st, DensF64* o);

@@ -239,23 +239,41 @@ __global__ void sym_kernel(const double* __restrict__ a, int64_t n, double* __re
 __global__ void oo_fold_f64_kernel(const double* __restrict__ part, int splits, int64_t nn, double* __restrict__ acc) {
     const int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x;
     if (e >= nn) return;
-    double v = 0.0;
-    for (int s = 0; s < splits; ++s) v += part[(int64_t)s * nn + e];
-    acc[e] -= v;
+    acc[e] -= fold_in_order(part + e, splits, nn);
 }
 
 // acc[e] += sum_z part[z][e] (in order) on the upper triangle
 __global__ void vv_fold_f64_kernel(const double* __restrict__ part, int nz, int64_t n, double* __restrict__ acc) {
     const int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x;
     if (e >= n * n || e / n > e % n) return;
-    double v = 0.0;
-    for (int z = 0; z < nz; ++z) v += part[(int64_t)z * n * n + e];
-    acc[e] += v;
+    acc[e] += fold_in_order(part + e, nz, n * n);
 }
 
 // P_oo's tile: nocc rows by nocc columns over a very long K, bound by the DMMA
 // rate of the padded tile (nocc 33: 64 x 48 instead of 128 x 64, 540 -> 250 us).
 constexpr int OO_M = 64, OO_N = 48;
+
+// P_vv's tile: 64 x 48 where its upper tiles cover a tenth less than those of
+// 128 x 64 (nvir 169: 9 x 3072 elements against 4 x 8192).
+bool vv_small(int64_t nvir) {
+    return 10 * dgemm_upper_tiles<OO_M, OO_N>(nvir) * OO_M * OO_N <=
+           9 * dgemm_upper_tiles<DG_BM, DG_BN>(nvir) * DG_BM * DG_BN;
+}
+int vv_tiles(int64_t nvir) {
+    return vv_small(nvir) ? dgemm_upper_tiles<OO_M, OO_N>(nvir) : dgemm_upper_tiles<DG_BM, DG_BN>(nvir);
+}
+
+// P_vv's products of nz orbitals, kvv ranges of K each.
+template <int BM, int BN>
+fc_status vv_products(const DensF64& o, int64_t off, int64_t ld, int nz, cudaStream_t st) {
+    const int64_t nvir = o.nvir, kps = ((ld + o.kvv - 1) / o.kvv + DG_BK - 1) / DG_BK * DG_BK;
+    const dim3 g((unsigned)dgemm_upper_tiles<BM, BN>(nvir), 1, (unsigned)(nz * o.kvv));
+    if (kps * (o.kvv - 1) >= ld)  // ranges without a k step write nothing
+        FC_CUDA(cudaMemsetAsync(o.part_vv, 0, (size_t)nz * o.kvv * nvir * nvir * 8, st));
+    dgemm_upper_kernel<EpiBatchStore, BM, BN><<<g, 256, dg_smem(BM, BN), st>>>(
+        o.as + off, o.ts + off, ld, nvir * ld, (int)nvir, ld, o.kvv, kps, EpiBatchStore{o.part_vv, nvir, nvir * nvir});
+    return check_launch("dgemm_upper_kernel<P_vv>");
+}
 
 bool g_dens_attr = false;
 
@@ -265,8 +283,10 @@ fc_status dens_attrs() {
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, xg::Cfg<128, true>::SMEM));
     FC_CUDA(cudaFuncSetAttribute(xgemm_kernel<128, EpiDensOO, true, LdPlanes>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, xg::Cfg<128, true>::SMEM));
-    FC_CUDA(cudaFuncSetAttribute(dgemm_batched_kernel<EpiBatchStore>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 DG_SMEM));
+    FC_CUDA(cudaFuncSetAttribute(dgemm_upper_kernel<EpiBatchStore, DG_BM, DG_BN>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, DG_SMEM));
+    FC_CUDA(cudaFuncSetAttribute(dgemm_upper_kernel<EpiBatchStore, OO_M, OO_N>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, dg_smem(OO_M, OO_N)));
     FC_CUDA(cudaFuncSetAttribute(dgemm_tn_kernel<EpiSplit, false, false, OO_M, OO_N>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, dg_smem(OO_M, OO_N)));
     g_dens_attr = true;
@@ -414,10 +434,14 @@ fc_status dens_f64_alloc(int64_t nocc, int64_t nvir, int64_t cc, cudaStream_t st
     o->splits = std::max(1, 2 * ctx().sm_count);  // two CTAs of the P_oo tile per SM
     o->gvv = (int)std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(nocc, 65535),
                                                          (int64_t(256) << 20) / (8 * nvir * nvir)));
+    // eight CTAs per SM, so that the last ones leave little of the chip idle
+    const int64_t ctas = vv_tiles(nvir) * (int64_t)o->gvv;
+    o->kvv = (int)std::max<int64_t>(
+        1, std::min<int64_t>({16, (8 * ctx().sm_count + ctas - 1) / ctas, 65535 / o->gvv, cc * nvir / (16 * DG_BK)}));
     const size_t slab = (size_t)nocc * nvir * cc * nvir;
     void *vs, *vp, *vv;
     FC_TRY(ws_get(WS_DSLAB, 2 * slab * 8, &vs));
-    FC_TRY(ws_get(WS_DSTORE, (size_t)o->gvv * nvir * nvir * 8, &vv));
+    FC_TRY(ws_get(WS_DSTORE, (size_t)o->gvv * o->kvv * nvir * nvir * 8, &vv));
     o->part_vv = (double*)vv;
     o->ts = (double*)vs;
     o->as = o->ts + slab;
@@ -440,18 +464,19 @@ fc_status dens_f64_slab(const DensF64& o, int64_t nk, cudaStream_t st, int64_t* 
     const int64_t nvir = o.nvir, nocc = o.nocc, ld = nk * nvir;
     // P_vv (upper tiles): the products of o.gvv occupied orbitals i in one
     // launch, folded in order of i (a launch per i left 6 CTAs on the chip at
-    // nvir 169: 33 x 0.5 ms; 0.6 ms in one launch)
+    // nvir 169: 33 x 0.5 ms; 0.97 ms in one launch of 132 CTAs, 0.39 in small tiles
+    // and four ranges of K)
     for (int64_t i = 0; i < nocc; i += o.gvv) {
         const int nz = (int)std::min<int64_t>(o.gvv, nocc - i);
-        const dim3 gv((unsigned)((nvir + DG_BN - 1) / DG_BN), (unsigned)((nvir + DG_BM - 1) / DG_BM), (unsigned)nz);
         const int64_t off = i * nvir * ld;
-        dgemm_batched_kernel<EpiBatchStore><<<gv, 256, DG_SMEM, st>>>(o.as + off, ld, nvir * ld, o.ts + off, ld,
-                                                                      nvir * ld, (int)nvir, (int)nvir, ld,
-                                                                      EpiBatchStore{o.part_vv, nvir, nvir * nvir}, 1);
-        vv_fold_f64_kernel<<<(unsigned)((nvir * nvir + 255) / 256), 256, 0, st>>>(o.part_vv, nz, nvir, o.acc_vv);
+        if (vv_small(nvir))
+            FC_TRY((vv_products<OO_M, OO_N>(o, off, ld, nz, st)));
+        else
+            FC_TRY((vv_products<DG_BM, DG_BN>(o, off, ld, nz, st)));
+        vv_fold_f64_kernel<<<(unsigned)((nvir * nvir + 255) / 256), 256, 0, st>>>(o.part_vv, nz * o.kvv, nvir, o.acc_vv);
         *nl += 2;
     }
-    FC_TRY(check_launch("dgemm_batched_kernel<P_vv>"));
+    FC_TRY(check_launch("vv_fold_f64_kernel"));
     // P_oo: rows i are nvir ld contiguous doubles in both slabs
     const int64_t K = nvir * ld;
     const int64_t kps = ((K + o.splits - 1) / o.splits + DG_BK - 1) / DG_BK * DG_BK;

@@ -70,6 +70,18 @@ def test_densities_f64_match_oracle(fc, naux, nocc, nvir):
     assert np.abs(g - g2).max() <= 1e-13 * np.abs(g2).max()
 
 
+# edges of P_vv's FP64 tiles (64 x 48, and 128 x 64 at nvir 128), K in one and
+# in several ranges; sums of at most nocc^2 nvir terms: 1e-12 of the largest
+@pytest.mark.parametrize("naux,nocc,nvir", [(20, 3, 48), (20, 6, 49), (20, 2, 96), (30, 4, 97), (12, 3, 128),
+                                            (15, 2, 193), (12, 1, 64)])
+def test_densities_f64_tiles(fc, naux, nocc, nvir):
+    from ferric_b200 import rimp2
+    b, eo, ev = synthetic.rimp2_inputs(naux, nocc, nvir)
+    got = rimp2.rimp2_energy_grad_dens(b, eo, ev, precision="f64")[4:]
+    for x, y in zip(got, _ref(b, eo, ev)[1:]):
+        assert np.abs(x - y).max() <= 1e-12 * np.abs(y).max() and np.allclose(x, x.T, rtol=0, atol=1e-15)
+
+
 @pytest.mark.parametrize("naux,nocc,nvir", SHAPES)
 def test_densities_mixed_match_oracle(fc, naux, nocc, nvir):
     from ferric_b200 import rimp2
