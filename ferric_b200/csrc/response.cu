@@ -59,7 +59,10 @@ fc_status response_2c(const double* x_ov, const double* b_ov, const double* vis,
     void* vc;
     FC_TRY(ws_get(WS_PART, (size_t)naux * nov * 8, &vc));
     double* cfit = (double*)vc;
-    const bool residues = 2.0 * naux * (double)naux * nov >= 4e9 && naux <= MG_KMAX;
+    // residues where the products outweigh the operands' conversion: a gradient
+    // chain with them at 2 naux^2 nov = 1.8e9 (naux 532, nov 3225) 1772 us, without
+    // 1853; at 5.5e9 3161 and 3641; at 9e8 1361 and 1318.
+    const bool residues = 2.0 * naux * (double)naux * nov >= 1.5e9 && naux <= MG_KMAX;
     const int splits = residues && nov <= INT32_MAX / 2 ? mg_splits(naux, naux, nov, false) : 1;
     int* flags = nullptr;
     double* gpart = nullptr;

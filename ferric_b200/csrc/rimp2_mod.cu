@@ -293,9 +293,10 @@ struct ChunkPair {
 
 // Where the residue form pays: the conversions (about 100 instructions per
 // element), the passes over G and the dozen launches are spread over enough
-// products.  Measured at the line (B200, gradient): see DESIGN's table.
+// products.  Gradient at 2 naux (nocc nvir)^2 = 1.7e9 (naux 364, nocc 17, nvir
+// 89): 355 us here, 395 DMMA; at 4.7e9 426 and 582; the forms cross near 1.3e9.
 bool mod_grad_pays(int64_t naux, int64_t nocc, int64_t nvir) {
-    return naux <= MG_KMAX && 2.0 * naux * (double)(nocc * nvir) * (double)(nocc * nvir) >= 2e9;
+    return naux <= MG_KMAX && 2.0 * naux * (double)(nocc * nvir) * (double)(nocc * nvir) >= 1.5e9;
 }
 
 // Returns FC_OK with *ran = false where the caller has to take the DMMA form
@@ -521,7 +522,8 @@ fc_status rimp2_grad_mod(const Rimp2Dev& d, cudaStream_t st, double* e_os, doubl
 
 // ------------------------------------------------------------- energies --
 
-// Measured at the line (B200): see DESIGN's table.
+// At 2 naux rows cols = 1.67e9 (naux 420, nocc 18, nvir 110; cols: half of the
+// row's columns on average) 163 us here, 177 DMMA.
 bool mod_energy_pays(int64_t naux, int64_t rows, int64_t cols) {
     return naux <= MG_KMAX && 2.0 * naux * (double)rows * (double)cols >= 1e9;
 }
