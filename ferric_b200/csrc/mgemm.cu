@@ -10,9 +10,9 @@ namespace fc {
 
 namespace {
 
-// 15 pairwise coprime integers up to 256 (the largest ones but for the last,
-// which makes their product P = 2^117.75 an FP64 number within 2^-56.7).
-constexpr int MOD[MG_N] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 193};
+// 16 pairwise coprime integers up to 256 (the largest ones but for the last
+// three, which make their product P = 2^125.22 an FP64 number within 2^-59).
+constexpr int MOD[MG_N] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 197, 193, 179};
 
 constexpr int symmod(int64_t x, int p) {
     int64_t r = x % p;
@@ -37,7 +37,7 @@ constexpr int64_t powmod2(int e, int p) {
     return v;
 }
 constexpr int MAGIC = 0x4B400000;  // bits of 1.5 2^23: MAGIC + v are those of 1.5 2^23 + v, |v| < 2^22
-constexpr int OFF_EXP = 60;        // integers are shifted by 2^60 to be positive
+constexpr int OFF_EXP = 63;        // integers are shifted by 2^63 to be positive
 
 // (P / MOD[l])^-1 mod MOD[l]
 constexpr int crt_inv(int l) {
@@ -50,14 +50,16 @@ constexpr int crt_inv(int l) {
 }
 
 // The remainder theorem in fractions: x / P = sum_l r_l inv_l / p_l (mod 1).
-// F_l = inv_l / p_l rounded to 72 bits: the sum's error, 2^-64 on average, is a
-// sixteenth of the operands' rounding.  Byte b of four F_l is a word, so four
-// terms of the sum's byte b are one dp4a, and the sum is nine 20-bit integers.
+// F_l = inv_l / p_l rounded to 72 bits: the sum's error, 2^-64.6 on average, and
+// that of the 64 bits that are kept, 2^-65.8, are below 2^-61.3 |x| |y| / P even
+// where the rows' norms are the smallest that mg_scale leaves.  Byte b of four
+// F_l is a word, so four terms of the sum's byte b are one dp4a, and the sum is
+// nine 20-bit integers.
 // (In FP64, on pairs of moduli, the same took 30 FP64 instructions per element,
 // which share their pipe with the tensor core: at K = 700 as long as a third of
 // its products.)
 constexpr int FB = 9;                      // bytes of F_l
-constexpr int NG = (MG_N + 3) / 4;         // groups of four moduli
+constexpr int NG = MG_N / 4;               // groups of four moduli
 struct Crt {
     uint32_t f[FB][NG];
     double p64;  // P / 2^64
@@ -73,8 +75,8 @@ constexpr Crt make_crt() {
     c.p64 = (double)(uint64_t)(P >> 64) + (double)(uint64_t)P / 18446744073709551616.0;
     return c;
 }
-static_assert(make_crt().p64 > 0.83 * 18014398509481984.0 && make_crt().p64 < 0.85 * 18014398509481984.0,
-              "P = 0.84 2^118: |x| <= 2^116.7 < P / 2");
+static_assert(make_crt().p64 > 1.166 * 2305843009213693952.0 && make_crt().p64 < 1.168 * 2305843009213693952.0,
+              "P = 1.167 2^125: |x| <= 2^124.2 < P / 2");
 __constant__ Crt c_crt = make_crt();
 
 // The element whose residues (unsigned bytes, any representatives) are the
@@ -83,7 +85,7 @@ __device__ __forceinline__ double crt_element(const uint32_t (&r)[NG]) {
     uint32_t a[FB];
 #pragma unroll
     for (int b = 0; b < FB; ++b) {
-        a[b] = 0;
+        a[b] = b ? 0 : 128;  // the byte that is dropped rounds to nearest
 #pragma unroll
         for (int g = 0; g < NG; ++g) a[b] = __dp4a(r[g], c_crt.f[b][g], a[b]);
     }
@@ -157,129 +159,252 @@ __device__ __forceinline__ void convert16(const F& x, double inv_scale, int8_t* 
     uint32_t lo[16], hi[16];
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-        const long long v = __double2ll_rn(x(i) * inv_scale) + (1ll << OFF_EXP);
+        const unsigned long long v = (unsigned long long)__double2ll_rn(x(i) * inv_scale) + (1ull << OFF_EXP);
         lo[i] = (uint32_t)v;
-        hi[i] = (uint32_t)((unsigned long long)v >> 32);
+        hi[i] = (uint32_t)(v >> 32);
     }
     store_residues<0>(lo, hi, dst, plane);
 }
 
-// Scale of a row with squared norm n2: the power of two s with
-// n2 / s^2 in (2^114.7, 2^116.7].
-__device__ __forceinline__ double mg_scale(double n2, int* bad) {
-    if (n2 == 0.0) return 1.0;
-    if (!(n2 >= 1e-200 && n2 <= 1e200)) {  // also NaN
-        *bad = 1;
-        return 1.0;
-    }
+// Scale of a row with squared norm n2: the power of two s with n2 / s^2 in
+// (2^122.2, 2^124.2]; 0 where the row is out of range (also NaN; `abs`, the sum
+// of |x|, tells a row of zeros from one whose squares underflow).
+__device__ __forceinline__ double mg_scale(double abs, double n2) {
+    if (abs == 0.0) return 1.0;
+    if (!(n2 >= 1e-140 && n2 <= 1e140)) return 0.0;
     int k;
     const double f = frexp(n2, &k);  // n2 = f 2^k, f in [0.5, 1)
-    int e = (116 - k) >> 1;          // n2 4^e < 2^116
-    const int up = k + 2 * (e + 1);  // n2 4^(e+1) = f 2^up, up = 117 or 118
-    if (up == 117 && f <= 0.8122) ++e;  // 0.8122 2^117 < 2^116.7
+    int e = (124 - k) >> 1;          // n2 4^e < 2^124
+    const int up = k + 2 * (e + 1);  // n2 4^(e+1) = f 2^up, up = 125 or 126
+    if (up == 125 && f <= 0.5743) ++e;  // 0.5743 2^125 < 2^124.2
     return ldexp(1.0, -e);
 }
 
-// Scales of the rows from their 2-norms, summed in a fixed order: one warp per
-// row, or with WIDE a CTA of eight (few long rows: 700 x 5577 took 26 us with a
-// warp each, 88 CTAs of dependent loads).
-template <bool WIDE>
-__global__ void __launch_bounds__(256) mg_row_scale_kernel(const double* __restrict__ x, int64_t ld, int64_t R,
-                                                           int64_t K, double* __restrict__ scale, int* bad) {
-    __shared__ double red[32];
-    constexpr int T = WIDE ? 256 : 32;  // threads per row
-    const int64_t r = WIDE ? blockIdx.x : (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (r >= R) return;
-    const int t = threadIdx.x % T;
-    const double* row = x + r * ld;
-    double s[4] = {0.0, 0.0, 0.0, 0.0};
-    int64_t k = t;
-    for (; k + 3 * T < K; k += 4 * T) {
-        double v[4];
+// Sums over the lanes of a warp of eight values each: lane l gets that of
+// v[l / 4], in nine exchanges instead of forty.
+__device__ __forceinline__ double warp_sum8(double (&v)[8]) {
+    const int lane = threadIdx.x & 31;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) v[u] = row[k + T * u];
+    for (int w = 4, o = 16; w > 0; w >>= 1, o >>= 1) {
+        const bool up = lane & o;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) s[u] += v[u] * v[u];
+        for (int i = 0; i < w; ++i) {
+            const double send = up ? v[i] : v[i + w], keep = up ? v[i + w] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
     }
-    for (; k < K; k += T) s[0] += row[k] * row[k];
-    double n2 = (s[0] + s[1]) + (s[2] + s[3]);
-    if constexpr (WIDE) n2 = block_sum(n2, red);
-    else n2 = warp_sum(n2);
-    if (t == 0) scale[r] = mg_scale(n2, bad);
+    double s = v[0];
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    return s + __shfl_xor_sync(0xffffffffu, s, 1);
 }
 
-// Partial squared norms of the columns over 256 rows each.
-__global__ void __launch_bounds__(256) mg_col_part_kernel(const double* __restrict__ x, int64_t ld, int64_t R,
-                                                          int64_t K, double* __restrict__ part) {
-    const int64_t c = (int64_t)blockIdx.x * 256 + threadIdx.x;
-    if (c >= R) return;
-    const int64_t k0 = (int64_t)blockIdx.y * 256, k1 = k0 + 256 < K ? k0 + 256 : K;
-    double s[4] = {0.0, 0.0, 0.0, 0.0};
-    int64_t k = k0;
-    for (; k + 3 < k1; k += 4) {
-        double v[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) v[u] = x[(k + u) * ld + c];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) s[u] += v[u] * v[u];
-    }
-    for (; k < k1; ++k) s[0] += x[k * ld + c] * x[k * ld + c];
-    part[(int64_t)blockIdx.y * R + c] = (s[0] + s[1]) + (s[2] + s[3]);
-}
-
-__global__ void __launch_bounds__(256) mg_col_scale_kernel(const double* __restrict__ part, int64_t R, int64_t nch,
-                                                           double* __restrict__ scale, int* bad) {
-    const int64_t c = (int64_t)blockIdx.x * 256 + threadIdx.x;
-    if (c >= R) return;
-    double s = 0.0;
-    for (int64_t y = 0; y < nch; ++y) s += part[y * R + c];
-    scale[c] = mg_scale(s, bad);
-}
-
-// Rows of x -> residues.  A warp takes 512 k of one row: coalesced loads into
-// its shared-memory strip (one double of padding per 16, so the 16 k a lane
-// then reads lie in other banks than its neighbours'), 16 bytes of each plane
-// per lane.  Bound by the integer pipes: about 100 instructions per element.
-__global__ void __launch_bounds__(256, 4) mg_rows_kernel(const double* __restrict__ x, int64_t ld, int64_t R, int64_t K,
-                                                      int64_t kp, const double* __restrict__ scale,
-                                                      int8_t* __restrict__ out) {
-    __shared__ double sm[8][512 + 32];
+// Partial (sum |x|, sum x^2) of the rows over 128 columns, rowp[column tile][R],
+// and of the columns over 128 rows, colp[row tile][C], in one read of x.
+__global__ void __launch_bounds__(256) mg_stats_kernel(const double* __restrict__ x, int64_t ld, int64_t R, int64_t C,
+                                                       double2* __restrict__ rowp, double2* __restrict__ colp,
+                                                       const int* bad) {
+    __shared__ double2 sh[8][128];
+    if (*bad) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t segs = (kp + 511) / 512;
-    const int64_t id = (int64_t)blockIdx.x * 8 + warp;
-    if (id >= R * segs) return;
-    const int64_t r = id / segs, k0 = (id % segs) * 512;
-    const double* row = x + r * ld;
-    double* s = sm[warp];
+    const int64_t c0 = (int64_t)blockIdx.x * 128 + lane, r0 = (int64_t)blockIdx.y * 128 + warp * 16;
+    double ca[4] = {}, cq[4] = {};
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        double a[8], q[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int64_t r = r0 + 8 * h + i;
+            double v[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = r < R && c0 + 32 * j < C ? x[r * ld + c0 + 32 * j] : 0.0;
+            a[i] = q[i] = 0.0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const double w = fabs(v[j]);
+                a[i] += w;
+                q[i] = fma(w, w, q[i]);
+                ca[j] += w;
+                cq[j] = fma(w, w, cq[j]);
+            }
+        }
+        const double sa = warp_sum8(a), sq = warp_sum8(q);
+        const int64_t r = r0 + 8 * h + (lane >> 2);
+        if ((lane & 3) == 0 && r < R) rowp[(int64_t)blockIdx.x * R + r] = make_double2(sa, sq);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sh[warp][lane + 32 * j] = make_double2(ca[j], cq[j]);
+    __syncthreads();
+    const int64_t c = (int64_t)blockIdx.x * 128 + threadIdx.x;
+    if (threadIdx.x < 128 && c < C) {
+        double2 s = sh[0][threadIdx.x];
+#pragma unroll
+        for (int w = 1; w < 8; ++w) {
+            s.x += sh[w][threadIdx.x].x;
+            s.y += sh[w][threadIdx.x].y;
+        }
+        colp[(int64_t)blockIdx.y * C + c] = s;
+    }
+}
+
+// Lanes that add up one entry's tiles: few tiles leave most of a warp idle.
+__host__ __device__ inline int fold_lanes(int64_t tiles) { return tiles > 32 ? 32 : 4; }
+
+// sum over the tiles of part[tile][n] for entry e (0 past the last), L lanes each.
+__device__ __forceinline__ double2 fold_tiles(const double2* __restrict__ part, int64_t tiles, int64_t n, int64_t e,
+                                              int L) {
+    double2 s = make_double2(0.0, 0.0);
+    if (e < n)
+        for (int64_t t = threadIdx.x & (L - 1); t < tiles; t += L) {
+            const double2 v = part[t * n + e];
+            s.x += v.x;
+            s.y += v.y;
+        }
+    for (int o = L >> 1; o > 0; o >>= 1) {
+        s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+        s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+    }
+    return s;
+}
+
+// The sums and scales along each axis (blockIdx.y), and from the shorter one
+// the squared Frobenius norm's partial sums.
+__global__ void __launch_bounds__(256) mg_stats_fold_kernel(const double2* __restrict__ rowp,
+                                                            const double2* __restrict__ colp, const MgMat x,
+                                                            const int* bad) {
+    __shared__ double red[32];
+    const int axis = blockIdx.y;
+    const double2* part = axis ? colp : rowp;
+    if (*bad) return;
+    const int64_t tiles = (x.n[1 - axis] + 127) / 128;
+    const int L = fold_lanes(tiles), t = threadIdx.x;
+    const int64_t e = (int64_t)blockIdx.x * (256 / L) + t / L;
+    if (e - t / L >= x.n[axis]) return;
+    const double2 s = fold_tiles(part, tiles, x.n[axis], e, L);
+    const bool lead = (t & (L - 1)) == 0 && e < x.n[axis];
+    if (lead) {
+        x.sum[axis][e] = s;
+        x.scale[axis][e] = mg_scale(s.x, s.y);
+    }
+    if (axis != x.short_axis()) return;
+    const double f = block_sum(lead ? s.y : 0.0, red);
+    if (t == 0) x.f2[blockIdx.x] = f;
+}
+
+// The guard's left side for the operand rows along `axis` of x: with the
+// partner's sums S_k = sum_n |y_nk|, T_k = sum_n y_nk^2,
+//     sum_n (sum_k |x_k y_nk|)^2 >= max((sum_k |x_k| S_k)^2 / N, sum_k x_k^2 T_k).
+// part[tile][rows]: those two sums over the k of a tile.
+__global__ void __launch_bounds__(256) mg_guard_fold_kernel(const double2* __restrict__ part, int64_t tiles,
+                                                            MgMat x, int axis, MgMat y, int py, int* bad) {
+    __shared__ double red[32];
+    double f = 0.0;
+    const int64_t fa = y.short_axis(), fe = 256 / fold_lanes((y.n[1 - fa] + 127) / 128);
+    for (int64_t k = threadIdx.x; k < (y.n[fa] + fe - 1) / fe; k += 256) f += y.f2[k];
+    f = block_sum(f, red);
+    if (threadIdx.x == 0) red[0] = f;
+    __syncthreads();
+    const int L = fold_lanes(tiles);
+    const int64_t r = (int64_t)blockIdx.x * (256 / L) + threadIdx.x / L;
+    const double2 s = fold_tiles(part, tiles, x.n[axis], r, L);
+    const double low = fmax(s.x * s.x / (double)y.n[py], s.y);
+    if (r < x.n[axis] && low < MG_GUARD * MG_GUARD * x.sum[axis][r].y * red[0]) *bad = 1;
+}
+
+// Rows of x -> residues (WRITE), and the guard's sums against the partner's
+// (GUARD).  A warp takes 512 k of one row: coalesced loads into its
+// shared-memory strip (one double of padding per 16, so the 16 k a lane then
+// reads lie in other banks than its neighbours'), 16 bytes of each plane per
+// lane.  Bound by the integer pipes: about 110 instructions per element.  The
+// warps of a CTA take the same k of eight rows, so the partner's sums come
+// from L1.
+template <bool WRITE, bool GUARD>
+__global__ void __launch_bounds__(256, 4) mg_rows_kernel(const MgMat x, int64_t kp, const double2* __restrict__ ys,
+                                                         double2* __restrict__ part, int8_t* __restrict__ out,
+                                                         int* bad) {
+    __shared__ double sm[WRITE ? 8 : 1][512 + 32];
+    const int64_t R = x.n[0], K = x.n[1];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t r = (int64_t)blockIdx.x * 8 + warp, k0 = (int64_t)blockIdx.y * 512;
+    if (*bad || r >= R) return;
+    const double* row = x.p + r * x.ld;
+    double* s = sm[WRITE ? warp : 0];
+    double l1 = 0.0, l2 = 0.0;
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
         const int k = i * 32 + lane;
-        s[k + (k >> 4)] = k0 + k < K ? row[k0 + k] : 0.0;
+        const double v = k0 + k < K ? row[k0 + k] : 0.0;
+        if (WRITE) s[k + (k >> 4)] = v;
+        if (GUARD && k0 + k < K) {
+            const double2 t = ys[k0 + k];
+            l1 = fma(fabs(v), t.x, l1);
+            l2 = fma(v * v, t.y, l2);
+        }
     }
-    __syncwarp();
-    const int64_t kk = k0 + lane * 16;
-    if (kk >= kp) return;
-    const double* mine = s + lane * 17;
-    convert16([&](int i) { return mine[i]; }, 1.0 / scale[r], out + r * kp + kk, R * kp);
+    if (GUARD) {
+        l1 = warp_sum(l1);
+        l2 = warp_sum(l2);
+        if (lane == 0) part[(int64_t)blockIdx.y * R + r] = make_double2(l1, l2);
+    }
+    if constexpr (WRITE) {
+        const double scale = x.scale[0][r];
+        if (!(scale > 0.0)) {
+            if (lane == 0) *bad = 1;
+            return;
+        }
+        __syncwarp();
+        const int64_t kk = k0 + lane * 16;
+        if (kk >= kp) return;
+        const double* mine = s + lane * 17;
+        convert16([&](int i) { return mine[i]; }, 1.0 / scale, out + r * kp + kk, R * kp);
+    }
 }
 
 // Columns of x (K x R) -> residues: a CTA takes 32 columns by 128 k through
 // shared memory (columns rotated by 4 per 16 k against bank conflicts).
-__global__ void __launch_bounds__(256, 4) mg_cols_kernel(const double* __restrict__ x, int64_t ld, int64_t R, int64_t K,
-                                                      int64_t kp, const double* __restrict__ scale,
-                                                      int8_t* __restrict__ out) {
-    __shared__ double sm[128 * 32];
+template <bool WRITE, bool GUARD>
+__global__ void __launch_bounds__(256, 4) mg_cols_kernel(const MgMat x, int64_t kp, const double2* __restrict__ ys,
+                                                         double2* __restrict__ part, int8_t* __restrict__ out,
+                                                         int* bad) {
+    __shared__ double sm[WRITE ? 128 * 32 : 1];
+    __shared__ double2 sg[GUARD ? 8 : 1][32];
+    if (__syncthreads_or(*bad)) return;  // (another CTA may raise it meanwhile)
+    const int64_t R = x.n[1], K = x.n[0];
     const int64_t c0 = (int64_t)blockIdx.x * 32, k0 = (int64_t)blockIdx.y * 128;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double l1 = 0.0, l2 = 0.0;
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-        const int idx = i * 256 + threadIdx.x, k = idx >> 5, c = idx & 31;
-        sm[k * 32 + ((c + 4 * (k >> 4)) & 31)] = k0 + k < K && c0 + c < R ? x[(k0 + k) * ld + c0 + c] : 0.0;
+        const int k = i * 8 + warp;
+        const double v = k0 + k < K && c0 + lane < R ? x.p[(k0 + k) * x.ld + c0 + lane] : 0.0;
+        if (WRITE) sm[k * 32 + ((lane + 4 * (k >> 4)) & 31)] = v;
+        if (GUARD && k0 + k < K) {
+            const double2 t = ys[k0 + k];
+            l1 = fma(fabs(v), t.x, l1);
+            l2 = fma(v * v, t.y, l2);
+        }
     }
+    if (GUARD) sg[warp][lane] = make_double2(l1, l2);
     __syncthreads();
-    const int c = threadIdx.x >> 3, kg = threadIdx.x & 7;
-    if (c0 + c >= R) return;
-    const double* mine = sm + kg * 16 * 32 + ((c + 4 * kg) & 31);
-    convert16([&](int i) { return mine[i * 32]; }, 1.0 / scale[c0 + c], out + (c0 + c) * kp + k0 + kg * 16, R * kp);
+    if (GUARD && warp == 0 && c0 + lane < R) {
+        double2 t = sg[0][lane];
+#pragma unroll
+        for (int w = 1; w < 8; ++w) {
+            t.x += sg[GUARD ? w : 0][lane].x;
+            t.y += sg[GUARD ? w : 0][lane].y;
+        }
+        part[(int64_t)blockIdx.y * R + c0 + lane] = t;
+    }
+    if constexpr (WRITE) {
+        const int c = threadIdx.x >> 3, kg = threadIdx.x & 7;
+        if (c0 + c >= R) return;
+        const double scale = x.scale[1][c0 + c];
+        if (!(scale > 0.0)) {
+            *bad = 1;
+            return;
+        }
+        const double* mine = sm + kg * 16 * 32 + ((c + 4 * kg) & 31);
+        convert16([&](int i) { return mine[i * 32]; }, 1.0 / scale, out + (c0 + c) * kp + k0 + kg * 16, R * kp);
+    }
 }
 
 // ------------------------------------------------------------------ GEMM --
@@ -303,24 +428,27 @@ struct MgArgs {
     const double* sn;
     MgOut o;
     uint32_t* scratch;
+    const int* bad;
     int* err;
 };
 
-// Persistent: a CTA takes tiles of 128 x 256; per tile it runs the 15 moduli
+// Persistent: a CTA takes tiles of 128 x 256; per tile it runs the 16 moduli
 // one after another, each over all of K, into one of two 256-column TMEM
 // accumulators, so the reduction of one modulus overlaps the products of the
 // next.  Sixteen warps reduce the int32 sums modulo p and park the residue
-// bytes of the tile (480 KiB per CTA: 71 MB in all, which L2 holds; twice that,
+// bytes of the tile (512 KiB per CTA: 76 MB in all, which L2 holds; twice that,
 // to form a tile's results under the next one's reductions, cost 23% at K =
 // 4800) until the last modulus is done; then each thread reads its own bytes
 // back and forms the FP64 results.  Lanes are consecutive m, so stores to
 // out[n * ld + m] are coalesced.
-// Bound by the int8 products at large K (16611^2 x 4800: 15.8 ms, 168 TFLOP/s
-// FP64-equivalent) and by the epilogue below K ~ 1000.  Sixteen epilogue warps
-// with the dp4a remainder theorem instead of eight with the FP64 one: 5577^2 x
-// 700 0.54 -> 0.48 ms, 16384^2 x 2150 8.0 -> 7.55.
+// Bound by the int8 products at large K (4800 x 16611 x 16611: 16.05 ms, 165
+// TFLOP/s FP64-equivalent) and by the epilogue below K ~ 1000.  Sixteen epilogue
+// warps with the dp4a remainder theorem instead of eight with the FP64 one: 5577^2
+// x 700 0.54 -> 0.48 ms, 16384^2 x 2150 8.0 -> 7.55 (15 moduli; the sixteenth costs
+// 5-7%: 2150 x 16384 x 16384 6.74 -> 7.21 ms, 700 x 5577 x 5577 0.286 -> 0.303).
 __global__ void __launch_bounds__(THREADS, 1)
     mg_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const MgArgs p) {
+    if (*p.bad) return;  // the product is not used
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw_u32 = smem_u32(smem_raw);
     const uint32_t base_u32 = (raw_u32 + 1023u) & ~1023u;
@@ -488,8 +616,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                 uint32_t e[4][NG];
 #pragma unroll
                 for (int g = 0; g < NG; ++g) {
-                    const uint32_t a0 = x[4 * g], a1 = 4 * g + 1 < MG_N ? x[4 * g + 1] : 0u;
-                    const uint32_t a2 = 4 * g + 2 < MG_N ? x[4 * g + 2] : 0u, a3 = 4 * g + 3 < MG_N ? x[4 * g + 3] : 0u;
+                    const uint32_t a0 = x[4 * g], a1 = x[4 * g + 1], a2 = x[4 * g + 2], a3 = x[4 * g + 3];
                     const uint32_t t0 = __byte_perm(a0, a1, 0x5140), t1 = __byte_perm(a0, a1, 0x7362);
                     const uint32_t u0 = __byte_perm(a2, a3, 0x5140), u1 = __byte_perm(a2, a3, 0x7362);
                     e[0][g] = __byte_perm(t0, u0, 0x5410);
@@ -514,32 +641,61 @@ __global__ void __launch_bounds__(THREADS, 1)
 
 }  // namespace
 
-fc_status mg_convert_rows(const double* src, int64_t ld, int64_t R, int64_t K, MgOperand* o, int* bad,
-                          cudaStream_t st) {
-    o->rows = o->plane = R;
-    o->K = K;
-    o->kp = mg_kp(K);
-    // one warp per row where that alone fills the chip's 64 warps per SM
-    if (R < 64 * ctx().sm_count && K >= 1024)
-        mg_row_scale_kernel<true><<<(unsigned)R, 256, 0, st>>>(src, ld, R, K, o->scale, bad);
-    else
-        mg_row_scale_kernel<false><<<(unsigned)((R + 7) / 8), 256, 0, st>>>(src, ld, R, K, o->scale, bad);
-    const int64_t work = R * ((o->kp + 511) / 512);
-    mg_rows_kernel<<<(unsigned)((work + 7) / 8), 256, 0, st>>>(src, ld, R, K, o->kp, o->scale, o->r);
-    return check_launch("residue conversion (rows)");
+MgMat mg_mat(const double* p, int64_t ld, int64_t R, int64_t C, double* stat) {
+    MgMat x;
+    x.p = p;
+    x.ld = ld;
+    x.n[0] = R;
+    x.n[1] = C;
+    x.sum[0] = (double2*)stat;
+    x.sum[1] = x.sum[0] + R;
+    x.scale[0] = stat + 2 * (R + C);
+    x.scale[1] = x.scale[0] + R;
+    x.f2 = x.scale[1] + C;
+    return x;
 }
 
-fc_status mg_convert_cols(const double* src, int64_t ld, int64_t R, int64_t K, MgOperand* o, double* part, int* bad,
-                          cudaStream_t st) {
-    o->rows = o->plane = R;
-    o->K = K;
-    o->kp = mg_kp(K);
-    const int64_t nch = mg_colchunks(K);
-    mg_col_part_kernel<<<dim3((unsigned)((R + 255) / 256), (unsigned)nch), 256, 0, st>>>(src, ld, R, K, part);
-    mg_col_scale_kernel<<<(unsigned)((R + 255) / 256), 256, 0, st>>>(part, R, nch, o->scale, bad);
-    mg_cols_kernel<<<dim3((unsigned)((R + 31) / 32), (unsigned)(o->kp / 128)), 256, 0, st>>>(src, ld, R, K, o->kp,
-                                                                                            o->scale, o->r);
-    return check_launch("residue conversion (columns)");
+fc_status mg_stats(const MgMat& x, double* part, const int* bad, cudaStream_t st) {
+    const int64_t R = x.n[0], C = x.n[1], tc = (C + 127) / 128, tr = (R + 127) / 128;
+    double2 *rowp = (double2*)part, *colp = rowp + R * tc;
+    mg_stats_kernel<<<dim3((unsigned)tc, (unsigned)tr), 256, 0, st>>>(x.p, x.ld, R, C, rowp, colp, bad);
+    const int64_t pr = 256 / fold_lanes(tc), pc = 256 / fold_lanes(tr);
+    const dim3 g((unsigned)std::max((R + pr - 1) / pr, (C + pc - 1) / pc), 2);
+    mg_stats_fold_kernel<<<g, 256, 0, st>>>(rowp, colp, x, bad);
+    return check_launch("residue sums");
+}
+
+// One pass over x: residues (r) and, with y, the guard's sums and their check.
+static fc_status mg_pass(const MgMat& x, int axis, int8_t* r, const MgMat* y, int py, double* part, int* bad,
+                         cudaStream_t st) {
+    const int64_t R = x.n[axis], K = x.n[1 - axis], kp = mg_kp(K);
+    const double2* ys = y ? y->sum[1 - py] : nullptr;
+    double2* gp = (double2*)part;
+    const int64_t tiles = axis ? kp / 128 : (kp + 511) / 512;
+    const dim3 g = axis ? dim3((unsigned)((R + 31) / 32), (unsigned)tiles) : dim3((unsigned)((R + 7) / 8), (unsigned)tiles);
+    if (axis) {
+        if (r && y) mg_cols_kernel<true, true><<<g, 256, 0, st>>>(x, kp, ys, gp, r, bad);
+        else if (r) mg_cols_kernel<true, false><<<g, 256, 0, st>>>(x, kp, ys, gp, r, bad);
+        else mg_cols_kernel<false, true><<<g, 256, 0, st>>>(x, kp, ys, gp, r, bad);
+    } else {
+        if (r && y) mg_rows_kernel<true, true><<<g, 256, 0, st>>>(x, kp, ys, gp, r, bad);
+        else if (r) mg_rows_kernel<true, false><<<g, 256, 0, st>>>(x, kp, ys, gp, r, bad);
+        else mg_rows_kernel<false, true><<<g, 256, 0, st>>>(x, kp, ys, gp, r, bad);
+    }
+    const int64_t per = 256 / fold_lanes(tiles);
+    if (y) mg_guard_fold_kernel<<<(unsigned)((R + per - 1) / per), 256, 0, st>>>(gp, tiles, x, axis, *y, py, bad);
+    return check_launch("residue conversion");
+}
+
+fc_status mg_convert(const MgMat& x, int axis, int8_t* r, const MgMat* y, int py, double* part, int* bad,
+                     cudaStream_t st, MgOperand* o) {
+    const int64_t R = x.n[axis], K = x.n[1 - axis];
+    *o = MgOperand{r, x.scale[axis], R, K, mg_kp(K), R};
+    return mg_pass(x, axis, r, y, py, part, bad, st);
+}
+
+fc_status mg_guard(const MgMat& x, int axis, const MgMat& y, int py, double* part, int* bad, cudaStream_t st) {
+    return mg_pass(x, axis, nullptr, &y, py, part, bad, st);
 }
 
 // Tile c of the product in launch order: split-major, then groups of GM m-tiles,
@@ -605,7 +761,7 @@ __global__ void __launch_bounds__(1024) mg_tiles_kernel(TileGrid g, int4* __rest
 size_t mg_scratch_bytes() { return CTA_SCRATCH * (size_t)ctx().sm_count; }
 
 fc_status mg_gemm(const MgOperand& A, const MgOperand& B, const MgOut& out, const int4* items, int64_t nitems,
-                  void* scratch, int* err, cudaStream_t st) {
+                  void* scratch, int* flags, cudaStream_t st) {
     static std::atomic<uint64_t> done{0};
     uint64_t bit = 0;
     if (attrs_needed(done, &bit)) {
@@ -617,7 +773,7 @@ fc_status mg_gemm(const MgOperand& A, const MgOperand& B, const MgOut& out, cons
     FC_TRY(make_tmap_i8_2d(&ta, A.r, A.kp, (uint64_t)(MG_N - 1) * A.plane + A.rows, A.kp, MG_KT, MG_BM));
     FC_TRY(make_tmap_i8_2d(&tb, B.r, B.kp, (uint64_t)(MG_N - 1) * B.plane + B.rows, B.kp, MG_KT, MG_BN));
     const MgArgs a{items,   nitems,  (int)A.rows, (int)B.rows, (int)A.plane, (int)B.plane,
-                   A.scale, B.scale, out, (uint32_t*)scratch, err};
+                   A.scale, B.scale, out, (uint32_t*)scratch, flags, flags + 1};
     const int grid = (int)std::min<int64_t>(nitems, ctx().sm_count);
     if (grid > 0)
         mg_gemm_kernel<<<grid, THREADS, SMEM, st>>>(ta, tb, a);
@@ -642,8 +798,8 @@ fc_status mg_fold(const double* part, int splits, int64_t M, int64_t N, double a
 int mg_splits(int64_t M, int64_t N, int64_t K, bool upper) {
     const int64_t tiles = std::max<int64_t>(1, mg_tiles(M, N, 1, upper, 1, nullptr)), nks = mg_kp(K) / MG_KT;
     int64_t s = std::max<int64_t>(1, std::min(ctx().sm_count / tiles, nks / 4));
-    s = std::max(s, (K + MG_KMAX - 1) / MG_KMAX);  // the ranges' sums stay exact
-    const int64_t kps = (nks + s - 1) / s;
+    // the ranges' sums stay exact: at most MG_KMAX elements each
+    const int64_t kps = std::min((nks + s - 1) / s, MG_KMAX / MG_KT);
     return (int)((nks + kps - 1) / kps);
 }
 
@@ -651,45 +807,39 @@ fc_status mg_multiply(const MgSrc& a, const MgSrc& b, int64_t K, const MgOut& ou
                       cudaStream_t st, bool* room) {
     *room = false;
     const bool same = a.p == b.p && a.ld == b.ld && a.rows == b.rows && a.cols == b.cols;
-    const int64_t seg = splits > 1 ? K : std::min<int64_t>(K, MG_KMAX / MG_KT * MG_KT);
     const int64_t rmax = std::max(a.rows, b.rows);
-    if (MG_N * rmax + MG_BN > INT32_MAX || K > INT32_MAX) return FC_OK;
-    const TileGrid gf = tile_grid(a.rows, b.rows, seg, upper, splits);
-    const TileGrid gl = tile_grid(a.rows, b.rows, K % seg ? K % seg : seg, upper, splits);
-    const int64_t nfull = mg_tiles(a.rows, b.rows, seg, upper, splits, nullptr);
+    const TileGrid g = tile_grid(a.rows, b.rows, K, upper, splits);
+    // the sums over a range of K stay exact, an item's word holds its split, the launches' grids their tiles
+    const int64_t gmax = 65535 * 128;
+    if (std::min<int64_t>(K, (int64_t)g.kps * MG_KT) > MG_KMAX || splits > 2047 || rmax > gmax || K > gmax) return FC_OK;
+    const int64_t items = mg_tiles(a.rows, b.rows, K, upper, splits, nullptr);
     size_t off = 0;
     auto take = [&](size_t bytes) {
         const size_t o = off;
         off += (bytes + 255) & ~size_t(255);
         return o;
     };
-    const size_t osa = take(a.rows * 8), osb = take(b.rows * 8);
-    const size_t opart = take((a.cols || b.cols) ? mg_colpart(rmax, seg) * 8 : 0);
-    const size_t ofull = take(nfull * sizeof(int4)), olast = take(nfull * sizeof(int4));
+    const size_t osa = take(mg_stat_doubles(a.rows, K) * 8), osb = take(same ? 0 : mg_stat_doubles(b.rows, K) * 8);
+    const size_t opart = take(mg_part_doubles(rmax, K) * 8), oitems = take(items * sizeof(int4));
     void* mg[WS_MG_SLOTS];
-    if (!ws_get_mg({mg_bytes(a.rows, seg), same ? 0 : mg_bytes(b.rows, seg), 0, mg_scratch_bytes(), off}, mg))
+    if (!ws_get_mg({mg_bytes(a.rows, K), same ? 0 : mg_bytes(b.rows, K), 0, mg_scratch_bytes(), off}, mg))
         return FC_OK;
     *room = true;
     char* m = (char*)mg[4];
-    mg_tiles_kernel<<<1, 1024, 0, st>>>(gf, (int4*)(m + ofull));
-    if (K % seg) mg_tiles_kernel<<<1, 1024, 0, st>>>(gl, (int4*)(m + olast));
-    auto convert = [&](const MgSrc& s, void* r, size_t os, int64_t k0, int64_t k, MgOperand* o) {
-        *o = MgOperand{(int8_t*)r, (double*)(m + os)};
-        return s.cols ? mg_convert_cols(s.p + k0 * s.ld, s.ld, s.rows, k, o, (double*)(m + opart), flags, st)
-                      : mg_convert_rows(s.p + k0, s.ld, s.rows, k, o, flags, st);
+    double* part = (double*)(m + opart);
+    int4* list = (int4*)(m + oitems);
+    mg_tiles_kernel<<<1, 1024, 0, st>>>(g, list);
+    auto mat = [&](const MgSrc& s, size_t o) {
+        return mg_mat(s.p, s.ld, s.cols ? K : s.rows, s.cols ? s.rows : K, (double*)(m + o));
     };
-    for (int64_t k0 = 0; k0 < K; k0 += seg) {
-        const int64_t k = std::min(seg, K - k0);
-        MgOperand A, B;
-        FC_TRY(convert(a, mg[0], osa, k0, k, &A));
-        if (same) B = A;
-        else FC_TRY(convert(b, mg[1], osb, k0, k, &B));
-        MgOut o = out;
-        if (k0) o.accumulate = 1;
-        const bool part = k != seg;
-        FC_TRY(mg_gemm(A, B, o, (const int4*)(m + (part ? olast : ofull)), nfull, mg[3], flags + 1, st));
-    }
-    return FC_OK;
+    const MgMat A = mat(a, osa), B = same ? A : mat(b, osb);
+    FC_TRY(mg_stats(A, part, flags, st));
+    if (!same) FC_TRY(mg_stats(B, part, flags, st));
+    MgOperand oa, ob;
+    FC_TRY(mg_convert(A, a.cols, (int8_t*)mg[0], &B, b.cols, part, flags, st, &oa));
+    if (same) ob = oa;
+    else FC_TRY(mg_convert(B, b.cols, (int8_t*)mg[1], &A, a.cols, part, flags, st, &ob));
+    return mg_gemm(oa, ob, out, list, items, mg[3], flags, st);
 }
 
 }  // namespace fc

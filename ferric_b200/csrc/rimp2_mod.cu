@@ -9,8 +9,8 @@
 // Every unordered pair is formed once and both of its amplitude blocks come
 // from it, so the products are 2 naux nvir^2 P + 2 naux nov^2, P the number of
 // unordered pairs.  The DMMA kernels of rimp2_f64.cu keep the integrals on
-// chip but run at 37 TFLOP/s at most; here a GEMM runs at 144-168 TFLOP/s
-// (FP64 products, measured at K = 2150 and 4800) and the passes over G and Tt
+// chip but run at 37 TFLOP/s at most; here a GEMM runs at 142-165 TFLOP/s
+// (FP64 products, adjoints at naux = 2150 and 4800) and the passes over G and Tt
 // (about 10 bytes per element beside 4 naux flops) are a tenth of the time.
 #include <algorithm>
 #include <cmath>
@@ -42,6 +42,7 @@ struct AmpArgs {
     int same;            // I == J: pairs i <= j, only columns >= rows of g are given
     int has_kappa;
     double kappa;
+    const int* bad;      // up: g is not used
     double* part;        // [item][3]: E_os, E_ss, sum of t Tt
     double* vir;         // [item][2 AT]: sums of t Tt by virtual of ta and of tb
 };
@@ -53,6 +54,7 @@ struct AmpArgs {
 // flight: tiles of 64 x 64 (two CTAs per SM) ran at 1.7 TB/s.
 template <int MODE>
 __global__ void __launch_bounds__(AN) amp_kernel(const AmpArgs p) {
+    if (*p.bad) return;
     extern __shared__ __align__(16) double sm[];
     __shared__ double red[32];
     double* X = sm;              // X[a][b] = (ia|jb), then Tt_ij[a, b]
@@ -300,7 +302,7 @@ bool mod_grad_pays(int64_t naux, int64_t nocc, int64_t nvir) {
 }
 
 // Returns FC_OK with *ran = false where the caller has to take the DMMA form
-// (no room for the residues, or operand rows out of range).
+// (no room for the residues, operand rows out of range, or a product's guard).
 fc_status rimp2_grad_mod(const Rimp2Dev& d, cudaStream_t st, double* e_os, double* e_ss, double* gamma,
                          double* de_docc, double* de_dvir, fc_stats* stats, const GammaSink* sink,
                          const DensOut* dens, bool* ran) {
@@ -354,12 +356,15 @@ fc_status rimp2_grad_mod(const Rimp2Dev& d, cudaStream_t st, double* e_os, doubl
     for (int64_t J = 0; J < nch; ++J) bq_bytes += mg_bytes(naux, std::min(cc, nocc - J * cc) * nvir);
     const int64_t nvch = (np_max + VP - 1) / VP;
     const size_t np_items = (size_t)np_max * ntiles;
-    auto misc = [&](Carver& c, double** bts, double** bqs, double** ts, double** cpart, int4** items) {
-        *bts = c.take<double>(nov);
-        *bqs = c.take<double>(naux * nch);
-        *ts = c.take<double>(cv);
-        *cpart = c.take<double>(std::max(mg_colpart(nov, naux), mg_colpart(cv, cv)));
-        *items = c.take<int4>(ht.size());
+    double *bstat, *tstat, *mpart;
+    std::vector<double*> qstat((size_t)nch, nullptr);  // sums of b_ov's column chunks
+    int4* items;
+    auto misc = [&](Carver& c) {
+        bstat = c.take<double>(mg_stat_doubles(naux, nov));
+        for (int64_t J = 0; nch > 1 && J < nch; ++J) qstat[(size_t)J] = c.take<double>(mg_stat_doubles(naux, cv));
+        tstat = c.take<double>(mg_stat_doubles(cv, cv));
+        mpart = c.take<double>(std::max(mg_part_doubles(naux, nov), mg_part_doubles(cv, cv)));
+        items = c.take<int4>(ht.size());
     };
     void *vT, *vpairs, *vpart, *vout;
     DensF64 dx{};
@@ -373,13 +378,11 @@ fc_status rimp2_grad_mod(const Rimp2Dev& d, cudaStream_t st, double* e_os, doubl
     FC_TRY(ws_get(WS_PART, (np_items * (3 + 2 * AT) + (size_t)np_max * 3 + (size_t)nvch * ntile * AT) * 8, &vpart));
     FC_TRY(ws_get(WS_OUT, (size_t)(nocc + 2) * 8 + 64, &vout));
     Carver cm;
-    double *bts, *bqs, *ts, *cpart;
-    int4* items;
-    misc(cm, &bts, &bqs, &ts, &cpart, &items);
+    misc(cm);
     void* mg[WS_MG_SLOTS];
     if (!ws_get_mg({mg_bytes(nov, naux), bq_bytes, mg_bytes(cv, cv), mg_scratch_bytes(), cm.off}, mg)) return FC_OK;
     cm = Carver{(char*)mg[4], 0};
-    misc(cm, &bts, &bqs, &ts, &cpart, &items);
+    misc(cm);
 
     double* T = (double*)vT;
     double* part = (double*)vpart;
@@ -403,9 +406,12 @@ fc_status rimp2_grad_mod(const Rimp2Dev& d, cudaStream_t st, double* e_os, doubl
         FC_TRY(timing_events2((int)(2 * ncp), &ev2));
         FC_CUDA(cudaEventRecord(c.ev0, st));
     }
-    MgOperand bt{(int8_t*)mg[0], bts};
-    FC_TRY(mg_convert_cols(d.b_ov, nov, nov, naux, &bt, cpart, flags, st));
-    int64_t nl = 3;
+    const MgMat B = mg_mat(d.b_ov, nov, naux, nov, bstat);
+    MgOperand bt;
+    FC_TRY(mg_stats(B, mpart, flags, st));
+    FC_TRY(mg_convert(B, 1, (int8_t*)mg[0], &B, 1, mpart, flags, st, &bt));
+    int64_t nl = 4;
+    std::vector<MgMat> bm((size_t)nch);
     int nadj = 0;
     double adj_flops = 0.0, adj_bytes = 0.0;
     size_t bq_off = 0;
@@ -415,7 +421,7 @@ fc_status rimp2_grad_mod(const Rimp2Dev& d, cudaStream_t st, double* e_os, doubl
         MgOperand& b = bq[(size_t)(k0 / cc)];
         if (stats) FC_CUDA(cudaEventRecord(ev2[2 * nadj], st));
         char& s = seen[(size_t)(r0 / cc)];
-        FC_TRY(mg_gemm(t, b, MgOut{gamma + r0 * nvir, nov, 0, 4.0, s}, its, nits, mg[3], flags + 1, st));
+        FC_TRY(mg_gemm(t, b, MgOut{gamma + r0 * nvir, nov, 0, 4.0, s}, its, nits, mg[3], flags, st));
         s = 1;
         if (stats) FC_CUDA(cudaEventRecord(ev2[2 * nadj + 1], st));
         ++nadj;
@@ -426,17 +432,9 @@ fc_status rimp2_grad_mod(const Rimp2Dev& d, cudaStream_t st, double* e_os, doubl
     for (int64_t x = 0; x < ncp; ++x) {
         const ChunkPair& cp = cps[(size_t)x];
         const int64_t J = cp.j0 / cc, ri = cp.ni * nvir, rj = cp.nj * nvir;
-        if (!bq[(size_t)J].r) {  // first use of chunk J's columns
-            MgOperand& b = bq[(size_t)J];
-            b.r = (int8_t*)mg[1] + bq_off;
-            b.scale = bqs + naux * J;
-            bq_off += mg_bytes(naux, rj);
-            FC_TRY(mg_convert_rows(d.b_ov + cp.j0 * nvir, nov, naux, rj, &b, flags, st));
-            nl += 2;
-        }
         if (stats) FC_CUDA(cudaEventRecord(ev[2 * x], st));
         FC_TRY(mg_gemm(bt.slice(cp.j0 * nvir, rj), bt.slice(cp.i0 * nvir, ri), MgOut{T, rj, 0, 1.0, 0},
-                       items + cp.t0[0], cp.nt[0], mg[3], flags + 1, st));
+                       items + cp.t0[0], cp.nt[0], mg[3], flags, st));
         if (stats) FC_CUDA(cudaEventRecord(ev[2 * x + 1], st));
         AmpArgs a{};
         a.g = T;
@@ -450,6 +448,7 @@ fc_status rimp2_grad_mod(const Rimp2Dev& d, cudaStream_t st, double* e_os, doubl
         a.eo = d.eps_occ;
         a.ev = d.eps_vir;
         a.same = cp.same();
+        a.bad = flags;
         a.part = part;
         a.vir = virp;
         amp_kernel<AMP_GRAD><<<dim3((unsigned)ntiles, (unsigned)cp.np), AN, AMP_SMEM, st>>>(a);
@@ -461,14 +460,28 @@ fc_status rimp2_grad_mod(const Rimp2Dev& d, cudaStream_t st, double* e_os, doubl
         amp_vir_fold_kernel<<<(unsigned)((nvir + 31) / 32), 256, 0, st>>>(vch, vc, (int)nvir, ntile * AT, de_dvir);
         FC_TRY(check_launch("residue gradient: amplitudes"));
         nl += 6;
-        MgOperand t{(int8_t*)mg[2], ts};
-        FC_TRY(mg_convert_rows(T, rj, ri, rj, &t, flags, st));
+        const MgMat tm = mg_mat(T, rj, ri, rj, tstat);
+        FC_TRY(mg_stats(tm, mpart, flags, st));
+        MgMat& bj = bm[(size_t)J];
+        if (!bj.p) {  // first use of chunk J's columns: converted under its product's guard
+            bj = nch == 1 ? B : mg_mat(d.b_ov + cp.j0 * nvir, nov, naux, rj, qstat[(size_t)J]);
+            if (nch > 1) FC_TRY(mg_stats(bj, mpart, flags, st));
+            FC_TRY(mg_convert(bj, 0, (int8_t*)mg[1] + bq_off, &tm, 0, mpart, flags, st, &bq[(size_t)J]));
+            bq_off += mg_bytes(naux, rj);
+            nl += nch > 1 ? 2 : 0;
+        } else {
+            FC_TRY(mg_guard(bj, 0, tm, 0, mpart, flags, st));
+        }
+        MgOperand t;
+        FC_TRY(mg_convert(tm, 0, (int8_t*)mg[2], &bj, 0, mpart, flags, st, &t));
         FC_TRY(adjoint(t, cp.i0, cp.j0, items + cp.t0[1], cp.nt[1]));
-        nl += 2;
+        nl += 6;
         if (!cp.same()) {
-            FC_TRY(mg_convert_cols(T, rj, rj, ri, &t, cpart, flags, st));
+            const MgMat& bi = bm[(size_t)(cp.i0 / cc)];
+            FC_TRY(mg_guard(bi, 0, tm, 1, mpart, flags, st));
+            FC_TRY(mg_convert(tm, 1, (int8_t*)mg[2], &bi, 0, mpart, flags, st, &t));
             FC_TRY(adjoint(t, cp.j0, cp.i0, items + cp.t0[2], cp.nt[2]));
-            nl += 3;
+            nl += 4;
         }
         // row I of the chunk pairs is done: Gamma's columns of chunk I are final
         if (sink && cp.j0 + cp.nj == nocc) FC_TRY(gamma_sink_block(sink, gamma, naux, nov, nvir, cp.i0, cp.ni, st));
@@ -597,11 +610,11 @@ fc_status energy_passes(const UmpSpin* spin, int nspin, std::vector<EnergyPass>&
     FC_TRY(ws_get(WS_PAIRS, hp.size() * sizeof(int2), &vpairs));
     FC_TRY(ws_get(WS_PART, (items_max * 3 + (size_t)np_max * 3) * 8, &vpart));
     FC_TRY(ws_get(WS_OUT, 256, &vout));
-    double *sc[2], *cpart;
+    double *stat[2], *mpart;
     int4* items;
     auto misc = [&](Carver& c) {
-        for (int s = 0; s < 2; ++s) sc[s] = c.take<double>(rows[s]);
-        cpart = c.take<double>(mg_colpart(rmax, naux));
+        for (int s = 0; s < nspin; ++s) stat[s] = c.take<double>(mg_stat_doubles(naux, rows[s]));
+        mpart = c.take<double>(mg_part_doubles(naux, rmax));
         items = c.take<int4>(ht.size());
     };
     Carver cm;
@@ -622,10 +635,18 @@ fc_status energy_passes(const UmpSpin* spin, int nspin, std::vector<EnergyPass>&
     FC_CUDA(cudaMemsetAsync(vout, 0, 256, st));
     Context& c = ctx();
     if (stats) FC_CUDA(cudaEventRecord(c.ev0, st));
-    MgOperand op[2] = {{(int8_t*)mg[0], sc[0]}, {(int8_t*)mg[1], sc[1]}};
-    for (int s = 0; s < nspin; ++s)
-        FC_TRY(mg_convert_cols(spin[s].b_ov, rows[s], rows[s], naux, &op[s], cpart, flags, st));
-    int nl = 3 * nspin;
+    MgMat B[2];
+    MgOperand op[2];
+    for (int s = 0; s < nspin; ++s) {
+        B[s] = mg_mat(spin[s].b_ov, rows[s], naux, rows[s], stat[s]);
+        FC_TRY(mg_stats(B[s], mpart, flags, st));
+        FC_TRY(mg_convert(B[s], 1, (int8_t*)mg[s], &B[s], 1, mpart, flags, st, &op[s]));
+    }
+    int nl = 4 * nspin;
+    if (nspin > 1) {  // the product of the two spins
+        for (int s = 0; s < 2; ++s) FC_TRY(mg_guard(B[s], 1, B[1 - s], 1, mpart, flags, st));
+        nl += 4;
+    }
     double flops = 0.0;
     for (int64_t k = 0; k < npass; ++k) {
         const EnergyPass& ps = passes[(size_t)k];
@@ -634,7 +655,7 @@ fc_status energy_passes(const UmpSpin* spin, int nspin, std::vector<EnergyPass>&
             const EnergyChunk& x = ch[(size_t)q];
             const int64_t ld = x.nj * B.nvir;
             FC_TRY(mg_gemm(op[ps.b].slice(x.j0 * B.nvir, ld), op[ps.a].slice(x.i0 * A.nvir, x.ni * A.nvir),
-                           MgOut{G, ld, 0, 1.0, 0}, items + x.t0, x.nt, mg[3], flags + 1, st));
+                           MgOut{G, ld, 0, 1.0, 0}, items + x.t0, x.nt, mg[3], flags, st));
             AmpArgs a{};
             a.g = G;
             a.ld = ld;
@@ -652,6 +673,7 @@ fc_status energy_passes(const UmpSpin* spin, int nspin, std::vector<EnergyPass>&
             a.same = ps.mode != AMP_CROSS;
             a.has_kappa = has_kappa;
             a.kappa = kappa;
+            a.bad = flags;
             a.part = part;
             const dim3 grid((unsigned)ps.ntiles, (unsigned)x.np);
             if (ps.mode == AMP_CROSS) amp_kernel<AMP_CROSS><<<grid, AN, AMP_SMEM, st>>>(a);

@@ -27,8 +27,8 @@ def _check(got, ref):
 def test_gradient_matches_oracle(fc, monkeypatch, naux, nocc, nvir, chunks):
     from ferric_b200 import rimp2
     b, eo, ev = synthetic.rimp2_inputs(naux, nocc, nvir)
-    cc = -(-nocc // chunks)
-    monkeypatch.setenv("FERRIC_CUDA_CHUNK_BYTES", str(23 * (cc * nvir) ** 2))
+    cc = -(-nocc // chunks)  # a chunk's block takes 8 bytes an element and 16 of residues
+    monkeypatch.setenv("FERRIC_CUDA_CHUNK_BYTES", str(24 * (cc * nvir) ** 2))
     st = {}
     got = rimp2.rimp2_energy_grad(b, eo, ev, stats=st)
     assert st["tile_n"] == 256 and st["main_launches"] == chunks * (chunks + 1) // 2
@@ -164,3 +164,113 @@ def test_response_2c(fc, naux, nov):
     yr = v.T @ x
     _close(y, yr)
     _close(g, -2.0 * (v.T @ b) @ yr.T)
+
+
+def _rowwise(got, a, b, c=64.0):
+    """Rows and columns of got = a b^T against 80-bit sums, each in its 2-norm: within c 2^-53 of the row (column)
+    of |a| |b|^T, where FP64 sums of these lengths lie (their own bound is K 2^-53 of it, element by element)."""
+    s = np.abs(a).max(axis=1, keepdims=True)  # (so that no square below underflows)
+    ref = a.astype(np.longdouble) @ b.T.astype(np.longdouble)
+    err = (np.abs(got - ref) / s).astype(np.float64)
+    mag = np.abs(a / s) @ np.abs(b).T
+    for ax in (0, 1):
+        e, m = np.linalg.norm(err, axis=ax), np.linalg.norm(mag, axis=ax)
+        assert (e <= c * 2.0 ** -53 * m).all(), (ax, float((e / (m + 1e-300)).max()))
+
+
+def _graded(case, m, n, k):
+    """Operands whose large elements meet small ones: opposite slopes, a triangle, rows of one slope and of the other,
+    one row apart, a row whose squares underflow."""
+    rng = np.random.default_rng(17)
+    a, b = rng.standard_normal((m, k)), rng.standard_normal((n, k))
+    q = np.arange(k)
+    if case == "slopes":
+        a *= np.exp(-q / 20.0)
+        b *= np.exp((q - k) / 20.0)
+    elif case == "triangle":  # the first rows of a factor meet the partner's smallest elements
+        a = np.where(q[None, :] <= np.arange(m)[:, None], a, 0.0)
+        b *= np.exp((q - k) * 30.0 / k)
+    elif case == "row":
+        a[3] *= np.exp(-q / 10.0)
+        b[:, :200] *= 1e-9
+    else:
+        a[3] *= 1e-170
+    return a, b
+
+
+CASES = ["slopes", "triangle", "row", "underflow"]
+
+
+@pytest.mark.parametrize("case", CASES)
+def test_graded_dressing(fc, case):
+    """B = M MO^T through a square dressing: t = MO tensor with unit orbitals, so the dressing is the product tested."""
+    from ferric_b200 import dress
+    naux, n, nl = 640, 256, 64
+    m, mo = _graded(case, naux, nl * n, naux)
+    t = np.zeros((naux, n, n))
+    t[:, :nl] = mo.T.reshape(naux, nl, n)
+    # (Q|lr) = sum C_left[mu, l] t[Q, nu, mu] C_right[nu, r]: the tensor need not be symmetric here
+    cl, cr = np.eye(n)[:, :nl], np.eye(n)
+    got = dress.mo_dress(np.ascontiguousarray(t.transpose(0, 2, 1)), m, np.ascontiguousarray(cl), cr)
+    sel = np.r_[0:7, naux - 7:naux]
+    _rowwise(got[sel], m[sel], mo)
+
+
+@pytest.mark.parametrize("case", CASES)
+def test_graded_response(fc, case):
+    from ferric_b200 import rimp2
+    naux, nov = 513, 4099
+    v, x = _graded(case, naux, nov, naux)
+    y, g = rimp2.rimp2_response_2c(np.ascontiguousarray(x.T), np.ascontiguousarray(x.T), np.ascontiguousarray(v.T))
+    sel = np.r_[0:7, naux - 7:naux]
+    _rowwise(y[sel], v[sel], x)
+
+
+def test_graded_rank_update(fc):
+    """K of orbitals whose W rows are a strong block and a weak one on other aux rows."""
+    from ferric_b200.dfjk import DfJK
+    n, naux, nocc = 257, 640, 192
+    rng = np.random.default_rng(5)
+    b = np.zeros((naux, n, n))
+    b[:320, :128, :128] = rng.standard_normal((320, 128, 128))
+    b[320:, 128:, 128:] = 1e-6 * rng.standard_normal((320, 129, 129))
+    b[320:, :128, :128] = 1e-11 * rng.standard_normal((320, 128, 128))
+    b = b + b.transpose(0, 2, 1)
+    c = np.linalg.qr(rng.standard_normal((n, nocc)))[0]
+    k = DfJK(b).k_from_occ(np.ascontiguousarray(c))
+    w = (b.reshape(-1, n) @ c).reshape(naux, n, nocc).transpose(1, 0, 2).reshape(n, -1)
+    sel = np.r_[0:3, 126:131]
+    _rowwise(k[sel], w[sel], w, c=256.0)  # W itself is rounded: 2^-53 sums of n terms
+
+
+def test_graded_spins(fc):
+    """Two spins on aux rows that hardly overlap: E_ab is a sum of graded products."""
+    from ferric_b200 import rimp2
+    naux, no, nv = 700, 12, 129
+    a, b = _graded("slopes", no * nv, no * nv, naux)
+    eo, ev = synthetic.rimp2_inputs(2, no, nv)[1:]
+    a, b = np.ascontiguousarray(a.T), np.ascontiguousarray(b.T)
+    e = rimp2.ump2_energy(a, eo, ev, b, eo, ev)
+    g = (a.T @ b).reshape(no, nv, no, nv)  # every element within 700 2^-53 sum_k |a_k b_k|, like the call's
+    d = eo[:, None, None, None] + eo[None, None, :, None] - ev[None, :, None, None] - ev[None, None, None, :]
+    ref = float((g * g / d).sum())
+    assert abs(e[2] - ref) <= 1e-12 * abs(ref)
+
+
+def test_graded_adjoint(fc):
+    """Amplitudes of two blocks of orbitals, each on its own aux rows: Gamma's rows are products of one block each."""
+    from ferric_b200 import rimp2
+    naux, no, nv = 700, 12, 129
+    b, eo, ev = synthetic.rimp2_inputs(naux, no, nv)
+    b[350:, :no * nv // 2] *= 1e-13
+    b[:350, no * nv // 2:] *= 1e-13
+    b[350:] *= 1e-9
+    _, g, go, gv = rimp2.rimp2_energy_grad(b, eo, ev)
+    gamma = orc.energy_gamma_deps(b, eo, ev)[2]
+    t2, _ = orc.t2_and_integrals(b, eo, ev)
+    t4 = t2.reshape(no, nv, no, nv)
+    tt = np.abs(2 * t4 - t4.transpose(0, 3, 2, 1)).reshape(no * nv, -1)
+    mag = 4 * np.abs(b) @ tt.T
+    e = np.abs(g - gamma)
+    for ax in (0, 1):
+        assert (np.linalg.norm(e, axis=ax) <= 700 * 2.0 ** -53 * np.linalg.norm(mag, axis=ax)).all()
