@@ -144,6 +144,16 @@ fc_status ws_get(int slot, size_t bytes, void** out) {
     return FC_OK;
 }
 
+bool ws_try(int slot, size_t bytes, void** out) {
+    Context& c = ctx();
+    if (c.pool_cap && bytes > c.ws[slot].bytes &&
+        ws_bytes() - c.ws[slot].bytes + c.handle_bytes + bytes + 256 > c.pool_cap)
+        return false;
+    if (ws_get(slot, bytes, out) == FC_OK) return true;
+    cudaGetLastError();
+    return false;
+}
+
 fc_status timing_events(int n, cudaEvent_t** out) {
     Context& c = ctx();
     while ((int)c.evs.size() < 2 * n) {

@@ -330,13 +330,16 @@ struct EpiScatterW {
     }
 };
 
-// mg (optional): the residue GEMM's flags; nsplit_mg of its partials count
-// unless one is raised.
+// mg (optional): the residue GEMM's flags; its nsplit_mg partials count unless
+// one is raised.
 __global__ void dfk_fold_kernel(const double* __restrict__ part, int nsplit, int64_t n, double* __restrict__ k,
-                                const int* __restrict__ mg, int nsplit_mg) {
+                                const int* __restrict__ mg, const double* __restrict__ part_mg, int nsplit_mg) {
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= n * n) return;
-    if (mg && !(mg[0] | mg[1])) nsplit = nsplit_mg;
+    if (mg && !(mg[0] | mg[1])) {
+        nsplit = nsplit_mg;
+        part = part_mg;
+    }
     const int64_t r = idx / n, c = idx % n;
     const int64_t lo = r < c ? r : c, hi = r < c ? c : r;
     k[idx] = fold_in_order(part + lo * n + hi, nsplit, n * n);
@@ -531,14 +534,12 @@ fc_status dfk_build_f64(fc_dfjk* h, const double* c_occ, int64_t nocc, double* k
     FC_TRY(ws_get(WS_T, n * kdim * 8, &vw));
     // K = W W^T through residues (mgemm.cuh) where the product is worth W's
     // conversion: n = 600, kdim = 144000: 2.50 -> 0.95 ms; even at n = 400, kdim = 64000.
-    const bool residues = (double)n * n * kdim >= 8e9 && n <= 65535;
-    const int nsplit_mg = residues ? mg_splits(n, n, kdim, true) : 0;
+    FC_TRY(ws_get(WS_PART, (int64_t)nsplit * n * n * 8, &vpart));
     void* vflags = nullptr;
-    FC_TRY(ws_get(WS_PART, (int64_t)std::max(nsplit, nsplit_mg) * n * n * 8, &vpart));
-    if (residues) {
-        FC_TRY(ws_get(WS_OUT, 256, &vflags));
-        FC_CUDA(cudaMemsetAsync(vflags, 0, 256, st));
-    }
+    const bool residues = (double)n * n * kdim >= 8e9 && n <= 65535 && ws_try(WS_OUT, 256, &vflags);
+    const int nsplit_mg = residues ? mg_splits(n, n, kdim, true) : 0;
+    double* part_mg = nullptr;
+    if (residues) FC_CUDA(cudaMemsetAsync(vflags, 0, 256, st));
     Context& c = ctx();
     if (stats) FC_CUDA(cudaEventRecord(c.ev0, st));
     transpose_kernel<<<(unsigned)((n * nocc + 255) / 256), 256, 0, st>>>(c_occ, n, nocc, (double*)vct);
@@ -564,8 +565,8 @@ fc_status dfk_build_f64(fc_dfjk* h, const double* c_occ, int64_t nocc, double* k
     bool room = false;
     if (residues) {
         const MgSrc w{(const double*)vw, kdim, n, false};
-        FC_TRY(mg_multiply(w, w, kdim, MgOut{(double*)vpart, n, n * n, 1.0, 0}, true, nsplit_mg, (int*)vflags, st,
-                           &room));
+        FC_TRY(mg_multiply(w, w, kdim, MgOut{nullptr, n, n * n, 1.0, 0}, true, nsplit_mg, (int*)vflags, st, &room,
+                           &part_mg));
     }
     const int* mg = room ? (const int*)vflags : nullptr;
     {  // every CTA leaves at once where the residue product stands
@@ -574,7 +575,7 @@ fc_status dfk_build_f64(fc_dfjk* h, const double* c_occ, int64_t nocc, double* k
         dgemm_tn_launch(g, st, (const double*)vw, kdim, (const double*)vw, kdim, (int)n, (int)n, kdim, kps, 1, epi, mg);
     }
     dfk_fold_kernel<<<(unsigned)((n * n + 255) / 256), 256, 0, st>>>((const double*)vpart, nsplit, n, k, mg,
-                                                                     nsplit_mg);
+                                                                     part_mg, nsplit_mg);
     FC_TRY(check_launch("DF-K kernels"));
     if (jf) {  // join J's second pass
         FC_CUDA(cudaEventRecord(c.join, c.side));

@@ -142,15 +142,11 @@ fc_status mo_dress(const double* eri3, bool host, int64_t naux, int64_t n, const
     // operands' conversion: the MO step per chunk (K = n) and the dressing
     // (K = naux).  The MO tensor then stays in its natural order (Q, l, r).  Whole
     // call at 2 naux^2 width = 5.5e9: 591 us against 517 DMMA; at 2.6e10: 1351, 1738.
+    void* vflags = nullptr;
     const bool residues = precision == FC_PREC_F64 && 2.0 * naux * (double)naux * width >= 1e10 && naux <= MG_KMAX &&
-                          n <= MG_KMAX && n >= 256;
-    int* mg_flags = nullptr;
-    if (residues) {
-        void* v;
-        FC_TRY(ws_get(WS_OUT, 256, &v));
-        mg_flags = (int*)v;
-        FC_CUDA(cudaMemsetAsync(v, 0, 256, st));
-    }
+                          n <= MG_KMAX && n >= 256 && ws_try(WS_OUT, 256, &vflags);
+    int* mg_flags = (int*)vflags;
+    if (residues) FC_CUDA(cudaMemsetAsync(vflags, 0, 256, st));
     double* clt = (double*)vct;  // C_left^T (nl x n)
     double* crt = clt + nl * n;  // C_right^T (nr x n)
     double* H = (double*)vh;

@@ -84,6 +84,7 @@ enum WsSlot {
     WS_MG_A,       // residues of one operand
     WS_MG_B,       // residues of the other operand
     WS_MG_T,       // residues of an intermediate (amplitudes)
+    WS_MG_G,       // FP64 results and partial results of residue products
     WS_MG_SCR,     // residues of the GEMM's tiles in flight
     WS_MG_MISC,    // scales, partial norms, tile lists
     WS_COUNT
@@ -115,9 +116,12 @@ fc_status pool_reserve(uint64_t bytes);  // handle allocation check
 // cudaMalloc for memory outside the slots (handles): gives the residue slots
 // back and tries again where the device is full.
 cudaError_t spare_malloc(void** p, size_t bytes);
-// Slots of at least need[k] bytes for WS_MG_A + k (0: not used), or false,
-// with nothing allocated, where they would take more than half of what the
-// pool cap or the device has left: the caller then takes its other path.
+// ws_get for scratch that a call can do without: false where it does not fit.
+bool ws_try(int slot, size_t bytes, void** out);
+// Slots of at least need[k] bytes for WS_MG_A + k (0: not used), or false where
+// they would take more than half of what the pool cap or the device has left:
+// the caller then takes its other path.  (What a refused call got so far stays
+// spare memory.)
 constexpr int WS_MG_SLOTS = WS_MG_MISC - WS_MG_A + 1;
 bool ws_get_mg(const size_t (&need)[WS_MG_SLOTS], void* (&out)[WS_MG_SLOTS]);
 cudaStream_t pick_stream(void* s);

@@ -119,13 +119,21 @@ fc_status imat_gemm(const double* A, const double* B, int64_t M, int64_t N, int6
     if (precision == FC_PREC_F64) {
         // 64 x 48 tiles where they pad at least a fifth less (M 202, N 33, K 118300:
         // 256 x 48 against 256 x 64; with two CTAs per SM 187 -> 113 us)
-        const bool skinny = 5 * rup(M, SKINNY_M) * rup(N, SKINNY_N) <= 4 * rup(M, DG_BM) * rup(N, DG_BN);
-        const int bm = skinny ? SKINNY_M : DG_BM, bn = skinny ? SKINNY_N : DG_BN;
-        const int tm = (int)((M + bm - 1) / bm), tn = (int)((N + bn - 1) / bn);
-        int nsplit = std::max(1, (2 * sms + tm * tn - 1) / (tm * tn));
-        int64_t kps = rup((K + nsplit - 1) / nsplit, DG_BK);
-        nsplit = (int)((K + kps - 1) / kps);
-        FC_TRY(ws_get(WS_PART, (size_t)nsplit * M * N * 8, &vpart));
+        bool skinny = 5 * rup(M, SKINNY_M) * rup(N, SKINNY_N) <= 4 * rup(M, DG_BM) * rup(N, DG_BN);
+        int tm, tn, nsplit;
+        int64_t kps;
+        auto plan = [&](int limit) {
+            const int bm = skinny ? SKINNY_M : DG_BM, bn = skinny ? SKINNY_N : DG_BN;
+            tm = (int)((M + bm - 1) / bm), tn = (int)((N + bn - 1) / bn);
+            nsplit = std::max(1, std::min(limit, (2 * sms + tm * tn - 1) / (tm * tn)));
+            kps = rup((K + nsplit - 1) / nsplit, DG_BK);
+            nsplit = (int)((K + kps - 1) / kps);
+            return (size_t)nsplit * M * N * 8;
+        };
+        if (!ws_try(WS_PART, plan(INT32_MAX), &vpart)) {  // fewer partials, in the tile that needs few
+            skinny = false;
+            FC_TRY(ws_get(WS_PART, plan(64), &vpart));
+        }
         dim3 g((unsigned)tn, (unsigned)tm, (unsigned)nsplit);
         EpiSplit epi{(double*)vpart, M * N, (int)N};
         if (skinny) dgemm_tn_launch<EpiSplit, SKINNY_M, SKINNY_N>(g, st, A, K, B, K, (int)M, (int)N, K, kps, 0, epi);

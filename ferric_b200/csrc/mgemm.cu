@@ -803,8 +803,8 @@ int mg_splits(int64_t M, int64_t N, int64_t K, bool upper) {
     return (int)((nks + kps - 1) / kps);
 }
 
-fc_status mg_multiply(const MgSrc& a, const MgSrc& b, int64_t K, const MgOut& out, bool upper, int splits, int* flags,
-                      cudaStream_t st, bool* room) {
+fc_status mg_multiply(const MgSrc& a, const MgSrc& b, int64_t K, MgOut out, bool upper, int splits, int* flags,
+                      cudaStream_t st, bool* room, double** part_out) {
     *room = false;
     const bool same = a.p == b.p && a.ld == b.ld && a.rows == b.rows && a.cols == b.cols;
     const int64_t rmax = std::max(a.rows, b.rows);
@@ -822,10 +822,12 @@ fc_status mg_multiply(const MgSrc& a, const MgSrc& b, int64_t K, const MgOut& ou
     const size_t osa = take(mg_stat_doubles(a.rows, K) * 8), osb = take(same ? 0 : mg_stat_doubles(b.rows, K) * 8);
     const size_t opart = take(mg_part_doubles(rmax, K) * 8), oitems = take(items * sizeof(int4));
     void* mg[WS_MG_SLOTS];
-    if (!ws_get_mg({mg_bytes(a.rows, K), same ? 0 : mg_bytes(b.rows, K), 0, mg_scratch_bytes(), off}, mg))
+    const size_t results = out.out ? 0 : (splits > 1 ? splits * out.split_stride : out.ld * b.rows) * 8;
+    if (!ws_get_mg({mg_bytes(a.rows, K), same ? 0 : mg_bytes(b.rows, K), 0, results, mg_scratch_bytes(), off}, mg))
         return FC_OK;
     *room = true;
-    char* m = (char*)mg[4];
+    if (!out.out) *part_out = out.out = (double*)mg[3];
+    char* m = (char*)mg[5];
     double* part = (double*)(m + opart);
     int4* list = (int4*)(m + oitems);
     mg_tiles_kernel<<<1, 1024, 0, st>>>(g, list);
@@ -839,7 +841,7 @@ fc_status mg_multiply(const MgSrc& a, const MgSrc& b, int64_t K, const MgOut& ou
     FC_TRY(mg_convert(A, a.cols, (int8_t*)mg[0], &B, b.cols, part, flags, st, &oa));
     if (same) ob = oa;
     else FC_TRY(mg_convert(B, b.cols, (int8_t*)mg[1], &A, a.cols, part, flags, st, &ob));
-    return mg_gemm(oa, ob, out, list, items, mg[3], flags, st);
+    return mg_gemm(oa, ob, out, list, items, mg[4], flags, st);
 }
 
 }  // namespace fc

@@ -109,8 +109,10 @@ fc_status mg_gemm(const MgOperand& A, const MgOperand& B, const MgOut& out, cons
 
 // A whole product of two FP64 matrices in device memory, converted here:
 // operand rows are the rows of p, or its columns (cols).  Uses the residue
-// slots but WS_MG_T and WS_MG_G; `splits` ranges of at most MG_KMAX each.
-// *room = false, and nothing is launched, where the residues do not fit.
+// slots but WS_MG_T; `splits` ranges of at most MG_KMAX each.  out.out ==
+// nullptr: the result, or the splits' partials, go to WS_MG_G (*part), where
+// they stay until the next residue call.
+// *room = false, and nothing is launched, where all that does not fit.
 // flags (two device ints, zeroed by the caller): rows out of range or the
 // guard, a wait's timeout; the product is valid where both stay 0.
 struct MgSrc {
@@ -118,8 +120,8 @@ struct MgSrc {
     int64_t ld, rows;
     bool cols;
 };
-fc_status mg_multiply(const MgSrc& a, const MgSrc& b, int64_t K, const MgOut& out, bool upper, int splits, int* flags,
-                      cudaStream_t st, bool* room);
+fc_status mg_multiply(const MgSrc& a, const MgSrc& b, int64_t K, MgOut out, bool upper, int splits, int* flags,
+                      cudaStream_t st, bool* room, double** part = nullptr);
 // out[n * ld + m] = alpha * sum of the splits' partials, in order.
 fc_status mg_fold(const double* part, int splits, int64_t M, int64_t N, double alpha, double* out, int64_t ld,
                   cudaStream_t st);

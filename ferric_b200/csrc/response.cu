@@ -62,18 +62,13 @@ fc_status response_2c(const double* x_ov, const double* b_ov, const double* vis,
     // residues where the products outweigh the operands' conversion: a gradient
     // chain with them at 2 naux^2 nov = 1.8e9 (naux 532, nov 3225) 1772 us, without
     // 1853; at 5.5e9 3161 and 3641; at 9e8 1361 and 1318.
-    const bool residues = 2.0 * naux * (double)naux * nov >= 1.5e9 && naux <= MG_KMAX;
-    const int splits = residues && nov <= INT32_MAX / 2 ? mg_splits(naux, naux, nov, false) : 1;
-    int* flags = nullptr;
+    void* vflags = nullptr;
+    const bool residues =
+        2.0 * naux * (double)naux * nov >= 1.5e9 && naux <= MG_KMAX && ws_try(WS_OUT, 256, &vflags);
+    const int splits = residues ? mg_splits(naux, naux, nov, false) : 1;
+    int* flags = (int*)vflags;
     double* gpart = nullptr;
-    if (residues) {
-        void *vf, *vp;
-        FC_TRY(ws_get(WS_OUT, 256, &vf));
-        FC_TRY(ws_get(WS_T, splits > 1 ? (size_t)splits * naux * naux * 8 : 0, &vp));
-        flags = (int*)vf;
-        gpart = (double*)vp;
-        FC_CUDA(cudaMemsetAsync(vf, 0, 256, st));
-    }
+    if (residues) FC_CUDA(cudaMemsetAsync(vflags, 0, 256, st));
     if (stats) FC_CUDA(cudaEventRecord(c.ev0, st));
     // y[P, ia] = sum_Q V[Q, P] x[Q, ia];  C[P, ia] = sum_Q V[Q, P] b[Q, ia]
     // gamma_2c[P, Q] = -w sum_ia C[P, ia] y[Q, ia]
@@ -89,9 +84,9 @@ fc_status response_2c(const double* x_ov, const double* b_ov, const double* vis,
                                &room));
         if (room)
             FC_TRY(mg_multiply({y_ov, nov, naux, false}, {cfit, nov, naux, false}, nov,
-                               splits > 1 ? MgOut{gpart, naux, naux * naux, 1.0, 0}
+                               splits > 1 ? MgOut{nullptr, naux, naux * naux, 1.0, 0}
                                           : MgOut{gamma_2c, naux, 0, -w, 0},
-                               false, splits, flags, st, &room));
+                               false, splits, flags, st, &room, &gpart));
         if (room && splits > 1) FC_TRY(mg_fold(gpart, splits, naux, naux, -w, gamma_2c, naux, st));
         mg = room ? flags : nullptr;
     }

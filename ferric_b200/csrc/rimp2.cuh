@@ -121,12 +121,13 @@ struct DensF64 {
     double* ts;       // [nocc nvir][ld]
     double* as;       // [nocc nvir][ld]
     double* part_oo;  // [splits][nocc x nocc]
-    double* part_vv;  // [gvv][kvv][nvir x nvir]
+    double* part_vv;  // [gvv][kvv][nvir x nvir] (nullptr: no room, acc_vv takes each product)
     double* acc_vv;   // [nvir x nvir] running P_vv (upper tiles)
     double* acc_oo;   // [nocc x nocc] running P_oo
     int splits, gvv, kvv;  // P_oo's ranges of K; P_vv's orbitals per launch, ranges of K
 };
 int64_t dens_chunk_f64(int64_t nocc, int64_t nvir, int64_t cc, int64_t budget);
+// (its partial results are spare memory: after every ws_get of the call)
 fc_status dens_f64_alloc(int64_t nocc, int64_t nvir, int64_t cc, cudaStream_t st, DensF64* o);
 // Block rows r0 .. r0 + nr nvir of the Tt slab (pitch nk nvir): t into the t slab.
 fc_status dens_f64_block(const DensF64& o, int64_t r0, int64_t nr, int64_t nk, cudaStream_t st, int64_t* nl);

@@ -285,6 +285,8 @@ fc_status dens_attrs() {
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, xg::Cfg<128, true>::SMEM));
     FC_CUDA(cudaFuncSetAttribute(dgemm_upper_kernel<EpiBatchStore, DG_BM, DG_BN>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, DG_SMEM));
+    FC_CUDA(cudaFuncSetAttribute(dgemm_upper_kernel<EpiStore, DG_BM, DG_BN>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, DG_SMEM));
     FC_CUDA(cudaFuncSetAttribute(dgemm_upper_kernel<EpiBatchStore, OO_M, OO_N>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, dg_smem(OO_M, OO_N)));
     FC_CUDA(cudaFuncSetAttribute(dgemm_tn_kernel<EpiSplit, false, false, OO_M, OO_N>,
@@ -431,7 +433,7 @@ fc_status dens_f64_alloc(int64_t nocc, int64_t nvir, int64_t cc, cudaStream_t st
     FC_TRY(dens_attrs());
     o->nocc = nocc;
     o->nvir = nvir;
-    o->splits = std::max(1, 2 * ctx().sm_count);  // two CTAs of the P_oo tile per SM
+    o->splits = std::max(1, ctx().sm_count);
     o->gvv = (int)std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(nocc, 65535),
                                                          (int64_t(256) << 20) / (8 * nvir * nvir)));
     // eight CTAs per SM, so that the last ones leave little of the chip idle
@@ -439,17 +441,25 @@ fc_status dens_f64_alloc(int64_t nocc, int64_t nvir, int64_t cc, cudaStream_t st
     o->kvv = (int)std::max<int64_t>(
         1, std::min<int64_t>({16, (8 * ctx().sm_count + ctas - 1) / ctas, 65535 / o->gvv, cc * nvir / (16 * DG_BK)}));
     const size_t slab = (size_t)nocc * nvir * cc * nvir;
-    void *vs, *vp, *vv;
+    const size_t nn = (size_t)nocc * nocc;
+    void *vs, *vp;
     FC_TRY(ws_get(WS_DSLAB, 2 * slab * 8, &vs));
-    FC_TRY(ws_get(WS_DSTORE, (size_t)o->gvv * o->kvv * nvir * nvir * 8, &vv));
-    o->part_vv = (double*)vv;
+    FC_TRY(ws_get(WS_DPART, ((size_t)o->splits * nn + nn + (size_t)nvir * nvir) * 8, &vp));
     o->ts = (double*)vs;
     o->as = o->ts + slab;
-    const size_t nn = (size_t)nocc * nocc;
-    FC_TRY(ws_get(WS_DPART, ((size_t)o->splits * nn + nn + (size_t)nvir * nvir) * 8, &vp));
     o->part_oo = (double*)vp;
     o->acc_oo = o->part_oo + (size_t)o->splits * nn;
     o->acc_vv = o->acc_oo + nn;
+    // spare memory for P_vv's products and twice as many ranges of K for P_oo
+    // (two CTAs of its tile per SM)
+    const size_t vv = (size_t)o->gvv * o->kvv * nvir * nvir * 8, oo = 2 * (size_t)o->splits * nn * 8;
+    void* spare[WS_MG_SLOTS];
+    o->part_vv = nullptr;
+    if (ws_get_mg({0, 0, 0, vv + oo, 0, 0}, spare)) {
+        o->part_vv = (double*)spare[WS_MG_G - WS_MG_A];
+        o->part_oo = o->part_vv + vv / 8;
+        o->splits *= 2;
+    }
     FC_CUDA(cudaMemsetAsync(o->acc_oo, 0, (nn + (size_t)nvir * nvir) * 8, st));
     return FC_OK;
 }
@@ -466,7 +476,15 @@ fc_status dens_f64_slab(const DensF64& o, int64_t nk, cudaStream_t st, int64_t* 
     // launch, folded in order of i (a launch per i left 6 CTAs on the chip at
     // nvir 169: 33 x 0.5 ms; 0.97 ms in one launch of 132 CTAs, 0.39 in small tiles
     // and four ranges of K)
-    for (int64_t i = 0; i < nocc; i += o.gvv) {
+    if (!o.part_vv) {  // no room for products side by side: each is added to the sum
+        const dim3 g((unsigned)dgemm_upper_tiles<DG_BM, DG_BN>(nvir));
+        for (int64_t i = 0; i < nocc; ++i)
+            dgemm_upper_kernel<EpiStore, DG_BM, DG_BN><<<g, 256, DG_SMEM, st>>>(
+                o.as + i * nvir * ld, o.ts + i * nvir * ld, ld, 0, (int)nvir, ld, 1, ld,
+                EpiStore{o.acc_vv, nvir, 1.0, 1});
+        *nl += nocc;
+    }
+    for (int64_t i = 0; o.part_vv && i < nocc; i += o.gvv) {
         const int nz = (int)std::min<int64_t>(o.gvv, nocc - i);
         const int64_t off = i * nvir * ld;
         if (vv_small(nvir))
@@ -476,7 +494,7 @@ fc_status dens_f64_slab(const DensF64& o, int64_t nk, cudaStream_t st, int64_t* 
         vv_fold_f64_kernel<<<(unsigned)((nvir * nvir + 255) / 256), 256, 0, st>>>(o.part_vv, nz * o.kvv, nvir, o.acc_vv);
         *nl += 2;
     }
-    FC_TRY(check_launch("vv_fold_f64_kernel"));
+    FC_TRY(check_launch("P_vv products"));
     // P_oo: rows i are nvir ld contiguous doubles in both slabs
     const int64_t K = nvir * ld;
     const int64_t kps = ((K + o.splits - 1) / o.splits + DG_BK - 1) / DG_BK * DG_BK;

@@ -356,46 +356,45 @@ fc_status rimp2_grad_mod(const Rimp2Dev& d, cudaStream_t st, double* e_os, doubl
     for (int64_t J = 0; J < nch; ++J) bq_bytes += mg_bytes(naux, std::min(cc, nocc - J * cc) * nvir);
     const int64_t nvch = (np_max + VP - 1) / VP;
     const size_t np_items = (size_t)np_max * ntiles;
-    double *bstat, *tstat, *mpart;
+    double *bstat, *tstat, *mpart, *part, *acc;
     std::vector<double*> qstat((size_t)nch, nullptr);  // sums of b_ov's column chunks
+    int2* pairs;
     int4* items;
+    const size_t out_bytes = (size_t)(nocc + 2) * 8 + 64;
     auto misc = [&](Carver& c) {
+        pairs = c.take<int2>(hp.size());
+        part = c.take<double>(np_items * (3 + 2 * AT) + (size_t)np_max * 3 + (size_t)nvch * ntile * AT);
+        acc = c.take<double>(out_bytes / 8);
         bstat = c.take<double>(mg_stat_doubles(naux, nov));
         for (int64_t J = 0; nch > 1 && J < nch; ++J) qstat[(size_t)J] = c.take<double>(mg_stat_doubles(naux, cv));
         tstat = c.take<double>(mg_stat_doubles(cv, cv));
         mpart = c.take<double>(std::max(mg_part_doubles(naux, nov), mg_part_doubles(cv, cv)));
         items = c.take<int4>(ht.size());
     };
-    void *vT, *vpairs, *vpart, *vout;
+    // All scratch is spare memory but the densities' slabs, which the DMMA form
+    // takes too (of the same size: it has one chunk where this form has one).
     DensF64 dx{};
-    if (dens) {
-        FC_TRY(dens_f64_alloc(nocc, nvir, nocc, st, &dx));
-        vT = dx.ts;
-    } else {
-        FC_TRY(ws_get(WS_T, (size_t)cv * cv * 8, &vT));
-    }
-    FC_TRY(ws_get(WS_PAIRS, hp.size() * sizeof(int2), &vpairs));
-    FC_TRY(ws_get(WS_PART, (np_items * (3 + 2 * AT) + (size_t)np_max * 3 + (size_t)nvch * ntile * AT) * 8, &vpart));
-    FC_TRY(ws_get(WS_OUT, (size_t)(nocc + 2) * 8 + 64, &vout));
+    if (dens) FC_TRY(dens_f64_alloc(nocc, nvir, nocc, st, &dx));
     Carver cm;
     misc(cm);
     void* mg[WS_MG_SLOTS];
-    if (!ws_get_mg({mg_bytes(nov, naux), bq_bytes, mg_bytes(cv, cv), mg_scratch_bytes(), cm.off}, mg)) return FC_OK;
-    cm = Carver{(char*)mg[4], 0};
+    if (!ws_get_mg({mg_bytes(nov, naux), bq_bytes, mg_bytes(cv, cv), dens ? 0 : (size_t)cv * cv * 8,
+                    mg_scratch_bytes(), cm.off},
+                   mg))
+        return FC_OK;
+    cm = Carver{(char*)mg[5], 0};
     misc(cm);
 
-    double* T = (double*)vT;
-    double* part = (double*)vpart;
+    double* T = dens ? dx.ts : (double*)mg[3];
     double* virp = part + 3 * np_items;
     double* psum = virp + np_items * 2 * AT;
     double* vch = psum + 3 * np_max;
-    double* acc = (double*)vout;       // E_os, E_ss
-    double* acc_occ = acc + 2;         // [nocc]
+    double* acc_occ = acc + 2;            // [nocc], behind E_os and E_ss
     int* flags = (int*)(acc_occ + nocc);  // out-of-range rows, wait timeout
-    const int2* dpairs = (const int2*)vpairs;
-    FC_CUDA(cudaMemcpyAsync(vpairs, hp.data(), hp.size() * sizeof(int2), cudaMemcpyHostToDevice, st));
+    const int2* dpairs = pairs;
+    FC_CUDA(cudaMemcpyAsync(pairs, hp.data(), hp.size() * sizeof(int2), cudaMemcpyHostToDevice, st));
     FC_CUDA(cudaMemcpyAsync(items, ht.data(), ht.size() * sizeof(int4), cudaMemcpyHostToDevice, st));
-    FC_CUDA(cudaMemsetAsync(vout, 0, (size_t)(nocc + 2) * 8 + 64, st));
+    FC_CUDA(cudaMemsetAsync(acc, 0, out_bytes, st));
     FC_CUDA(cudaMemsetAsync(de_dvir, 0, nvir * 8, st));
 
     Context& c = ctx();
@@ -421,7 +420,7 @@ fc_status rimp2_grad_mod(const Rimp2Dev& d, cudaStream_t st, double* e_os, doubl
         MgOperand& b = bq[(size_t)(k0 / cc)];
         if (stats) FC_CUDA(cudaEventRecord(ev2[2 * nadj], st));
         char& s = seen[(size_t)(r0 / cc)];
-        FC_TRY(mg_gemm(t, b, MgOut{gamma + r0 * nvir, nov, 0, 4.0, s}, its, nits, mg[3], flags, st));
+        FC_TRY(mg_gemm(t, b, MgOut{gamma + r0 * nvir, nov, 0, 4.0, s}, its, nits, mg[4], flags, st));
         s = 1;
         if (stats) FC_CUDA(cudaEventRecord(ev2[2 * nadj + 1], st));
         ++nadj;
@@ -434,7 +433,7 @@ fc_status rimp2_grad_mod(const Rimp2Dev& d, cudaStream_t st, double* e_os, doubl
         const int64_t J = cp.j0 / cc, ri = cp.ni * nvir, rj = cp.nj * nvir;
         if (stats) FC_CUDA(cudaEventRecord(ev[2 * x], st));
         FC_TRY(mg_gemm(bt.slice(cp.j0 * nvir, rj), bt.slice(cp.i0 * nvir, ri), MgOut{T, rj, 0, 1.0, 0},
-                       items + cp.t0[0], cp.nt[0], mg[3], flags, st));
+                       items + cp.t0[0], cp.nt[0], mg[4], flags, st));
         if (stats) FC_CUDA(cudaEventRecord(ev[2 * x + 1], st));
         AmpArgs a{};
         a.g = T;
@@ -605,14 +604,14 @@ fc_status energy_passes(const UmpSpin* spin, int nspin, std::vector<EnergyPass>&
         rmax = std::max(rmax, rows[s]);
     }
     const int64_t npass = (int64_t)passes.size();
-    void *vG, *vpairs, *vpart, *vout;
-    FC_TRY(ws_get(WS_T, g_max * 8, &vG));
-    FC_TRY(ws_get(WS_PAIRS, hp.size() * sizeof(int2), &vpairs));
-    FC_TRY(ws_get(WS_PART, (items_max * 3 + (size_t)np_max * 3) * 8, &vpart));
-    FC_TRY(ws_get(WS_OUT, 256, &vout));
-    double *stat[2], *mpart;
+    // all scratch is spare memory: the DMMA form needs next to none
+    double *stat[2], *mpart, *part, *acc;
+    int2* pairs;
     int4* items;
     auto misc = [&](Carver& c) {
+        pairs = c.take<int2>(hp.size());
+        part = c.take<double>(items_max * 3 + (size_t)np_max * 3);
+        acc = c.take<double>(32);
         for (int s = 0; s < nspin; ++s) stat[s] = c.take<double>(mg_stat_doubles(naux, rows[s]));
         mpart = c.take<double>(mg_part_doubles(naux, rmax));
         items = c.take<int4>(ht.size());
@@ -620,19 +619,18 @@ fc_status energy_passes(const UmpSpin* spin, int nspin, std::vector<EnergyPass>&
     Carver cm;
     misc(cm);
     void* mg[WS_MG_SLOTS];
-    if (!ws_get_mg({mg_bytes(rows[0], naux), nspin > 1 ? mg_bytes(rows[1], naux) : 0, 0, mg_scratch_bytes(), cm.off},
+    if (!ws_get_mg({mg_bytes(rows[0], naux), nspin > 1 ? mg_bytes(rows[1], naux) : 0, 0, g_max * 8,
+                    mg_scratch_bytes(), cm.off},
                    mg))
         return FC_OK;
-    cm = Carver{(char*)mg[4], 0};
+    cm = Carver{(char*)mg[5], 0};
     misc(cm);
-    double* G = (double*)vG;
-    double* part = (double*)vpart;
+    double* G = (double*)mg[3];
     double* psum = part + 3 * items_max;
-    double* acc = (double*)vout;
     int* flags = (int*)(acc + 2 * npass);
-    FC_CUDA(cudaMemcpyAsync(vpairs, hp.data(), hp.size() * sizeof(int2), cudaMemcpyHostToDevice, st));
+    FC_CUDA(cudaMemcpyAsync(pairs, hp.data(), hp.size() * sizeof(int2), cudaMemcpyHostToDevice, st));
     FC_CUDA(cudaMemcpyAsync(items, ht.data(), ht.size() * sizeof(int4), cudaMemcpyHostToDevice, st));
-    FC_CUDA(cudaMemsetAsync(vout, 0, 256, st));
+    FC_CUDA(cudaMemsetAsync(acc, 0, 256, st));
     Context& c = ctx();
     if (stats) FC_CUDA(cudaEventRecord(c.ev0, st));
     MgMat B[2];
@@ -655,12 +653,12 @@ fc_status energy_passes(const UmpSpin* spin, int nspin, std::vector<EnergyPass>&
             const EnergyChunk& x = ch[(size_t)q];
             const int64_t ld = x.nj * B.nvir;
             FC_TRY(mg_gemm(op[ps.b].slice(x.j0 * B.nvir, ld), op[ps.a].slice(x.i0 * A.nvir, x.ni * A.nvir),
-                           MgOut{G, ld, 0, 1.0, 0}, items + x.t0, x.nt, mg[3], flags, st));
+                           MgOut{G, ld, 0, 1.0, 0}, items + x.t0, x.nt, mg[4], flags, st));
             AmpArgs a{};
             a.g = G;
             a.ld = ld;
-            a.pairs = (const int2*)vpairs + x.p0;
-            a.tiles = (const int2*)vpairs + ps.tiles0;
+            a.pairs = pairs + x.p0;
+            a.tiles = pairs + ps.tiles0;
             a.ntiles = ps.ntiles;
             a.i0 = (int)x.i0;
             a.j0 = (int)x.j0;
