@@ -70,7 +70,8 @@ int64_t chunk_budget() {
     }
     Context& c = ctx();
     if (c.pool_cap) {
-        int64_t left = (int64_t)c.pool_cap - (int64_t)(ws_bytes() + c.handle_bytes);
+        // (a plan does not depend on which call filled the spare slots before)
+        int64_t left = (int64_t)c.pool_cap - (int64_t)(ws_bytes() - ws_spare_bytes() + c.handle_bytes);
         if (left / 2 < b) b = left / 2 > 0 ? left / 2 : 1;
     }
     return b;

@@ -3,6 +3,7 @@
 // install/decide/status; ferric-core/src/gpu/pool.rs:1-30: the pool ledger).
 #include "fc_internal.cuh"
 
+#include <algorithm>
 #include <cstring>
 
 namespace fc {
@@ -52,6 +53,12 @@ uint64_t ws_bytes() {
     return t;
 }
 
+uint64_t ws_spare_bytes() {
+    uint64_t t = 0;
+    for (int s = WS_MG_A; s <= WS_MG_MISC; ++s) t += ctx().ws[s].bytes;
+    return t;
+}
+
 // Give back the residue slots (false if they held nothing).
 static bool drop_mg() {
     Context& c = ctx();
@@ -85,23 +92,28 @@ cudaError_t spare_malloc(void** p, size_t bytes) {
     return e;
 }
 
-bool ws_get_mg(const size_t (&need)[WS_MG_SLOTS], void* (&out)[WS_MG_SLOTS]) {
+bool ws_get_mg(const size_t (&need)[WS_MG_SLOTS], void* (&out)[WS_MG_SLOTS], bool keep) {
     Context& c = ctx();
-    uint64_t extra = 0;
+    uint64_t total = 0, held = 0, extra = 0;  // what the call needs, what the slots then hold, what they grow by
     for (int k = 0; k < WS_MG_SLOTS; ++k) {
-        const Workspace& w = c.ws[WS_MG_A + k];
-        if (need[k] > w.bytes) extra += need[k] + 256 - w.bytes;
+        const size_t have = c.ws[WS_MG_A + k].bytes, want = need[k] ? need[k] + 256 : 0;
+        total += want;
+        held += std::max(have, want);
+        extra += need[k] > have ? want - have : 0;
     }
     if (extra) {
-        if (c.pool_cap) {
-            const uint64_t held = ws_bytes() + c.handle_bytes;
-            if (held >= c.pool_cap || extra > (c.pool_cap - held) / 2) return false;
-        }
-        size_t avail = 0, total = 0;
-        if (cudaMemGetInfo(&avail, &total) != cudaSuccess || extra > avail / 2) {
+        const uint64_t spare = ws_spare_bytes();
+        size_t avail = 0, all = 0;
+        if (cudaMemGetInfo(&avail, &all) != cudaSuccess) {
             cudaGetLastError();
             return false;
         }
+        uint64_t limit = (avail + spare) / 2;
+        if (c.pool_cap) {
+            const uint64_t others = ws_bytes() - spare + c.handle_bytes;
+            limit = std::min(limit, others < c.pool_cap ? (c.pool_cap - others) / 2 : 0);
+        }
+        if (total > limit || (held > limit && (keep || !drop_mg()))) return false;
     }
     for (int k = 0; k < WS_MG_SLOTS; ++k) {
         out[k] = nullptr;

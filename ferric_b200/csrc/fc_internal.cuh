@@ -109,6 +109,7 @@ struct Context {
 Context& ctx();
 fc_status require_init();
 uint64_t ws_bytes();
+uint64_t ws_spare_bytes();  // of these, what a later ws_get gets back on demand (WS_MG_*)
 // Workspace slot `slot` with at least `bytes` (16-byte rounded); refuses with
 // FC_ERR_POOL_FULL before allocating when the cap would be exceeded.
 fc_status ws_get(int slot, size_t bytes, void** out);
@@ -119,11 +120,13 @@ cudaError_t spare_malloc(void** p, size_t bytes);
 // ws_get for scratch that a call can do without: false where it does not fit.
 bool ws_try(int slot, size_t bytes, void** out);
 // Slots of at least need[k] bytes for WS_MG_A + k (0: not used), or false where
-// they would take more than half of what the pool cap or the device has left:
+// they would take more than half of what the pool cap or the device has left
+// without the residue slots (which are given back first where other calls'
+// sizes fill that half; not with `keep`, in a call that uses some already):
 // the caller then takes its other path.  (What a refused call got so far stays
 // spare memory.)
 constexpr int WS_MG_SLOTS = WS_MG_MISC - WS_MG_A + 1;
-bool ws_get_mg(const size_t (&need)[WS_MG_SLOTS], void* (&out)[WS_MG_SLOTS]);
+bool ws_get_mg(const size_t (&need)[WS_MG_SLOTS], void* (&out)[WS_MG_SLOTS], bool keep = false);
 cudaStream_t pick_stream(void* s);
 // At least 2*n timing events (created on first use, kept by the context).
 fc_status timing_events(int n, cudaEvent_t** out);

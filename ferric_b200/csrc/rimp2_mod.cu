@@ -380,7 +380,7 @@ fc_status rimp2_grad_mod(const Rimp2Dev& d, cudaStream_t st, double* e_os, doubl
     void* mg[WS_MG_SLOTS];
     if (!ws_get_mg({mg_bytes(nov, naux), bq_bytes, mg_bytes(cv, cv), dens ? 0 : (size_t)cv * cv * 8,
                     mg_scratch_bytes(), cm.off},
-                   mg))
+                   mg, dens != nullptr))
         return FC_OK;
     cm = Carver{(char*)mg[5], 0};
     misc(cm);

@@ -118,3 +118,22 @@ def test_products_under_cap(fc):
     ref = dress.mo_dress(bb, m, cl, cr)
     with _cap(90919168):
         _close(dress.mo_dress(bb, m, cl, cr), ref)
+
+def test_spare_memory_leaves_later_plans_alone(fc):
+    """What an FP64 energy keeps for its next call is given back on demand: it takes no chunks from a later gradient."""
+    import ferric_b200._lib as L
+    from ferric_b200 import rimp2
+    ins, small = _dev(*synthetic.rimp2_inputs(640, 24, 129)), _dev(*synthetic.rimp2_inputs(1200, 10, 95))
+
+    def launches():
+        st = {}
+        rimp2.rimp2_energy_grad(*ins, precision="mixed", stats=st)
+        return st["main_launches"]
+
+    with _cap(1 << 40):
+        launches()  # its workspace is there
+        # half of 300 MB holds the amplitudes of all 24 orbitals (11 (24 144)^2 bytes), and what the energy takes
+        L.init(0, L.lib.fc_pool_used() + (300 << 20))
+        before, st = launches(), {}
+        rimp2.rimp2_energy(*small, stats=st)
+        assert st["tile_n"] == 256 and launches() == before == 1
