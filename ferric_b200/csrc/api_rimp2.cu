@@ -416,7 +416,10 @@ static fc_status grad_host_impl(const double* b_ov, int64_t naux, int64_t nocc, 
                                        stats, sink.stream ? &sink : nullptr, dens ? &dn : nullptr);
     // the caller may reuse b_ov once this returns, also after an error
     if (us) FC_CUDA(cudaStreamSynchronize(us));
-    if (gs != FC_OK) return gs;
+    if (gs != FC_OK) {  // ... and gamma
+        if (sink.stream) FC_CUDA(cudaStreamSynchronize(sink.stream));
+        return gs;
+    }
     if (!sink.stream) FC_CUDA(cudaMemcpyAsync(gamma, dg, nel * 8, cudaMemcpyDeviceToHost, st));
     FC_CUDA(cudaMemcpyAsync(de_docc, dd, nocc * 8, cudaMemcpyDeviceToHost, st));
     FC_CUDA(cudaMemcpyAsync(de_dvir, (double*)dd + nocc, nvir * 8, cudaMemcpyDeviceToHost, st));
