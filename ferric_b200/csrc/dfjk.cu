@@ -581,7 +581,14 @@ fc_status dfk_build_f64(fc_dfjk* h, const double* c_occ, int64_t nocc, double* k
         FC_CUDA(cudaEventRecord(c.join, c.side));
         FC_CUDA(cudaStreamWaitEvent(st, c.join, 0));
     }
-    return dfk_stats(h, nocc, room ? 10 : 4, room ? MG_BM : DG_BM, room ? MG_BN : DG_BN, st, stats);
+    FC_TRY(dfk_stats(h, nocc, room ? 4 + MG_LAUNCHES_SAME : 4, DG_BM, DG_BN, st, stats));
+    bool stands = false;
+    if (stats && room) FC_TRY(mg_outcome((const int*)vflags, "DF-K", &stands));
+    if (stands) {
+        stats->tile_m = MG_BM;
+        stats->tile_n = MG_BN;
+    }
+    return FC_OK;
 }
 
 // J's second pass on the side stream, after everything `st` holds so far.
@@ -628,7 +635,8 @@ static fc_status dfjk_build_occ(fc_dfjk* h, const double* c_occ, int64_t nocc, d
         FC_CUDA(cudaEventElapsedTime(&jms, ev[0], ev[1]));
         *stats = sk;  // kernel_ms spans the whole call (the join comes before its last event)
         stats->flops = sk.flops + 2.0 * (double)h->naux * (double)h->pair;  // + J pass 2
-        stats->launches = sk.launches + 3 + (h->l_chol ? 1 : 0);
+        // J's: d (the mixed form has its row terms from stage 1), pass 2 and its fold, the metric solve
+        stats->launches = sk.launches + (sk.launches == 1 ? 0 : (mixed ? 3 : 4) + (h->l_chol ? 1 : 0));
         stats->aux_launches = 1;
         stats->aux_ms = jms;
         stats->aux_flops = 2.0 * (double)h->naux * (double)h->pair;

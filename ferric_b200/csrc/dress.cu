@@ -156,6 +156,7 @@ fc_status mo_dress(const double* eri3, bool host, int64_t naux, int64_t n, const
     dress_transpose_kernel<<<(unsigned)((n * nr + 255) / 256), 256, 0, st>>>(c_right, n, nr, crt);
     FC_TRY(check_launch("dress_transpose_kernel"));
     int launches = 2;
+    bool room = residues;  // for every residue product
     for (int64_t q0 = 0; q0 < naux; q0 += qc) {
         const int64_t qn = std::min(qc, naux - q0);
         const double* t3 = eri3 + q0 * n * n;
@@ -177,13 +178,14 @@ fc_status mo_dress(const double* eri3, bool host, int64_t naux, int64_t n, const
         }
         if (residues) {  // (Q|lr) = sum_nu H[(q, l)][nu] C_right[nu, r]
             const MgOut o{mot + q0 * width, nr, 0, 1.0, 0};
-            bool room = false;
-            FC_TRY(mg_multiply({c_right, nr, nr, true}, {H, n, qn * nl, false}, n, o, false, 1, mg_flags, st, &room));
+            bool fits = false;
+            FC_TRY(mg_multiply({c_right, nr, nr, true}, {H, n, qn * nl, false}, n, o, false, 1, mg_flags, st, &fits));
             const int M = (int)(qn * nl);
             dim3 g((unsigned)((nr + DG_BN - 1) / DG_BN), (unsigned)((M + DG_BM - 1) / DG_BM), 1);
             EpiStore epi{o.out, nr, 1.0, 0};
-            dgemm_tn_launch(g, st, H, n, crt, n, M, (int)nr, n, n, 0, epi, room ? mg_flags : nullptr);
-            launches += 4;
+            dgemm_tn_launch(g, st, H, n, crt, n, M, (int)nr, n, n, 0, epi, fits ? mg_flags : nullptr);
+            launches += fits ? MG_LAUNCHES : 0;
+            room &= fits;
         } else {  // the same, stored as MOt[l*nr + r][Q]
             const int M = (int)(qn * nl);
             dim3 g((unsigned)((nr + DG_BN - 1) / DG_BN), (unsigned)((M + DG_BM - 1) / DG_BM), 1);
@@ -200,15 +202,16 @@ fc_status mo_dress(const double* eri3, bool host, int64_t naux, int64_t n, const
     }
     if (residues) {
         // B[P][w] = sum_Q M[P][Q] MO[Q][w]
-        bool room = false;
+        bool fits = false;
         FC_TRY(mg_multiply({mot, width, width, true}, {m, naux, naux, false}, naux, MgOut{b, width, 0, 1.0, 0}, false, 1,
-                           mg_flags, st, &room));
+                           mg_flags, st, &fits));
         dim3 g((unsigned)((width + DG_BN - 1) / DG_BN), (unsigned)((naux + DG_BM - 1) / DG_BM), 1);
         EpiStore epi{b, width, 1.0, 0};
         dgemm_tn_kernel<EpiStore, false, true><<<g, 256, DG_SMEM, st>>>(
-            m, naux, mot, width, (int)naux, (int)width, naux, naux, 0, epi, room ? mg_flags : nullptr);
+            m, naux, mot, width, (int)naux, (int)width, naux, naux, 0, epi, fits ? mg_flags : nullptr);
         FC_TRY(check_launch("dressing GEMM (FP64, residues)"));
-        launches += 8;
+        launches += fits ? 1 + MG_LAUNCHES : 1;
+        room &= fits;
     } else if (precision == FC_PREC_F64) {
         // B[P][w] = sum_Q M[P][Q] MOt[w][Q]
         dim3 g((unsigned)((width + DG_BN - 1) / DG_BN), (unsigned)((naux + DG_BM - 1) / DG_BM), 1);
@@ -264,13 +267,15 @@ fc_status mo_dress(const double* eri3, bool host, int64_t naux, int64_t n, const
         float ms = 0.f, m4 = 0.f;
         FC_CUDA(cudaEventElapsedTime(&ms, cx.ev0, cx.ev1));
         FC_CUDA(cudaEventElapsedTime(&m4, ev[0], ev[1]));
+        bool stands = false;
+        if (room) FC_TRY(mg_outcome(mg_flags, "MO dressing", &stands));
         stats->kernel_ms = ms;
         stats->flops = 2.0 * naux * (double)n * n * nl + 2.0 * naux * (double)nl * n * nr +
                        2.0 * (double)naux * naux * width;
         stats->precision = precision == FC_PREC_F64 ? FC_PREC_F64 : FC_PREC_MIXED;
         stats->launches += launches;
         stats->tile_m = 128;
-        stats->tile_n = residues ? MG_BN : precision == FC_PREC_F64 ? DG_BN : 128;
+        stats->tile_n = stands ? MG_BN : precision == FC_PREC_F64 ? DG_BN : 128;
         stats->k_panel = precision == FC_PREC_F64 ? 0 : xg::KP * xg::KT;
         stats->main_launches = 1;
         stats->main_ms = m4;

@@ -128,6 +128,16 @@ bool ws_try(int slot, size_t bytes, void** out);
 constexpr int WS_MG_SLOTS = WS_MG_MISC - WS_MG_A + 1;
 bool ws_get_mg(const size_t (&need)[WS_MG_SLOTS], void* (&out)[WS_MG_SLOTS], bool keep = false);
 cudaStream_t pick_stream(void* s);
+// Failure-path test hook of the pair kernel and the residue GEMM.
+// FERRIC_CUDA_WAIT_MS bounds the MMA warp's waits for operand stages (default
+// 4 s); with FERRIC_CUDA_TEST_DROP_LOAD=1 CTA 0's producer issues no load for
+// its first stage, so that bounded wait runs out (nothing in flight,
+// FC_ERR_TIMEOUT) while every other wait keeps its 4 s limit.
+struct WaitHooks {
+    uint64_t wait_ns;
+    int drop_load;
+};
+WaitHooks wait_hooks();
 // At least 2*n timing events (created on first use, kept by the context).
 fc_status timing_events(int n, cudaEvent_t** out);
 // Sum of elapsed times of the n event pairs (waits for the last one).

@@ -430,6 +430,7 @@ struct MgArgs {
     uint32_t* scratch;
     const int* bad;
     int* err;
+    WaitHooks hooks;
 };
 
 // Persistent: a CTA takes tiles of 128 x 256; per tile it runs the 16 moduli
@@ -492,6 +493,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     if (warp == 0) {
         if (lane == 0) {
             uint32_t g = 0;
+            const bool drop = p.hooks.drop_load && blockIdx.x == 0;  // stage g == 0 gets no load
             for (int64_t t = blockIdx.x; t < p.nitems && !*abort_flag; t += gridDim.x) {
                 const int4 it = p.items[t];
                 const int nk = it.w & 0xfffff;
@@ -499,6 +501,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                     for (int kt = 0; kt < nk; ++kt, ++g) {
                         const int s = g % S;
                         if (!tc::mbar_wait(&empty[s], ((g / S) & 1) ^ 1, abort_flag, p.err)) goto prod_done;
+                        if (drop && g == 0) continue;
                         tc::mbar_arrive_expect_tx(&full[s], STAGE);
                         uint8_t* st = base + s * STAGE;
                         tc::tma_load_2d(st, &tmA, &full[s], (it.z + kt) * MG_KT, l * p.planeM + it.x * MG_BM);
@@ -506,9 +509,10 @@ __global__ void __launch_bounds__(THREADS, 1)
                     }
             }
         prod_done:
-            // the loads in flight land before the CTA leaves
+            // the loads in flight land before the CTA leaves (a dropped stage has none)
             for (uint32_t q = 0; q < (uint32_t)S && q < g; ++q) {
                 const uint32_t gg = g - 1 - q;
+                if (drop && gg == 0) continue;
                 int no_abort = 0;
                 tc::mbar_wait(&full[gg % S], (gg / S) & 1, &no_abort, p.err);
             }
@@ -524,7 +528,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                     tc::fence_after_sync();
                     for (int kt = 0; kt < nk; ++kt, ++g) {
                         const int s = g % S;
-                        if (!tc::mbar_wait(&full[s], (g / S) & 1, abort_flag, p.err)) goto mma_done;
+                        if (!tc::mbar_wait(&full[s], (g / S) & 1, abort_flag, p.err, p.hooks.wait_ns)) goto mma_done;
                         tc::fence_after_sync();
                         const uint64_t da = tc::sdesc_k128(base_u32 + s * STAGE);
                         const uint64_t db = tc::sdesc_k128(base_u32 + s * STAGE + A_BYTES);
@@ -773,7 +777,7 @@ fc_status mg_gemm(const MgOperand& A, const MgOperand& B, const MgOut& out, cons
     FC_TRY(make_tmap_i8_2d(&ta, A.r, A.kp, (uint64_t)(MG_N - 1) * A.plane + A.rows, A.kp, MG_KT, MG_BM));
     FC_TRY(make_tmap_i8_2d(&tb, B.r, B.kp, (uint64_t)(MG_N - 1) * B.plane + B.rows, B.kp, MG_KT, MG_BN));
     const MgArgs a{items,   nitems,  (int)A.rows, (int)B.rows, (int)A.plane, (int)B.plane,
-                   A.scale, B.scale, out, (uint32_t*)scratch, flags, flags + 1};
+                   A.scale, B.scale, out, (uint32_t*)scratch, flags, flags + 1, wait_hooks()};
     const int grid = (int)std::min<int64_t>(nitems, ctx().sm_count);
     if (grid > 0)
         mg_gemm_kernel<<<grid, THREADS, SMEM, st>>>(ta, tb, a);
@@ -793,6 +797,14 @@ fc_status mg_fold(const double* part, int splits, int64_t M, int64_t N, double a
                   cudaStream_t st) {
     mg_fold_kernel<<<(unsigned)((M * N + 255) / 256), 256, 0, st>>>(part, splits, M, N, alpha, out, ld);
     return check_launch("mg_fold_kernel");
+}
+
+fc_status mg_outcome(const int* flags, const char* what, bool* stands) {
+    int hf[2];
+    FC_CUDA(cudaMemcpy(hf, flags, sizeof(hf), cudaMemcpyDeviceToHost));
+    if (hf[1]) return fail(FC_ERR_TIMEOUT, std::string(what) + ": a pipeline wait ran out");
+    *stands = !hf[0];
+    return FC_OK;
 }
 
 int mg_splits(int64_t M, int64_t N, int64_t K, bool upper) {

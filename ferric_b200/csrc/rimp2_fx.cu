@@ -1748,19 +1748,21 @@ int fx_exchange_choice(int nk, int grad) {
     return 1;
 }
 
-// Failure-path test hook of the pair kernel.  FERRIC_CUDA_WAIT_MS bounds the
-// MMA warp's waits for operand stages (default 4 s); with
-// FERRIC_CUDA_TEST_DROP_LOAD=1 CTA 0's producer issues no load for its first
-// stage, so that bounded wait runs out (nothing in flight, FC_ERR_TIMEOUT)
-// while every other wait of the kernel keeps its 4 s limit.
-static void fx_test_hooks(PairFxArgs* a) {
-    a->wait_ns = tc::WAIT_LIMIT_NS;
+WaitHooks wait_hooks() {
+    WaitHooks h{tc::WAIT_LIMIT_NS, 0};
     if (const char* e = std::getenv("FERRIC_CUDA_WAIT_MS")) {
         const long long v = std::atoll(e);
-        if (v > 0 && v <= 60000) a->wait_ns = (uint64_t)v * 1000000ull;
+        if (v > 0 && v <= 60000) h.wait_ns = (uint64_t)v * 1000000ull;
     }
     const char* d = std::getenv("FERRIC_CUDA_TEST_DROP_LOAD");
-    a->drop_load = (d && d[0] == '1') ? 1 : 0;
+    h.drop_load = d && d[0] == '1';
+    return h;
+}
+
+static void fx_test_hooks(PairFxArgs* a) {
+    const WaitHooks h = wait_hooks();
+    a->wait_ns = h.wait_ns;
+    a->drop_load = h.drop_load;
 }
 
 // FP64 X / Y tiles of the pair kernel's CTAs (global scratch, L2-resident).

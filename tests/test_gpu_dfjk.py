@@ -245,7 +245,9 @@ def test_small_builds_match_oracle(fc, n, naux, nocc):
     st = {}
     j, k = jk.j(d), jk.k_from_occ(c, stats=st)
     assert (st["launches"] == 1) == (naux * n * n * 8 <= 2 << 20)
-    j2, k2 = jk.jk_from_occ(c)
+    one = st["launches"] == 1
+    j2, k2 = jk.jk_from_occ(c, stats=st)
+    assert (st["launches"] == 1) == one
     # sums of up to naux n^2 terms in another order: 1e-13 of the largest element
     for x, y in ((j, orc.df_j_square(b, d)), (k, orc.df_k_occ(b, c))):
         assert np.abs(x - y).max() <= 1e-13 * np.abs(y).max() and np.array_equal(x, x.T)

@@ -124,9 +124,9 @@ def test_dfk_rank_update(fc, n, naux, nocc):
     assert torch.equal(k, k.T)
     c[3, 2] = float("nan")
     torch.cuda.synchronize()
-    k = jk.k_from_occ(c)
+    k = jk.k_from_occ(c, stats=st)
     torch.cuda.synchronize()
-    assert bool(torch.isnan(k).all())
+    assert st["tile_n"] == 64 and bool(torch.isnan(k).all())
     jk.close()
 
 
@@ -145,9 +145,9 @@ def test_dressing(fc, naux, n, nl, nr):
     _close(b, ref)
     m[5, 7] = float("inf")  # its row takes the DMMA form: not finite there, the others as before
     torch.cuda.synchronize()
-    b = dress.mo_dress(t, m, cl, cr)
+    b = dress.mo_dress(t, m, cl, cr, stats=st)
     torch.cuda.synchronize()
-    assert not bool(torch.isfinite(b[5]).any())
+    assert st["tile_n"] == 64 and not bool(torch.isfinite(b[5]).any())
     _close(torch.cat([b[:5], b[6:]]), torch.cat([ref[:5], ref[6:]]))
 
 
@@ -160,7 +160,7 @@ def test_response_2c(fc, naux, nov):
     torch.cuda.synchronize()
     st = {}
     y, g = rimp2.rimp2_response_2c(x, b, v, stats=st)
-    assert st["launches"] > 3
+    assert st["launches"] > 3 and st["tile_n"] == 256
     yr = v.T @ x
     _close(y, yr)
     _close(g, -2.0 * (v.T @ b) @ yr.T)
@@ -211,7 +211,9 @@ def test_graded_dressing(fc, case):
     t[:, :nl] = mo.T.reshape(naux, nl, n)
     # (Q|lr) = sum C_left[mu, l] t[Q, nu, mu] C_right[nu, r]: the tensor need not be symmetric here
     cl, cr = np.eye(n)[:, :nl], np.eye(n)
-    got = dress.mo_dress(np.ascontiguousarray(t.transpose(0, 2, 1)), m, np.ascontiguousarray(cl), cr)
+    st = {}
+    got = dress.mo_dress(np.ascontiguousarray(t.transpose(0, 2, 1)), m, np.ascontiguousarray(cl), cr, stats=st)
+    assert st["tile_n"] == 64
     sel = np.r_[0:7, naux - 7:naux]
     _rowwise(got[sel], m[sel], mo)
 
@@ -221,7 +223,10 @@ def test_graded_response(fc, case):
     from ferric_b200 import rimp2
     naux, nov = 513, 4099
     v, x = _graded(case, naux, nov, naux)
-    y, g = rimp2.rimp2_response_2c(np.ascontiguousarray(x.T), np.ascontiguousarray(x.T), np.ascontiguousarray(v.T))
+    st = {}
+    y, g = rimp2.rimp2_response_2c(np.ascontiguousarray(x.T), np.ascontiguousarray(x.T), np.ascontiguousarray(v.T),
+                                   stats=st)
+    assert st["tile_n"] == 64
     sel = np.r_[0:7, naux - 7:naux]
     _rowwise(y[sel], v[sel], x)
 
@@ -237,7 +242,11 @@ def test_graded_rank_update(fc):
     b[320:, :128, :128] = 1e-11 * rng.standard_normal((320, 128, 128))
     b = b + b.transpose(0, 2, 1)
     c = np.linalg.qr(rng.standard_normal((n, nocc)))[0]
-    k = DfJK(b).k_from_occ(np.ascontiguousarray(c))
+    st = {}
+    jk = DfJK(b)
+    k = jk.k_from_occ(np.ascontiguousarray(c), stats=st)
+    jk.close()
+    assert st["tile_n"] == 64
     w = (b.reshape(-1, n) @ c).reshape(naux, n, nocc).transpose(1, 0, 2).reshape(n, -1)
     sel = np.r_[0:3, 126:131]
     _rowwise(k[sel], w[sel], w, c=256.0)  # W itself is rounded: 2^-53 sums of n terms
