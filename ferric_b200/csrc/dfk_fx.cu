@@ -241,9 +241,10 @@ fc_status stage1_attr() {
 }
 
 // W = B C: every column tile reads all of B's slices, so the stage, HBM-bound,
-// takes the narrowest tile that holds all columns (with two tiles of 64 for
-// nocc 81 it ran 1.77 ms, B's slices alone are 0.79 at the copy rate).  Up to 64
-// columns two accumulator sets overlap the drain with the next item.
+// takes the narrowest tile that holds all columns (nocc 81, n 872, naux 2256: 1.43
+// ms; with two tiles of 64 1.77, B's slices alone are 0.79 at the copy rate).  Up
+// to 64 columns two accumulator sets overlap the drain with the next item.  Above
+// 128, where one tile cannot hold them, tiles of 64 (wider ones there were not measured).
 int stage1_bn(int64_t nocc) { return nocc <= 64 ? 64 : nocc <= 96 ? 96 : nocc <= 128 ? 128 : 64; }
 
 template <int BN>

@@ -225,6 +225,21 @@ def test_fused_jk_device_api_and_metric(fc):
     jk.close()
 
 
+@pytest.mark.parametrize("nocc,tile", [(64, 64), (65, 96), (96, 96), (97, 128), (112, 128), (113, 128), (128, 128),
+                                       (129, 64)])
+def test_mixed_column_tiles(fc, nocc, tile):
+    """The edges of stage 1's column tiles, and of the 32-column groups of J's row terms in its epilogue: K and J as
+    in the tests above, to their bounds."""
+    from ferric_b200.dfjk import DfJK
+    b, c, d = synthetic.dfjk_inputs(140, 30, nocc)
+    jk, st = DfJK(b, precision="mixed"), {}
+    jk.k_from_occ(c, stats=st)
+    jk.close()
+    assert st["tile_n"] == tile
+    test_mixed_dfk_exact_slices(fc, 140, 30, nocc)
+    test_fused_jk_from_occ(fc, 140, 30, nocc)
+
+
 def test_fused_jk_empty_channel(fc):
     from ferric_b200.dfjk import DfJK
     b, c, d = synthetic.dfjk_inputs(20, 30, 3)
