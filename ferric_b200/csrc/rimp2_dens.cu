@@ -249,9 +249,14 @@ __global__ void vv_fold_f64_kernel(const double* __restrict__ part, int nz, int6
     acc[e] += fold_in_order(part + e, nz, n * n);
 }
 
-// P_oo's tile: nocc rows by nocc columns over a very long K, bound by the DMMA
-// rate of the padded tile (nocc 33: 64 x 48 instead of 128 x 64, 540 -> 250 us).
+// The small tile of P_oo and P_vv.  P_oo (nocc rows by nocc columns over a very
+// long K) is bound by the DMMA rate of its padded tiles, so it takes the small
+// one where that covers a tenth less than 128 x 64: nocc 33, nvir 169 237 us
+// against 508, nocc 64, nvir 150 635 and 779, nocc 96, nvir 100 840 and 1020; at
+// nocc 97 to 128, where it covers an eighth more, 1217 and 1030, 1335 and 1110.
 constexpr int OO_M = 64, OO_N = 48;
+int64_t oo_padded(int64_t nocc, int bm, int bn) { return (nocc + bm - 1) / bm * bm * ((nocc + bn - 1) / bn * bn); }
+bool oo_small(int64_t nocc) { return 10 * oo_padded(nocc, OO_M, OO_N) <= 9 * oo_padded(nocc, DG_BM, DG_BN); }
 
 // P_vv's tile: 64 x 48 where its upper tiles cover a tenth less than those of
 // 128 x 64 (nvir 169: 9 x 3072 elements against 4 x 8192).
@@ -289,6 +294,7 @@ fc_status dens_attrs() {
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, DG_SMEM));
     FC_CUDA(cudaFuncSetAttribute(dgemm_upper_kernel<EpiBatchStore, OO_M, OO_N>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, dg_smem(OO_M, OO_N)));
+    FC_CUDA(cudaFuncSetAttribute(dgemm_tn_kernel<EpiSplit>, cudaFuncAttributeMaxDynamicSharedMemorySize, DG_SMEM));
     FC_CUDA(cudaFuncSetAttribute(dgemm_tn_kernel<EpiSplit, false, false, OO_M, OO_N>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, dg_smem(OO_M, OO_N)));
     g_dens_attr = true;
@@ -498,11 +504,13 @@ fc_status dens_f64_slab(const DensF64& o, int64_t nk, cudaStream_t st, int64_t* 
     // P_oo: rows i are nvir ld contiguous doubles in both slabs
     const int64_t K = nvir * ld;
     const int64_t kps = ((K + o.splits - 1) / o.splits + DG_BK - 1) / DG_BK * DG_BK;
-    const dim3 go((unsigned)((nocc + OO_N - 1) / OO_N), (unsigned)((nocc + OO_M - 1) / OO_M), (unsigned)o.splits);
+    const bool small = oo_small(nocc);
+    const int bm = small ? OO_M : DG_BM, bn = small ? OO_N : DG_BN;
+    const dim3 go((unsigned)((nocc + bn - 1) / bn), (unsigned)((nocc + bm - 1) / bm), (unsigned)o.splits);
     EpiSplit es{o.part_oo, nocc * nocc, (int)nocc};
     FC_CUDA(cudaMemsetAsync(o.part_oo, 0, (size_t)o.splits * nocc * nocc * 8, st));
-    dgemm_tn_kernel<EpiSplit, false, false, OO_M, OO_N>
-        <<<go, 256, dg_smem(OO_M, OO_N), st>>>(o.as, K, o.ts, K, (int)nocc, (int)nocc, K, kps, 0, es);
+    const auto kernel = small ? dgemm_tn_kernel<EpiSplit, false, false, OO_M, OO_N> : dgemm_tn_kernel<EpiSplit>;
+    kernel<<<go, 256, dg_smem(bm, bn), st>>>(o.as, K, o.ts, K, (int)nocc, (int)nocc, K, kps, 0, es, nullptr);
     FC_TRY(check_launch("dgemm_tn_kernel<P_oo>"));
     oo_fold_f64_kernel<<<(unsigned)((nocc * nocc + 255) / 256), 256, 0, st>>>(o.part_oo, o.splits, nocc * nocc,
                                                                               o.acc_oo);

@@ -70,10 +70,12 @@ def test_densities_f64_match_oracle(fc, naux, nocc, nvir):
     assert np.abs(g - g2).max() <= 1e-13 * np.abs(g2).max()
 
 
-# edges of P_vv's FP64 tiles (64 x 48, and 128 x 64 at nvir 128), K in one and
-# in several ranges; sums of at most nocc^2 nvir terms: 1e-12 of the largest
+# edges of P_vv's FP64 tiles (64 x 48, and 128 x 64 at nvir 128) and of P_oo's
+# (64 x 48 at 48, 65 and 96 orbitals, 128 x 64 at 97), K in one and in several
+# ranges; sums of at most nocc^2 nvir terms: 1e-12 of the largest
 @pytest.mark.parametrize("naux,nocc,nvir", [(20, 3, 48), (20, 6, 49), (20, 2, 96), (30, 4, 97), (12, 3, 128),
-                                            (15, 2, 193), (12, 1, 64)])
+                                            (15, 2, 193), (12, 1, 64), (9, 48, 11), (9, 65, 10), (8, 96, 7),
+                                            (8, 97, 7)])
 def test_densities_f64_tiles(fc, naux, nocc, nvir):
     from ferric_b200 import rimp2
     b, eo, ev = synthetic.rimp2_inputs(naux, nocc, nvir)
