@@ -227,17 +227,16 @@ struct EpiBatchStore {
     }
 };
 
-// s + x[0] + x[stride] + ... (n terms, in order), eight loads in flight.
+// s + x[0] + x[stride] + ... (n terms, in order), sixteen loads in flight, the
+// last ones too.
 __device__ __forceinline__ double fold_in_order(const double* __restrict__ x, int n, int64_t stride, double s = 0.0) {
-    int i = 0;
-    for (; i + 8 <= n; i += 8) {
-        double v[8];
+    for (int i = 0; i < n; i += 16, x += 16 * stride) {
+        double v[16];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) v[u] = x[(int64_t)(i + u) * stride];
+        for (int u = 0; u < 16; ++u) v[u] = i + u < n ? __ldg(x + u * stride) : 0.0;
 #pragma unroll
-        for (int u = 0; u < 8; ++u) s += v[u];
+        for (int u = 0; u < 16; ++u) s += v[u];
     }
-    for (; i < n; ++i) s += x[(int64_t)i * stride];
     return s;
 }
 
