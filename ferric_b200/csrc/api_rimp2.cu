@@ -465,7 +465,7 @@ fc_status ump2_dispatch(const UmpSpin& a, const UmpSpin& b, int64_t naux, int32_
     *e_aa = *e_bb = *e_ab = 0.0;
     if (naux == 0) return FC_OK;
     const int64_t nova = a.nocc * a.nvir, novb = b.nocc * b.nvir;
-    if (precision == FC_PREC_F64 && nova && novb && mod_energy_pays(naux, nova + novb, (nova + novb + 1) / 2)) {
+    if (precision == FC_PREC_F64 && nova && novb && mod_energy_pays(naux, nova + novb, (nova + novb + 1) / 2, 2)) {
         bool ran = false;
         FC_TRY(ump2_energy_mod(a, b, naux, chunk_budget(), st, e_aa, e_bb, e_ab, stats, &ran));
         if (ran) return FC_OK;

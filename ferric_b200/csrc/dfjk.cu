@@ -535,7 +535,8 @@ fc_status dfk_build_f64(fc_dfjk* h, const double* c_occ, int64_t nocc, double* k
     FC_TRY(ws_get(WS_MISC, nocc * n * 8, &vct));
     FC_TRY(ws_get(WS_T, n * kdim * 8, &vw));
     // K = W W^T through residues (mgemm.cuh) where the product is worth W's
-    // conversion: n = 600, kdim = 144000: 2.50 -> 0.95 ms; even at n = 400, kdim = 64000.
+    // conversion.  J and K at n^2 kdim = 9.2e9 (n 350, kdim 75000) 1416 us with them, 1553
+    // without; at 3.6e9 (300, 40000) 777 and 751; even near 6e9.
     FC_TRY(ws_get(WS_PART, (int64_t)nsplit * n * n * 8, &vpart));
     void* vflags = nullptr;
     const bool residues = (double)n * n * kdim >= 8e9 && n <= 65535 && ws_try(WS_OUT, 256, &vflags);

@@ -141,9 +141,13 @@ fc_status mo_dress(const double* eri3, bool host, int64_t naux, int64_t n, const
     // FP64 through residues (mgemm.cuh) where the products outweigh their
     // operands' conversion: the MO step per chunk (K = n) and the dressing
     // (K = naux).  The MO tensor then stays in its natural order (Q, l, r).  Whole
-    // call at 2 naux^2 width = 5.5e9: 591 us against 517 DMMA; at 2.6e10: 1351, 1738.
+    // call at 2 naux^2 width = 1.05e10 (naux 800, width 8200) 840 us against 897 DMMA, at
+    // 2.6e10 (1000, 13200) 1283 and 1642, at 3.3e9 (616, 4321) 576 and 478.  Fewer aux
+    // functions spread the conversion over less: at 1.1e10 (500, 22100) 1428 and 1309, at
+    // 1.5e10 (500, 30000) 1619 and 1702.
     void* vflags = nullptr;
-    const bool residues = precision == FC_PREC_F64 && 2.0 * naux * (double)naux * width >= 1e10 && naux <= MG_KMAX &&
+    const double flops = 2.0 * naux * (double)naux * width;
+    const bool residues = precision == FC_PREC_F64 && flops >= (naux >= 640 ? 1e10 : 1.5e10) && naux <= MG_KMAX &&
                           n <= MG_KMAX && n >= 256 && ws_try(WS_OUT, 256, &vflags);
     int* mg_flags = (int*)vflags;
     if (residues) FC_CUDA(cudaMemsetAsync(vflags, 0, 256, st));

@@ -59,12 +59,15 @@ fc_status response_2c(const double* x_ov, const double* b_ov, const double* vis,
     void* vc;
     FC_TRY(ws_get(WS_PART, (size_t)naux * nov * 8, &vc));
     double* cfit = (double*)vc;
-    // residues where the products outweigh the operands' conversion: a gradient
-    // chain with them at 2 naux^2 nov = 1.8e9 (naux 532, nov 3225) 1772 us, without
-    // 1853; at 5.5e9 3161 and 3641; at 9e8 1361 and 1318.
+    // residues where the products outweigh the operands' conversion: at 2 naux^2
+    // nov = 1.8e9 (naux 532, nov 3225) 471 us, without 532; at 3.3e9 (616, 4321) 508 and
+    // 767; at 9.2e8 (448, 2289) 406 and 344.  Short rows favour DMMA, whose third
+    // product is then short: at 1.6e9 (900, 1000) 449 and 325, at 2.4e9 (900, 1500) 481
+    // and 511.
+    const double flops = 2.0 * naux * (double)naux * nov;
+    const bool pays = flops >= 1.5e9 && (2 * nov >= 3 * naux || flops >= 3e9) && naux <= MG_KMAX;
     void* vflags = nullptr;
-    const bool residues =
-        2.0 * naux * (double)naux * nov >= 1.5e9 && naux <= MG_KMAX && ws_try(WS_OUT, 256, &vflags);
+    const bool residues = pays && ws_try(WS_OUT, 256, &vflags);
     const int splits = residues ? mg_splits(naux, naux, nov, false) : 1;
     int* flags = (int*)vflags;
     double* gpart = nullptr;

@@ -65,8 +65,9 @@ bool mod_grad_pays(int64_t naux, int64_t nocc, int64_t nvir);
 fc_status rimp2_grad_mod(const Rimp2Dev& d, cudaStream_t st, double* e_os, double* e_ss, double* gamma,
                          double* de_docc, double* de_dvir, fc_stats* stats, const GammaSink* sink,
                          const DensOut* dens, bool* ran);
-// Energies: rows x cols products over naux (one spin: nov x nov / 2).
-bool mod_energy_pays(int64_t naux, int64_t rows, int64_t cols);
+// Energies: rows x cols products over naux (one spin: nov x nov / 2; nspin 2:
+// both spins' rows together).
+bool mod_energy_pays(int64_t naux, int64_t rows, int64_t cols, int nspin = 1);
 fc_status rimp2_energy_mod(const Rimp2Dev& d, cudaStream_t st, double* e_os, double* e_ss, fc_stats* stats,
                            bool* ran);
 

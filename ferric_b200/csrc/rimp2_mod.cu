@@ -293,10 +293,11 @@ struct ChunkPair {
 
 }  // namespace
 
-// Where the residue form pays: the conversions (about 100 instructions per
-// element), the passes over G and the dozen launches are spread over enough
-// products.  Gradient at 2 naux (nocc nvir)^2 = 1.7e9 (naux 364, nocc 17, nvir
-// 89): 355 us here, 395 DMMA; at 4.7e9 426 and 582; the forms cross near 1.3e9.
+// Where the residue form pays: the conversions (about 110 instructions per
+// element), the passes over G and the launches are spread over enough
+// products.  Gradient at 2 naux (nocc nvir)^2 = 1.67e9 (naux 364, nocc 17, nvir
+// 89): 348 us here, 378 DMMA; at 4.7e9 435 and 570; the forms cross near 1.3e9
+// (340, 16, 85: 333 and 326).
 bool mod_grad_pays(int64_t naux, int64_t nocc, int64_t nvir) {
     return naux <= MG_KMAX && 2.0 * naux * (double)(nocc * nvir) * (double)(nocc * nvir) >= 1.5e9;
 }
@@ -534,10 +535,13 @@ fc_status rimp2_grad_mod(const Rimp2Dev& d, cudaStream_t st, double* e_os, doubl
 
 // ------------------------------------------------------------- energies --
 
-// At 2 naux rows cols = 1.67e9 (naux 420, nocc 18, nvir 110; cols: half of the
-// row's columns on average) 163 us here, 177 DMMA.
-bool mod_energy_pays(int64_t naux, int64_t rows, int64_t cols) {
-    return naux <= MG_KMAX && 2.0 * naux * (double)rows * (double)cols >= 1e9;
+// At 2 naux rows cols = 1.65e9 (naux 420, nocc 18, nvir 110; cols: half of the
+// row's columns on average) 153 us here, 190 DMMA.  Below, DMMA's last wave
+// decides: 153 and 160 at 1.0e9 (700, 10, 120), 150 and 143 at 1.24e9 (400, 16,
+// 110), 136 and 99 at 5e8.  The two spins' energies, three passes each: 329 and
+// 386 at 2.7e9, 326 and 318 at 1.9e9.
+bool mod_energy_pays(int64_t naux, int64_t rows, int64_t cols, int nspin) {
+    return naux <= MG_KMAX && 2.0 * naux * (double)rows * (double)cols >= (nspin > 1 ? 2.2e9 : 1.1e9);
 }
 
 namespace {

@@ -123,7 +123,7 @@ def test_spare_memory_leaves_later_plans_alone(fc):
     """What an FP64 energy keeps for its next call is given back on demand: it takes no chunks from a later gradient."""
     import ferric_b200._lib as L
     from ferric_b200 import rimp2
-    ins, small = _dev(*synthetic.rimp2_inputs(640, 24, 129)), _dev(*synthetic.rimp2_inputs(1200, 10, 95))
+    ins, small = _dev(*synthetic.rimp2_inputs(640, 24, 129)), _dev(*synthetic.rimp2_inputs(1200, 10, 105))
 
     def launches():
         st = {}
