@@ -18,7 +18,7 @@ __version__ = "0.1.0"
 
 
 def __getattr__(name):
-    if name in ("FcError", "FcStats", "init", "last_error"):
+    if name in ("FcError", "FcStats", "init", "last_error", "pool_used", "release_workspace"):
         from . import _lib
         return getattr(_lib, name)
     raise AttributeError(name)

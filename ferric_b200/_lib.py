@@ -168,6 +168,16 @@ def init(device=0, pool_bytes=0):
         _initialised = (device, pool_bytes)
 
 
+def release_workspace():
+    """Free the device memory that the library keeps for its next calls (handles keep theirs)."""
+    check(lib.fc_release_workspace())
+
+
+def pool_used():
+    """Bytes that the library holds on the device: kept workspaces and handles."""
+    return int(lib.fc_pool_used())
+
+
 def ensure_init():
     if _initialised is None:
         dev = 0

@@ -11,6 +11,13 @@ the next step of an analytic gradient wants) or an all-reduce of the whole
 Gamma.  The reference's MPI path (ferric-mp2/src/mpi_rimp2.rs:16-43) cuts
 aux bands and all-reduces per-i intermediates instead.
 
+FP64 shards run on the DMMA kernels, whose chunk pairs are what the processes
+share out; a call on one GPU takes the faster residue products where it is
+large (ferric_b200/csrc/mgemm.cuh).  So a few processes can take longer than
+one: at the C20H42 def2-TZVP shapes (naux 2150, nocc 81, nvir 791) a gradient
+takes 258 ms on one GPU and about 1300 ms / n over n, less only from six
+processes on.  Mixed shards have the kernels of the unsharded call.
+
 DF-JK: each process holds an aux band of B (the reference's partition,
 ferric-scf/src/parallel.rs:215-231) and all-reduces its J and K (df_j.rs:101-115,
 df_k.rs:1522-1526); dressed tensors only (no metric solve across bands).

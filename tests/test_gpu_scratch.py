@@ -1,7 +1,6 @@
 """Scratch limits: a pool cap that leaves the FP64 calls what their DMMA forms take lets them run, whatever a faster
 form would like to have, and memory that the library gives back on demand shrinks no later call."""
 import contextlib
-import ctypes
 
 import numpy as np
 import pytest
@@ -16,9 +15,8 @@ pytestmark = pytest.mark.gpu
 def _cap(scratch):
     """At most `scratch` bytes beside what handles hold."""
     import ferric_b200._lib as L
-    L.lib.fc_pool_used.restype = ctypes.c_uint64
-    L.check(L.lib.fc_release_workspace())
-    L.init(0, L.lib.fc_pool_used() + scratch)
+    L.release_workspace()
+    L.init(0, L.pool_used() + scratch)
     try:
         yield
     finally:
@@ -132,7 +130,7 @@ def test_spare_memory_leaves_later_plans_alone(fc):
 
     with _cap(1 << 40):
         assert launches() == 1  # its workspace is there
-        held = L.lib.fc_pool_used()
+        held = L.pool_used()
         # the least that leaves all 24 orbitals in one chunk is less than that and what the energy keeps
         for mib in range(240, 640, 20):
             L.init(0, held + (mib << 20))
@@ -140,5 +138,18 @@ def test_spare_memory_leaves_later_plans_alone(fc):
                 break
         st = {}
         rimp2.rimp2_energy(*small, stats=st)
-        assert st["tile_n"] == 256 and L.lib.fc_pool_used() > held + (20 << 20)
+        assert st["tile_n"] == 256 and L.pool_used() > held + (20 << 20)
         assert launches() == 1
+
+
+def test_release_workspace(fc):
+    """What calls keep is freed on request, and the next call takes it again."""
+    import ferric_b200
+    from ferric_b200 import rimp2
+    ins = _dev(*synthetic.rimp2_inputs(640, 24, 129))
+    ferric_b200.release_workspace()
+    held = ferric_b200.pool_used()
+    e = rimp2.rimp2_energy(*ins)
+    assert ferric_b200.pool_used() > held + (100 << 20)
+    ferric_b200.release_workspace()
+    assert ferric_b200.pool_used() == held and rimp2.rimp2_energy(*ins) == e
