@@ -468,6 +468,7 @@ fc_status rimp2_grad_f64(const Rimp2Dev& d, cudaStream_t st, double* e_os, doubl
                                              4 * d.chunk_bytes)
                             : grad_chunk_f64(nocc, nvir, d.chunk_bytes, d.nshards);
     const int64_t nch = (nocc + cc - 1) / cc;
+    const bool single = nch == 1 && !dens && d.nshards == 1;  // no tables, no running sums
     struct CP {
         int64_t i0, ni, j0, nj, p0, np;
     };
@@ -483,13 +484,13 @@ fc_status rimp2_grad_f64(const Rimp2Dev& d, cudaStream_t st, double* e_os, doubl
             x.j0 = J * cc;
             x.nj = std::min(cc, nocc - x.j0);
             x.p0 = (int64_t)hp.size();
-            for (int64_t i = x.i0; i < x.i0 + x.ni; ++i)
+            x.np = I == J ? x.ni * (x.ni + 1) / 2 : x.ni * x.nj;
+            for (int64_t i = x.i0; !single && i < x.i0 + x.ni; ++i)
                 for (int64_t j = (I == J ? i : x.j0); j < x.j0 + x.nj; ++j) hp.push_back(make_int2((int)i, (int)j));
-            x.np = (int64_t)hp.size() - x.p0;
             cps.push_back(x);
         }
     const int64_t npairs_all = (int64_t)hp.size();
-    for (int ta = 0; ta < ntile; ++ta)
+    for (int ta = 0; !single && ta < ntile; ++ta)
         for (int tb = 0; tb < ntile; ++tb) hp.push_back(make_int2(ta, tb));
     const int64_t ncp = (int64_t)cps.size();
     const std::vector<int> owner = chunk_pair_owner(nocc, cc, d.nshards);
@@ -515,12 +516,11 @@ fc_status rimp2_grad_f64(const Rimp2Dev& d, cudaStream_t st, double* e_os, doubl
                                  I == nch - 1});
     }
     const int64_t nsteps = (int64_t)steps.size();
-    const bool single = nch == 1 && !dens && d.nshards == 1;  // no tables, no running sums
     DensF64 dx{};
 
-    void *vpairs, *vpart, *vT, *vout;
+    void *vpairs = nullptr, *vpart, *vT, *vout;
     const size_t blk = (size_t)cc * nvir * cc * nvir;  // doubles of one amplitude block
-    FC_TRY(ws_get(WS_PAIRS, hp.size() * sizeof(int2), &vpairs));
+    if (!single) FC_TRY(ws_get(WS_PAIRS, hp.size() * sizeof(int2), &vpairs));
     FC_TRY(ws_get(WS_T, 2 * blk * sizeof(double), &vT));
     FC_TRY(ws_get(WS_PART, (size_t)max_items * (2 + 2 + PR_T) * sizeof(double), &vpart));
     FC_TRY(ws_get(WS_OUT, (size_t)(2 * ncp + nocc) * sizeof(double) + 64, &vout));

@@ -1,9 +1,10 @@
 """FP64 RI-MP2 through residue products (csrc/mgemm.cu, rimp2_mod.cu) against
-the FP64 oracle.  Sizes sit at the edges of the amplitude tiles (64), the GEMM
+the FP64 oracle.  Sizes sit at the edges of the amplitude tiles (32), the GEMM
 tiles (128 x 256) and the k-steps (128); ``stats["tile_n"]`` tells the route
 (256: residues, 64: DMMA).  Tolerance: the sums of the test run over at most
 n = 5000 terms, |error| <= n 2^-53 |x| |y| in either order, 1e-12 of the
-largest element (measured 3e-15)."""
+largest element (measured 3e-15); where large elements of one operand meet
+small ones of the other, 2^-53 of sums of |x_k y_k| by row and by column."""
 import numpy as np
 import pytest
 
