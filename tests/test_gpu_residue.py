@@ -219,6 +219,23 @@ def test_graded_dressing(fc, case):
     _rowwise(got[sel], m[sel], mo)
 
 
+def test_guard_passes_ordinary_slopes(fc):
+    """Slopes of e^-6 over the row: 0.02 by the guard's measure, above its line, and the residues' error (2^-61 / 0.02
+    of |a| |b|^T) is below a single FP64 rounding's."""
+    from ferric_b200 import dress
+    naux, n, nl = 640, 256, 64
+    rng = np.random.default_rng(23)
+    q = np.arange(naux) * 6.0 / naux
+    m, mo = rng.standard_normal((naux, naux)) * np.exp(-q), rng.standard_normal((nl * n, naux)) * np.exp(q)
+    t = np.zeros((naux, n, n))
+    t[:, :, :nl] = mo.T.reshape(naux, nl, n).transpose(0, 2, 1)
+    st = {}
+    got = dress.mo_dress(t, m, np.ascontiguousarray(np.eye(n)[:, :nl]), np.eye(n), stats=st)
+    assert st["tile_n"] == 256
+    sel = np.r_[0:7, naux - 7:naux]
+    _rowwise(got[sel], m[sel], mo, c=1.0)
+
+
 @pytest.mark.parametrize("case", CASES)
 def test_graded_response(fc, case):
     from ferric_b200 import rimp2
