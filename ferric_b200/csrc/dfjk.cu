@@ -586,7 +586,7 @@ fc_status dfk_build_f64(fc_dfjk* h, const double* c_occ, int64_t nocc, double* k
     }
     FC_TRY(dfk_stats(h, nocc, room ? 4 + MG_LAUNCHES_SAME : 4, DG_BM, DG_BN, st, stats));
     bool stands = false;
-    if (stats && room) FC_TRY(mg_outcome((const int*)vflags, "DF-K", &stands));
+    if (stats && room) FC_TRY(mg_outcome((const int*)vflags, "DF-K", st, &stands));
     if (stands) {
         stats->tile_m = MG_BM;
         stats->tile_n = MG_BN;

@@ -272,7 +272,7 @@ fc_status mo_dress(const double* eri3, bool host, int64_t naux, int64_t n, const
         FC_CUDA(cudaEventElapsedTime(&ms, cx.ev0, cx.ev1));
         FC_CUDA(cudaEventElapsedTime(&m4, ev[0], ev[1]));
         bool stands = false;
-        if (room) FC_TRY(mg_outcome(mg_flags, "MO dressing", &stands));
+        if (room) FC_TRY(mg_outcome(mg_flags, "MO dressing", st, &stands));
         stats->kernel_ms = ms;
         stats->flops = 2.0 * naux * (double)n * n * nl + 2.0 * naux * (double)nl * n * nr +
                        2.0 * (double)naux * naux * width;

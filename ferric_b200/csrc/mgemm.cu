@@ -799,9 +799,10 @@ fc_status mg_fold(const double* part, int splits, int64_t M, int64_t N, double a
     return check_launch("mg_fold_kernel");
 }
 
-fc_status mg_outcome(const int* flags, const char* what, bool* stands) {
+fc_status mg_outcome(const int* flags, const char* what, cudaStream_t st, bool* stands) {
     int hf[2];
-    FC_CUDA(cudaMemcpy(hf, flags, sizeof(hf), cudaMemcpyDeviceToHost));
+    FC_CUDA(cudaMemcpyAsync(hf, flags, sizeof(hf), cudaMemcpyDeviceToHost, st));
+    FC_CUDA(cudaStreamSynchronize(st));
     if (hf[1]) return fail(FC_ERR_TIMEOUT, std::string(what) + ": a pipeline wait ran out");
     *stands = !hf[0];
     return FC_OK;

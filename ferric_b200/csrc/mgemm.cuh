@@ -123,9 +123,9 @@ struct MgSrc {
 fc_status mg_multiply(const MgSrc& a, const MgSrc& b, int64_t K, MgOut out, bool upper, int splits, int* flags,
                       cudaStream_t st, bool* room, double** part = nullptr);
 constexpr int MG_LAUNCHES = 10, MG_LAUNCHES_SAME = 6;  // kernels of a product of two matrices, of one with itself
-// After a synchronisation: whether the products under `flags` stand (or their
-// DMMA form ran); FC_ERR_TIMEOUT where a wait ran out.
-fc_status mg_outcome(const int* flags, const char* what, bool* stands);
+// Synchronises: whether the products under `flags` stand (or their DMMA form
+// ran); FC_ERR_TIMEOUT where a wait ran out.
+fc_status mg_outcome(const int* flags, const char* what, cudaStream_t st, bool* stands);
 // out[n * ld + m] = alpha * sum of the splits' partials, in order.
 fc_status mg_fold(const double* part, int splits, int64_t M, int64_t N, double alpha, double* out, int64_t ld,
                   cudaStream_t st);

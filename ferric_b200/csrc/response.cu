@@ -109,7 +109,7 @@ fc_status response_2c(const double* x_ov, const double* b_ov, const double* vis,
         stats->flops = 6.0 * (double)naux * naux * nov;
         stats->precision = FC_PREC_F64;
         bool stands = false;
-        if (mg) FC_TRY(mg_outcome(mg, "RI response", &stands));
+        if (mg) FC_TRY(mg_outcome(mg, "RI response", st, &stands));
         stats->launches += 3 + (mg ? 3 * MG_LAUNCHES + (splits > 1 ? 1 : 0) : 0);
         stats->tile_m = stands ? MG_BM : DG_BM;
         stats->tile_n = stands ? MG_BN : DG_BN;
