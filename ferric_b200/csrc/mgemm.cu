@@ -676,7 +676,7 @@ static fc_status mg_pass(const MgMat& x, int axis, int8_t* r, const MgMat* y, in
     const double2* ys = y ? y->sum[1 - py] : nullptr;
     double2* gp = (double2*)part;
     const int64_t tiles = axis ? kp / 128 : (kp + 511) / 512;
-    const dim3 g = axis ? dim3((unsigned)((R + 31) / 32), (unsigned)tiles) : dim3((unsigned)((R + 7) / 8), (unsigned)tiles);
+    const dim3 g((unsigned)(axis ? (R + 31) / 32 : (R + 7) / 8), (unsigned)tiles);
     if (axis) {
         if (r && y) mg_cols_kernel<true, true><<<g, 256, 0, st>>>(x, kp, ys, gp, r, bad);
         else if (r) mg_cols_kernel<true, false><<<g, 256, 0, st>>>(x, kp, ys, gp, r, bad);
@@ -824,7 +824,8 @@ fc_status mg_multiply(const MgSrc& a, const MgSrc& b, int64_t K, MgOut out, bool
     const TileGrid g = tile_grid(a.rows, b.rows, K, upper, splits);
     // the sums over a range of K stay exact, an item's word holds its split, the launches' grids their tiles
     const int64_t gmax = 65535 * 128;
-    if (std::min<int64_t>(K, (int64_t)g.kps * MG_KT) > MG_KMAX || splits > 2047 || rmax > gmax || K > gmax) return FC_OK;
+    if (std::min<int64_t>(K, (int64_t)g.kps * MG_KT) > MG_KMAX || splits > 2047 || rmax > gmax || K > gmax)
+        return FC_OK;
     const int64_t items = mg_tiles(a.rows, b.rows, K, upper, splits, nullptr);
     size_t off = 0;
     auto take = [&](size_t bytes) {
